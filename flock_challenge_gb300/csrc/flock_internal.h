@@ -74,14 +74,14 @@ int flock_launch_lig_intro_eq(const void* f, size_t n, const void* lo, const voi
 int flock_launch_glue_eq(void* b, size_t n, const void* lo, const void* hi, int lo_bits, const uint64_t beta[2],
                          cudaStream_t st);
 int flock_launch_glue(void* b, const void* add, size_t n, const uint64_t beta[2], cudaStream_t st);
-// LO holds nq << flock_induce_basis_lo_bits(n) entries, HI nq << (n - that).
-int flock_induce_basis_lo_bits(int n);
-// what_lin: [n][32] F128, What_k(x^b) (the normalized subspace polynomials on
-// the index bits; What_k(q) is their XOR over the set bits of q).
-// scratch: flock_induce_basis_scratch_bytes(n) bytes (slice partials of small bases)
-size_t flock_induce_basis_scratch_bytes(int n);
-int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, const void* what_lin, const void* alpha_w,
-                              void* W, void* LO, void* HI, void* basis, void* scratch, cudaStream_t st);
+// The basis of nq queries (sorted, distinct positions of a code of 2^log_d
+// positions) over n coordinates. what_lin: [n][32] F128, What_k(x^b) (the
+// normalized subspace polynomials on the index bits; What_k(q) is their XOR
+// over the set bits of q). LO: flock_induce_basis_rows_bytes(n, log_d, nq)
+// bytes of scratch.
+size_t flock_induce_basis_rows_bytes(int n, int log_d, int nq);
+int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, int log_d, const void* what_lin,
+                              const void* alpha_w, void* LO, void* basis, cudaStream_t st);
 int flock_launch_gather_rows(const void* mat, const uint32_t* rows, int n_rows, int width, void* out,
                              cudaStream_t st);
 int flock_launch_gather_nodes(const void* tree, const uint32_t* idx, int n, void* out, cudaStream_t st);

@@ -7,8 +7,8 @@
 //    tables, returning the message and h = sum f eq (ligerito.rs:5684-5702),
 //    and its glue b += beta eq(z);
 //  * induced basis (ligerito.rs:1989-2160): basis[j] = sum_i alpha_i Xhat_j(q_i)
-//    with Xhat_j = prod_{k in bits(j)} What_k; computed as a sum over queries of
-//    products of low/high tensor halves;
+//    with Xhat_j = prod_{k in bits(j)} What_k: the transpose of the code's
+//    transform applied to the weights alpha_i at the opened positions;
 //  * glue b += beta * basis, row and tree-node gathers for openings.
 #include "flock_internal.h"
 #include "gf128.cuh"
@@ -114,111 +114,129 @@ __global__ void glue_kernel(gf128* __restrict__ b, const gf128* __restrict__ add
     b[j] = gf_add(b[j], gf_mul(beta, add[j]));
 }
 
-// What_k(q_i) for k < n (ligerito.rs:1776-1824: s_0 = q, s_k = s^2 + s_{k-1}(v_{k-1}) s,
-// normalized by 1 / s_k(v_k)). Each s_k is GF(2)-linear in its argument (a
-// square plus a constant multiple of a linear map), so What_k(q) is the XOR,
-// over the set bits b of the 32-bit index q, of lin[k][b] = What_k(x^b): one
-// thread per (query, k), no product.
-__global__ void what_kernel(const uint32_t* __restrict__ queries, int nq, int n, const gf128* __restrict__ lin,
-                            gf128* __restrict__ W) {
-  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)nq * n) return;
-  const int i = (int)(e / n), k = (int)(e % n);
-  const uint32_t q = queries[i];
-  const gf128* row = lin + (size_t)k * 32;
-  gf128 acc = gf_zero();
-  for (int b = 0; b < 32; b++)
-    if ((q >> b) & 1) acc = gf_add(acc, row[b]);
-  W[e] = acc;
-}
-
-// T[i][j] = scale_i * prod_{k < bits, bit k of j} W[i][k0 + k]; scale_i = alpha_i or 1.
-// CTA (query i, chunk c) first builds the sub-tables of the low TB_LO bits
-// (scaled) and of the remaining high bits (at most TB_HI) in shared memory,
-// then forms its 256 entries with one product each (a chain of up to `bits`
-// dependent products per entry before).
+// LO[i][j] = alpha_i prod_{k < bits, bit k of j} What_k(q_i)
+// (ligerito.rs:1776-1824: s_0 = q, s_k = s^2 + s_{k-1}(v_{k-1}) s, normalized by
+// 1 / s_k(v_k)). Each s_k is GF(2)-linear in its argument (a square plus a
+// constant multiple of a linear map), so What_k(q) is the XOR, over the set
+// bits b of the 32-bit index q, of lin[k][b] = What_k(x^b): no product. CTA
+// (query i, chunk c) forms those values, then the sub-tables of the low TB_LO
+// bits (scaled) and of the remaining high bits (at most TB_HI) in shared
+// memory, then its 256 entries with one product each.
 constexpr int TB_LO = 5, TB_HI = 7, TB_THREADS = 256;
 static_assert((1 << TB_LO) <= 32 && 32 + (1 << TB_HI) <= TB_THREADS, "sub-table builders fit the CTA");
 __global__ void __launch_bounds__(TB_THREADS)
-tensor_kernel(const gf128* __restrict__ W, int nq, int n, int k0, int bits, const gf128* __restrict__ scale,
-              gf128* __restrict__ T) {
-  __shared__ gf128 lo_t[1 << TB_LO], hi_t[1 << TB_HI];
+query_tensor_kernel(const uint32_t* __restrict__ queries, int bits, const gf128* __restrict__ lin,
+                    const gf128* __restrict__ alpha, gf128* __restrict__ LO) {
+  __shared__ gf128 w[TB_LO + TB_HI], lo_t[1 << TB_LO], hi_t[1 << TB_HI];
   const int lb = bits < TB_LO ? bits : TB_LO, hb = bits - lb;
   const size_t len = (size_t)1 << bits;
   const size_t chunks = (len + TB_THREADS - 1) / TB_THREADS;
   const int i = (int)(blockIdx.x / chunks);
   const size_t c = blockIdx.x % chunks;
-  const gf128* w = W + (size_t)i * n + k0;
   const int t = threadIdx.x;
-  if (t < (1 << lb)) {
-    gf128 acc = scale ? scale[i] : gf_one();
-    for (int k = 0; k < lb; k++)
-      if ((t >> k) & 1) acc = gf_mul(acc, w[k]);
-    lo_t[t] = acc;
-  } else if (t >= 32 && t - 32 < (1 << hb)) {
-    const int u = t - 32;
-    gf128 acc = gf_one();
-    for (int k = 0; k < hb; k++)
-      if ((u >> k) & 1) acc = gf_mul(acc, w[lb + k]);
-    hi_t[u] = acc;
+  // four lanes per coordinate, eight index bits each
+  if (t < 64) {  // two whole warps
+    const int k = t >> 2, b0 = (t & 3) * 8;
+    gf128 acc = gf_zero();
+    if (k < bits) {
+      const uint32_t q = queries[i] >> b0;
+      const gf128* row = lin + (size_t)k * 32 + b0;
+#pragma unroll
+      for (int b = 0; b < 8; b++)
+        if ((q >> b) & 1) acc = gf_add(acc, row[b]);
+    }
+#pragma unroll
+    for (int off = 1; off < 4; off <<= 1)
+#pragma unroll
+      for (int v = 0; v < 4; v++) acc.w[v] ^= __shfl_xor_sync(0xffffffffu, acc.w[v], off);
+    if ((t & 3) == 0 && k < TB_LO + TB_HI) w[k] = acc;
+  }
+  __syncthreads();
+  // one loop for both sub-tables: a small body (the latency of a cold kernel)
+  {
+    const bool is_lo = t < (1 << lb), is_hi = t >= 32 && t - 32 < (1 << hb);
+    const int u = is_lo ? t : t - 32, k0 = is_lo ? 0 : lb, nb = is_lo ? lb : hb;
+    if (is_lo || is_hi) {
+      gf128 acc = is_lo ? alpha[i] : gf_one();
+#pragma unroll 1
+      for (int k = 0; k < nb; k++)
+        if ((u >> k) & 1) acc = gf_mul(acc, w[k0 + k]);
+      if (is_lo) lo_t[u] = acc;
+      else hi_t[u] = acc;
+    }
   }
   __syncthreads();
   const size_t j = c * TB_THREADS + t;
-  if (j < len) T[(size_t)i * len + j] = gf_mul(lo_t[j & ((1 << lb) - 1)], hi_t[j >> lb]);
+  if (j < len) LO[(size_t)i * len + j] = gf_mul(lo_t[j & ((1 << lb) - 1)], hi_t[j >> lb]);
 }
 
-// basis[j] = sum_i LO[i][j & mask] * HI[i][j >> lo_bits]. Slice blockIdx.y
-// sums the queries [y q_per, (y + 1) q_per) into row y of out (the slices'
-// rows are then XOR-reduced), so small bases still fill the GPU.
-__global__ void __launch_bounds__(256)
-basis_kernel(const gf128* __restrict__ LO, const gf128* __restrict__ HI, int nq, int lo_bits, int hi_bits,
-             int q_per, gf128* __restrict__ out) {
-  size_t n = (size_t)1 << (lo_bits + hi_bits);
-  size_t lo_n = (size_t)1 << lo_bits, hi_n = (size_t)1 << hi_bits;
-  const int i0 = blockIdx.y * q_per, i1 = i0 + q_per < nq ? i0 + q_per : nq;
-  for (size_t j = (size_t)blockIdx.x * blockDim.x + threadIdx.x; j < n; j += (size_t)gridDim.x * blockDim.x) {
-    size_t jl = j & (lo_n - 1), jh = j >> lo_bits;
-    gf256 acc = {{0, 0, 0, 0}};
-    for (int i = i0; i < i1; i++) gf256_acc(acc, gf_mul_wide(LO[(size_t)i * lo_n + jl], HI[(size_t)i * hi_n + jh]));
-    out[(size_t)blockIdx.y * n + j] = gf256_reduce(acc);
+// The induced basis as a transposed transform. The code's position q holds
+// sum_j msg_j Xhat_j(q), so basis = E^T v for the code's encoding E (the rate
+// 2^-rate replication, then the additive NTT, ntt.cu) and the vector v with
+// alpha_i at q_i. The low lo_bits coordinates of j are expanded per query (the
+// rows LO_i of query_tensor_kernel); over the remaining pos_bits = log_d -
+// lo_bits position bits the transposed layers run from the deepest up, on LO
+// rows as lanes: a butterfly u' = u + t v, v' = v + u' transposes to s = u + v,
+// u = s, v = v + t s; last the replicas add up. That is
+// (pos_bits - rate) 2^(log_d - 1) products instead of the nq 2^n of adding
+// HI_i[j_hi] LO_i[j_lo] query by query (218 queries of 2^19 coordinates:
+// 1,153 us through byte tables rebuilt per query, 141 us here; 53 queries of
+// 2^10: 31 us in sliced products, 10 us here).
+// A CTA owns 2^log_tl lanes and all positions in shared memory, one layer
+// between two barriers. Bound by the carry-less products (ALU and multiplier
+// pipes) at large n, by the chain of pos_bits - rate dependent products at
+// small n. The loop body stays at IB_ILP products: the first pass through a
+// larger one costs more in instruction fetches than it saves (three layers
+// unrolled in registers: 25 us against 7 us at 2^9 coordinates, 138 us against
+// 141 us at 2^19).
+constexpr int IB_THREADS = 256;
+constexpr int IB_ILP = 2;
+constexpr size_t IB_MAX_SMEM = (size_t)128 << 10;
+
+// queries: sorted, distinct. tw: the plain twiddle table of 2^log_d positions
+// (its first layers do not depend on which positions a lane stands for).
+__global__ void __launch_bounds__(IB_THREADS, 2)
+induced_basis_kernel(const gf128* __restrict__ LO, const uint32_t* __restrict__ queries, int nq, int lo_bits,
+                     int pos_bits, int rate, int log_tl, const gf128* __restrict__ tw, gf128* __restrict__ basis) {
+  extern __shared__ gf128 V[];  // [position][lane]
+  const uint32_t tl_mask = (1u << log_tl) - 1, lane0 = blockIdx.x << log_tl;
+  for (uint32_t e = threadIdx.x; e < (1u << (pos_bits + log_tl)); e += IB_THREADS) V[e] = gf_zero();
+  __syncthreads();
+  // several queries may share a position block
+  for (uint32_t it = threadIdx.x; it < (uint32_t)nq << log_tl; it += IB_THREADS) {
+    const uint32_t i = it >> log_tl, lane = it & tl_mask;
+    const gf128 v = LO[((size_t)i << lo_bits) + lane0 + lane];
+    uint32_t* d = V[((queries[i] >> lo_bits) << log_tl) | lane].w;
+#pragma unroll
+    for (int k = 0; k < 4; k++) atomicXor(d + k, v.w[k]);
   }
-}
-
-// The same basis through byte tables, for large bases (LO_BITS = 10 or 11):
-// CTA h owns the 2^LO_BITS entries of high index h and walks the queries; per
-// query it builds the byte tables of HI[i][h] (one row per thread, computed
-// directly) and adds HI[i][h] LO[i][jl] for its entries (four or eight per
-// thread) as 16 table lookups each instead of a carry-less multiply. A barrier
-// before each build orders the previous query's lookups before the new
-// writes, so one table suffices; three CTAs per SM overlap one CTA's build
-// with the others' lookups.
-constexpr int BT_THREADS = 256;
-constexpr size_t BT_SMEM = (size_t)GF_TAB_ENTRIES * 16;
-static_assert(BT_THREADS == 256, "one byte-table row per thread");
-
-template <int LO_BITS>
-__global__ void __launch_bounds__(BT_THREADS, 3)
-basis_tab_kernel(const gf128* __restrict__ LO, const gf128* __restrict__ HI, int nq, int hi_bits,
-                 gf128* __restrict__ basis) {
-  constexpr int PER_THREAD = (1 << LO_BITS) / BT_THREADS;
-  extern __shared__ uint4 btab[];
-  const size_t lo_n = (size_t)1 << LO_BITS, hi_n = (size_t)1 << hi_bits;
-  const uint32_t rot = threadIdx.x & 7;
-  for (size_t h = blockIdx.x; h < hi_n; h += gridDim.x) {
-    gf128 acc[PER_THREAD];
+  __syncthreads();
+  const uint32_t items = 1u << (pos_bits - 1 + log_tl);
+#pragma unroll 1
+  for (int t = pos_bits - 1; t >= rate; t--) {
+    const int sh = pos_bits - 1 - t;
+    const gf128* twl = tw + ((1u << t) - 1);
+#pragma unroll 1
+    for (uint32_t it0 = threadIdx.x; it0 < items; it0 += IB_ILP * IB_THREADS) {
 #pragma unroll
-    for (int k = 0; k < PER_THREAD; k++) acc[k] = gf_zero();
-    for (int i = 0; i < nq; i++) {
-      __syncthreads();
-      gf_tab_row_direct(HI[(size_t)i * hi_n + h], btab, threadIdx.x);
-      __syncthreads();
-      const gf128* lo = LO + (size_t)i * lo_n + threadIdx.x;
-#pragma unroll
-      for (int k = 0; k < PER_THREAD; k++) acc[k] = gf_add(acc[k], gf_mul_tab(btab, lo[k * BT_THREADS], rot));
+      for (int k = 0; k < IB_ILP; k++) {
+        const uint32_t it = it0 + k * IB_THREADS;
+        if (it < items) {
+          const uint32_t lane = it & tl_mask, g = it >> log_tl, lo = g & ((1u << sh) - 1), hi = g >> sh;
+          const uint32_t p0 = (((hi << (sh + 1)) | lo) << log_tl) | lane, p1 = p0 + (1u << (sh + log_tl));
+          const gf128 v = V[p1], u = gf_add(V[p0], v);
+          V[p0] = u;
+          V[p1] = gf_add(v, gf_mul(u, gf_load(&twl[hi])));
+        }
+      }
     }
-    gf128* out = basis + (h << LO_BITS) + threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < PER_THREAD; k++) out[k * BT_THREADS] = acc[k];
+    __syncthreads();
+  }
+  const uint32_t out_n = 1u << (pos_bits - rate);
+  for (uint32_t e = threadIdx.x; e < out_n << log_tl; e += IB_THREADS) {
+    gf128 acc = V[e];
+    for (uint32_t c = 1; c < (1u << rate); c++) acc = gf_add(acc, V[e + ((c * out_n) << log_tl)]);
+    basis[((size_t)(e >> log_tl) << lo_bits) + lane0 + (e & tl_mask)] = acc;
   }
 }
 
@@ -294,52 +312,42 @@ int flock_launch_glue(void* b, const void* add, size_t n, const uint64_t beta[2]
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
-// byte-table path from 2^18 entries: CTAs of 2^10 entries at 2^18, of 2^11
-// above (at least 256 CTAs; 2^11 measured faster than 2^10 and 2^9 at 2^19)
-constexpr int kBasisTabMinBits = 18;
-constexpr int kBasisSlices = 8;
-size_t flock_induce_basis_scratch_bytes(int n) { return n >= kBasisTabMinBits ? 0 : ((size_t)kBasisSlices << n) * 16; }
+namespace {
+// Lanes (2^lo_bits) of the induced basis over n coordinates of a code of
+// 2^log_d positions: half the coordinates, more where the positions would not
+// fit a CTA's shared memory otherwise (two lanes of 2^12 positions).
+int induce_lo_bits(int n, int log_d) {
+  int k = (n + 1) / 2;
+  if (log_d - k > 10) k = log_d - 10;
+  if (k > TB_LO + TB_HI) k = TB_LO + TB_HI;
+  return k < n ? k : n;
+}
+}  // namespace
 
-int flock_induce_basis_lo_bits(int n) { return n >= kBasisTabMinBits ? (n == kBasisTabMinBits ? 10 : 11) : (n + 1) / 2; }
+size_t flock_induce_basis_rows_bytes(int n, int log_d, int nq) { return ((size_t)nq << induce_lo_bits(n, log_d)) * 16; }
 
-int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, const void* what_lin, const void* alpha_w,
-                              void* W, void* LO, void* HI, void* basis, void* scratch, cudaStream_t st) {
-  what_kernel<<<(unsigned)(((size_t)nq * n + 127) / 128), 128, 0, st>>>(d_queries, nq, n, (const gf128*)what_lin,
-                                                                          (gf128*)W); flock_count_launch();
-  const int lo_bits = flock_induce_basis_lo_bits(n), hi_bits = n - lo_bits;
-  const bool tab = n >= kBasisTabMinBits;
-  if (lo_bits > TB_LO + TB_HI || hi_bits > TB_LO + TB_HI) return FLOCK_ERR_SHAPE;
-  auto tgrid = [&](int bits) { return (unsigned)((size_t)nq * ((((size_t)1 << bits) + TB_THREADS - 1) / TB_THREADS)); };
-  tensor_kernel<<<tgrid(lo_bits), TB_THREADS, 0, st>>>((const gf128*)W, nq, n, 0, lo_bits, (const gf128*)alpha_w,
-                                                       (gf128*)LO); flock_count_launch();
-  tensor_kernel<<<tgrid(hi_bits), TB_THREADS, 0, st>>>((const gf128*)W, nq, n, lo_bits, hi_bits, nullptr,
-                                                       (gf128*)HI); flock_count_launch();
-  if (tab) {
-    flock_once_per_device((const void*)basis_tab_kernel<10>, [] {
-      cudaFuncSetAttribute(basis_tab_kernel<10>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BT_SMEM);
-      cudaFuncSetAttribute(basis_tab_kernel<11>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)BT_SMEM);
-    });
-    const unsigned grid = (unsigned)((size_t)1 << hi_bits);
-    if (lo_bits == 10)
-      basis_tab_kernel<10><<<grid, BT_THREADS, BT_SMEM, st>>>((const gf128*)LO, (const gf128*)HI, nq, hi_bits,
-                                                              (gf128*)basis);
-    else
-      basis_tab_kernel<11><<<grid, BT_THREADS, BT_SMEM, st>>>((const gf128*)LO, (const gf128*)HI, nq, hi_bits,
-                                                              (gf128*)basis);
-  } else {
-    // slices of the query sum: about 2^18 threads in all, at most kBasisSlices
-    // (one thread per entry ran 106 dependent products at 2^16 entries)
-    int slices = 1;
-    while (slices < kBasisSlices && ((size_t)slices << n) < ((size_t)1 << 18) && slices < nq) slices *= 2;
-    const int q_per = (nq + slices - 1) / slices;
-    const dim3 grid(grid_for((size_t)1 << n, 256, 152 * 8), slices);
-    basis_kernel<<<grid, 256, 0, st>>>((const gf128*)LO, (const gf128*)HI, nq, lo_bits, hi_bits, q_per,
-                                       (gf128*)(slices > 1 ? scratch : basis));
-    flock_count_launch();
-    if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
-    if (slices > 1) return flock_launch_reduce_rows(scratch, slices, 1 << n, basis, st);
-    return FLOCK_OK;
-  }
+int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, int log_d, const void* what_lin,
+                              const void* alpha_w, void* LO, void* basis, cudaStream_t st) {
+  const int lo_bits = induce_lo_bits(n, log_d), pos_bits = log_d - lo_bits, rate = log_d - n;
+  if (nq < 1 || n < 1 || rate < 0 || log_d > 30) return FLOCK_ERR_SHAPE;
+  // lanes per CTA: up to four (64-byte runs of LO and basis rows) while the
+  // grid keeps two CTAs per SM and the positions fit
+  int log_tl = 0;
+  while (log_tl < 2 && log_tl < lo_bits && ((size_t)1 << (lo_bits - log_tl - 1)) >= 256) log_tl++;
+  while (log_tl > 0 && ((size_t)16 << (pos_bits + log_tl)) > IB_MAX_SMEM) log_tl--;
+  const size_t smem = (size_t)16 << (pos_bits + log_tl);
+  if (smem > IB_MAX_SMEM) return FLOCK_ERR_SHAPE;
+  const void* tw = flock_ntt_twiddles(log_d);
+  if (!tw) return FLOCK_ERR_OOM;
+  const size_t chunks = (((size_t)1 << lo_bits) + TB_THREADS - 1) / TB_THREADS;
+  query_tensor_kernel<<<(unsigned)((size_t)nq * chunks), TB_THREADS, 0, st>>>(
+      d_queries, lo_bits, (const gf128*)what_lin, (const gf128*)alpha_w, (gf128*)LO);
+  flock_count_launch();
+  flock_once_per_device((const void*)induced_basis_kernel, [] {
+    cudaFuncSetAttribute(induced_basis_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)IB_MAX_SMEM);
+  });
+  induced_basis_kernel<<<1u << (lo_bits - log_tl), IB_THREADS, smem, st>>>(
+      (const gf128*)LO, d_queries, nq, lo_bits, pos_bits, rate, log_tl, (const gf128*)tw, (gf128*)basis);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }

@@ -302,7 +302,7 @@ struct ProverState {
   cudaStream_t st_normal = nullptr, st_high = nullptr;
   ZcRound1Tables* d_r1t = nullptr;
   DBuf in, z, a, b, stripe, cw, tree, A0, B0, A1, B1, eqlo, eqhi, eqout, rdev, part, red, lag, small, eqin, comb,
-      zvec, zvec0, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, W, LO, HI, basis, qbuf, abuf, rows, nidx, nodes,
+      zvec, zvec0, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, LO, basis, qbuf, abuf, rows, nidx, nodes,
       grind, lvl_cw[2], lvl_tree[2], chW, chG, zceq, zcr, zcjobs;
   DBuf csc_ap, csc_ai, csc_bp, csc_bi;
   bool csc_ready = false;
@@ -336,7 +336,7 @@ struct ProverState {
   std::vector<DBuf*> bufs() {
     std::vector<DBuf*> v = {&in, &z, &a, &b, &stripe, &cw, &tree, &A0, &B0, &A1, &B1, &eqlo, &eqhi, &eqout, &rdev, &part, &red,
             &lag, &small, &eqin, &comb, &zvec, &zvec0, &tlo0, &thi0, &tlo1, &thi1, &tables, &bc, &f1, &b1,
-            &W, &LO, &HI, &basis, &qbuf, &abuf, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
+            &LO, &basis, &qbuf, &abuf, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
             &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &zcr, &zcjobs, &csc_ap, &csc_ai, &csc_bp, &csc_bi};
     for (DBuf& d : skl) v.push_back(&d);
     return v;
@@ -1254,7 +1254,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         FK(flock_launch_glue_eq(bcur, len, S->eqlo.p, S->eqhi.p, lob, bp, st));
       }
     };
-    auto induce = [&](int nvars, const std::vector<uint32_t>& q, const std::vector<F>& alpha_v) {
+    auto induce = [&](int nvars, size_t block_len, const std::vector<uint32_t>& q, const std::vector<F>& alpha_v) {
       const Sks& sk = sks_for(nvars);
       auto aw = eq_table(alpha_v);
       aw.resize(q.size());
@@ -1269,14 +1269,10 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       h2d(*S, dq, q.data(), q.size() * 4);
       void* dal = S->abuf.get(q.size() * 16);
       h2d(*S, dal, aw.data(), q.size() * 16);
-      int lo_bits = flock_induce_basis_lo_bits(nvars), hi_bits = nvars - lo_bits;
-      void* dW = S->W.get(q.size() * nvars * 16);
-      void* dLO = S->LO.get((q.size() << lo_bits) * 16);
-      void* dHI = S->HI.get((q.size() << hi_bits) * 16);
+      const int log_d = ilog2(block_len);
+      void* dLO = S->LO.get(flock_induce_basis_rows_bytes(nvars, log_d, (int)q.size()));
       void* dbs = S->basis.get(((size_t)16) << nvars);
-      const size_t scr = flock_induce_basis_scratch_bytes(nvars);
-      FK(flock_launch_induce_basis(dq, (int)q.size(), nvars, dsk, dal, dW, dLO, dHI, dbs,
-                                   scr ? S->part.get(scr) : nullptr, st));
+      FK(flock_launch_induce_basis(dq, (int)q.size(), nvars, log_d, dsk, dal, dLO, dbs, st));
       return dbs;
     };
 
@@ -1313,7 +1309,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     auto a0 = tr.sample_vec(ilog2(cfg.queries[0]));
     // the induced basis needs the queries only: its kernels are queued first
     // and run while the host prepares the opening (multiproof indices)
-    void* dbs0 = induce(n1, q0, a0);
+    void* dbs0 = induce(n1, block0, q0, a0);
     Open open0 = open_rows(*S, dcw, dtree, block0, 1 << lbs, q0);
     introduce(dbs0);
     std::vector<Open> rec_opens;
@@ -1350,7 +1346,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       grind_nonces.push_back(grind((uint32_t)cfg.grind_bits[i + 1]));
       auto qi = sample_queries(tr, prev_block, cfg.queries[i + 1]);
       auto ai = tr.sample_vec(ilog2(cfg.queries[i + 1]));
-      void* dbs = induce(n_next, qi, ai);
+      void* dbs = induce(n_next, prev_block, qi, ai);
       rec_opens.push_back(open_rows(*S, S->lvl_cw[slot].p, S->lvl_tree[slot].p, prev_block, prev_width, qi));
       introduce(dbs);
       slot = ns;
