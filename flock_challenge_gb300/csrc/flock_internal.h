@@ -45,6 +45,15 @@ int flock_launch_eq_split_multi(const FlockEqJob* d_jobs, int n_jobs, size_t max
 int flock_launch_zc_round(const void* A, const void* B, size_t n_pairs, int bind, const uint64_t rho[2], void* Aout,
                           void* Bout, const void* eq_lo, const void* eq_hi, int lo_bits, void* partials, int grid,
                           cudaStream_t st);
+// A small round (n_pairs <= FLOCK_ZC_SMALL_PAIRS): skip != 0
+// is round 0 from the bit rows, otherwise the 2 n_pairs entry pairs are bound at
+// rho; eq: n_pairs entries, eq_next: n_pairs / 2 entries written for the next
+// round. flock_zc_small_grid(n_pairs) rows of partials.
+constexpr size_t FLOCK_ZC_SMALL_PAIRS = (size_t)1 << 17;
+int flock_zc_small_grid(size_t n_pairs);
+int flock_launch_zc_round_small(const void* in0, const void* in1, size_t n_pairs, int skip, const uint64_t rho[2],
+                                const void* lag, void* Aout, void* Bout, const void* eq, void* eq_next,
+                                void* partials, cudaStream_t st);
 int flock_launch_bind_pairs(const void* A, const void* B, size_t n, const uint64_t rho[2], void* Aout, void* Bout,
                             cudaStream_t st);
 

@@ -248,3 +248,76 @@ __device__ __forceinline__ gf128p gf_load_p(const gf128p* q) {
   for (int i = 0; i < 9; i++) p.m[i] = q->m[i];
   return p;
 }
+
+// ---- small sumcheck rounds --------------------------------------------------
+// A round of few pairs is bound by one thread's chain of products and by
+// fetching its code, so two neighbouring lanes share a pair, one product each
+// per step, and the steps run through one loop body (unrolled, a pair's six or
+// eight products are up to 50 KB of instructions, which a launch of a few warps
+// waits for).
+__device__ __forceinline__ gf128 gf_shfl_xor(gf128 a, int m) {
+#pragma unroll
+  for (int k = 0; k < 4; k++) a.w[k] = __shfl_xor_sync(0xffffffffu, a.w[k], m);
+  return a;
+}
+
+// Lane h = threadIdx.x & 1 of a pair holds value h of the pair in both tables:
+// a0 (and a1, with bind: the value is a0 + r (a0 + a1), left in a0), the same for b.
+// Returns the lane's message product, a_h b_h on lane h = 1 - SUM_LANE and
+// (a_0 + a_1) (b_0 + b_1) on lane SUM_LANE, times e where WEIGHT. All lanes call it.
+template <bool WEIGHT, int SUM_LANE>
+__device__ __forceinline__ gf128 gf_round_small(gf128& a0, gf128 a1, gf128& b0, gf128 b1, bool bind, gf128 r,
+                                                gf128 e) {
+  gf128 p = gf_zero();
+#pragma unroll 1
+  for (int s = bind ? 0 : 2; s < (WEIGHT ? 4 : 3); s++) {
+    gf128 x, y = r;
+    if (s == 0) {
+      x = gf_add(a0, a1);
+    } else if (s == 1) {
+      x = gf_add(b0, b1);
+    } else if (s == 2) {
+      x = a0;
+      y = b0;
+      const gf128 ao = gf_shfl_xor(a0, 1), bo = gf_shfl_xor(b0, 1);
+      if ((threadIdx.x & 1) == SUM_LANE) {
+        x = gf_add(x, ao);
+        y = gf_add(y, bo);
+      }
+    } else {
+      x = p;
+      y = e;
+    }
+    const gf128 q = gf_mul(x, y);
+    if (s == 0) a0 = gf_add(a0, q);
+    else if (s == 1) b0 = gf_add(b0, q);
+    else p = q;
+  }
+  return p;
+}
+
+// XOR of p over a block's even threads into out[even_to] and over its odd
+// threads into out[1 - even_to]; at most 256 threads, all call it.
+__device__ __forceinline__ void gf_block_sum_lanes(gf128 p, int even_to, gf128* __restrict__ out) {
+  __shared__ gf128 red[8][2];
+#pragma unroll
+  for (int off = 16; off > 1; off >>= 1) p = gf_add(p, gf_shfl_xor(p, off));
+  const int lane = threadIdx.x & 31;
+  if (lane < 2) red[threadIdx.x >> 5][lane] = p;
+  __syncthreads();
+  if (threadIdx.x < 2) {
+    gf128 v = red[0][threadIdx.x];
+    for (int k = 1; k < (int)(blockDim.x >> 5); k++) v = gf_add(v, red[k][threadIdx.x]);
+    out[threadIdx.x ^ even_to] = v;
+  }
+}
+
+// Threads per block of a small round over n_pairs pairs (two lanes a pair):
+// blocks of two warps spread a round over the SMs while that makes at most 256
+// rows of partial sums, blocks of eight beyond.
+__host__ __device__ inline int gf_small_threads(size_t n_pairs) { return n_pairs <= ((size_t)1 << 13) ? 64 : 256; }
+__host__ __device__ inline int gf_small_grid(size_t n_pairs) {
+  const size_t per = gf_small_threads(n_pairs) / 2;
+  const size_t g = (n_pairs + per - 1) / per;
+  return (int)(g < 1 ? 1 : g);
+}

@@ -785,7 +785,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     // are built by one launch before the first round (no eq work between a
     // round's kernel and the host's read of its message).
     struct RoundEq {
-      bool grp;
+      bool grp, small;
       int a_bits, m_bits, f0, lob;
       F dinv;
       std::vector<F> vars;  // the variables of the split tables
@@ -799,7 +799,8 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       q.a_bits = std::max(0, 2 - i);
       q.f0 = std::max(9, 7 + i);
       q.m_bits = std::max(0, 13 - q.f0);
-      q.grp = q.m_bits > 0 && nv > q.a_bits + q.m_bits;
+      q.small = ((size_t)1 << nv) <= FLOCK_ZC_SMALL_PAIRS;  // 2^nv pairs
+      q.grp = !q.small && q.m_bits > 0 && nv > q.a_bits + q.m_bits;
       for (int k = q.f0; q.grp && k < 13; k++) q.grp = shift_var(k);
       q.dinv = F::one();
       if (q.grp) {
@@ -808,6 +809,9 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         rg.insert(rg.end(), rr.begin() + q.a_bits + q.m_bits, rr.end());
         q.lob = std::min(nv - q.m_bits, 8);
         q.vars = std::move(rg);
+      } else if (q.small) {
+        q.lob = nv;  // one table over all variables
+        q.vars = std::move(rr);
       } else {
         // a CTA takes whole rows of 2^lob pairs: rows of 2^(nv - 10) pairs,
         // at least 2^8 (one pair per thread) and at most 2^12, keep the grid
@@ -838,13 +842,15 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       F* dvars = (F*)S->zcr.get(vars.size() * 16 + 16);
       h2d(*S, dvars, vars.data(), vars.size() * 16);
       F* deq = (F*)S->zceq.get(tot * 16);
-      std::vector<FlockEqJob> jobs(n_mlv);
+      // a small round's table comes out of the small round before it
+      std::vector<FlockEqJob> jobs;
       for (int i = 0; i < n_mlv; i++)
-        jobs[i] = {dvars + var_off[i], deq + eq_off[i].first, deq + eq_off[i].second, qs[i].lob,
-                   (int)qs[i].vars.size() - qs[i].lob};
+        if (i == 0 || !qs[i].small || !qs[i - 1].small)
+          jobs.push_back({dvars + var_off[i], deq + eq_off[i].first, deq + eq_off[i].second, qs[i].lob,
+                          (int)qs[i].vars.size() - qs[i].lob});
       auto* djobs = (FlockEqJob*)S->zcjobs.get(jobs.size() * sizeof(FlockEqJob));
       h2d(*S, djobs, jobs.data(), jobs.size() * sizeof(FlockEqJob));
-      FK(flock_launch_eq_split_multi(djobs, n_mlv, max_entries, st));
+      FK(flock_launch_eq_split_multi(djobs, (int)jobs.size(), max_entries, st));
     }
     // The last rounds, from kHostTailPairs pairs down, run on the host: a GPU
     // round of a few hundred pairs is a latency-bound launch plus a round
@@ -867,6 +873,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         FK(flock_launch_zc_round_grp(i == 0 ? da : curA, i == 0 ? db : curB, n_pairs, i == 0, rp, dlag,
                                      i == 0 ? dA0 : nxtA, i == 0 ? dB0 : nxtB, elo, ehi, q.lob, q.a_bits, q.m_bits,
                                      1 << (q.f0 - 9), dpart, grid, st));
+      } else if (q.small) {
+        grid = flock_zc_small_grid(n_pairs);
+        dpart = part_buf(*S, (size_t)grid * 2 * 16);
+        FK(flock_launch_zc_round_small(i == 0 ? da : curA, i == 0 ? db : curB, n_pairs, i == 0, rp, dlag,
+                                       i == 0 ? dA0 : nxtA, i == 0 ? dB0 : nxtB, elo,
+                                       (F*)S->zceq.p + eq_off[std::min(i + 1, n_mlv - 1)].first, dpart, st));
       } else {
         grid = (int)std::max<size_t>(std::min<size_t>(n_pairs >> q.lob, 152 * 4), 1);
         dpart = part_buf(*S, (size_t)grid * 2 * 16);

@@ -444,43 +444,72 @@ reduce_rows_kernel(const gf128* __restrict__ in, size_t count, int width, gf128*
 // eq table split: lo[i] = prod_{k<lo_bits} f(r_k, bit k of i), hi[i] over the
 // next hi_bits variables; f(r, 1) = r, f(r, 0) = 1 + r. Each CTA first builds
 // the eq tables of 7-bit chunks of the variables in shared memory (at most
-// 4 x 128 entries per set), so an entry costs (chunks - 1) products instead
-// of one per variable.
-constexpr int EQ_CHUNK = 7, EQ_MAX_CHUNKS = 4;
+// 4 x 128 entries per set), a chunk's from those of its low four and high three
+// variables, so an entry costs (chunks - 1) products instead of one per
+// variable. Bound by the chain of products (three, one or two, chunks - 1) up
+// to some 2^16 entries (13 + 1 variables: 18 us with up to seven products a
+// chunk entry and eight entries a thread, 7.4 us here), by the products beyond.
+constexpr int EQ_CHUNK = 7, EQ_MAX_CHUNKS = 4, EQ_HALF = 4;
 // One table pair, CTA `blk` of `nblk` (the calling kernel's grid slice).
 __device__ __forceinline__ void eq_split_body(const gf128* __restrict__ r, int lo_bits, int hi_bits,
                                               gf128* __restrict__ lo, gf128* __restrict__ hi, size_t blk,
                                               size_t nblk) {
-  __shared__ gf128 t[2][EQ_MAX_CHUNKS][1 << EQ_CHUNK];
-  for (int e = threadIdx.x; e < 2 * EQ_MAX_CHUNKS * (1 << EQ_CHUNK); e += blockDim.x) {
-    const int set = e / (EQ_MAX_CHUNKS << EQ_CHUNK), c = (e >> EQ_CHUNK) % EQ_MAX_CHUNKS, v = e & ((1 << EQ_CHUNK) - 1);
-    const int nb = set ? hi_bits : lo_bits;
-    const gf128* rr = (set ? r + lo_bits : r) + EQ_CHUNK * c;
-    const int cb = nb - EQ_CHUNK * c < EQ_CHUNK ? nb - EQ_CHUNK * c : EQ_CHUNK;
-    if (cb <= 0 || v >= (1 << cb)) continue;
+  __shared__ gf128 half_t[2 * EQ_MAX_CHUNKS][2][1 << EQ_HALF];
+  __shared__ gf128 t[2 * EQ_MAX_CHUNKS][1 << EQ_CHUNK];
+  const int nc_lo = (lo_bits + EQ_CHUNK - 1) / EQ_CHUNK, nc = nc_lo + (hi_bits + EQ_CHUNK - 1) / EQ_CHUNK;
+  // chunk c of both sets: its first variable and number of variables
+  auto chunk = [&](int c, int& v0, int& nv) {
+    const bool is_lo = c < nc_lo;
+    const int k = EQ_CHUNK * (is_lo ? c : c - nc_lo), left = (is_lo ? lo_bits : hi_bits) - k;
+    v0 = (is_lo ? 0 : lo_bits) + k;
+    nv = left < EQ_CHUNK ? left : EQ_CHUNK;
+  };
+  for (int e = threadIdx.x; e < nc << (EQ_HALF + 1); e += blockDim.x) {
+    const int c = e >> (EQ_HALF + 1), h = (e >> EQ_HALF) & 1, v = e & ((1 << EQ_HALF) - 1);
+    int v0, nv;
+    chunk(c, v0, nv);
+    const int hv = h ? nv - EQ_HALF : nv < EQ_HALF ? nv : EQ_HALF;
+    if (v >= 1 << (hv > 0 ? hv : 0)) continue;
     gf128 acc = gf_one();
-    for (int k = 0; k < cb; k++) {
-      gf128 rk = rr[k];
+#pragma unroll 1
+    for (int k = 0; k < hv; k++) {
+      gf128 rk = gf_load(&r[v0 + (h ? EQ_HALF : 0) + k]);
       if (!((v >> k) & 1)) rk.w[0] ^= 1;
-      acc = gf_mul(acc, rk);
+      acc = k == 0 ? rk : gf_mul(acc, rk);
     }
-    t[set][c][v] = acc;
+    half_t[c][h][v] = acc;
+  }
+  __syncthreads();
+#pragma unroll 1
+  for (int e = threadIdx.x; e < nc << EQ_CHUNK; e += blockDim.x) {
+    const int c = e >> EQ_CHUNK, v = e & ((1 << EQ_CHUNK) - 1);
+    int v0, nv;
+    chunk(c, v0, nv);
+    if (v < 1 << nv)
+      t[c][v] = nv > EQ_HALF ? gf_mul(half_t[c][0][v & ((1 << EQ_HALF) - 1)], half_t[c][1][v >> EQ_HALF])
+                             : half_t[c][0][v];
   }
   __syncthreads();
   const size_t nlo = (size_t)1 << lo_bits, nhi = (size_t)1 << hi_bits;
+#pragma unroll 1
   for (size_t e = blk * blockDim.x + threadIdx.x; e < nlo + nhi; e += nblk * blockDim.x) {
     const bool is_lo = e < nlo;
     const size_t idx = is_lo ? e : e - nlo;
-    const int set = is_lo ? 0 : 1, nb = is_lo ? lo_bits : hi_bits;
-    const int nch = (nb + EQ_CHUNK - 1) / EQ_CHUNK;
-    gf128 acc = gf_one();
-    for (int c = 0; c < nch; c++) {
-      const gf128 f = t[set][c][(idx >> (EQ_CHUNK * c)) & ((1 << EQ_CHUNK) - 1)];
-      acc = c == 0 ? f : gf_mul(acc, f);
-    }
+    const int c0 = is_lo ? 0 : nc_lo, c1 = is_lo ? nc_lo : nc;
+    gf128 acc = c0 < c1 ? t[c0][idx & ((1 << EQ_CHUNK) - 1)] : gf_one();
+#pragma unroll 1
+    for (int c = c0 + 1; c < c1; c++)
+      acc = gf_mul(acc, t[c][(idx >> (EQ_CHUNK * (c - c0))) & ((1 << EQ_CHUNK) - 1)]);
     if (is_lo) lo[idx] = acc;
     else hi[idx] = acc;
   }
+}
+
+// CTAs of a table pair of n entries: one entry per thread up to two CTAs per
+// SM (more entries a thread above: the chunk tables are built per CTA).
+size_t eq_grid(size_t n) {
+  const size_t g = (n + 255) / 256;
+  return g < 1 ? 1 : g > 304 ? 304 : g;
 }
 
 __global__ void __launch_bounds__(256)
@@ -762,6 +791,78 @@ zc_round_grp_kernel(const void* __restrict__ in0, const void* __restrict__ in1, 
   block_reduce2(g1, gi, partials);
 }
 
+// Small rounds (at most FLOCK_ZC_SMALL_PAIRS pairs): bound by one thread's
+// chain (loads, products four deep, the block's sum), not by throughput. Two
+// lanes take a pair (gf_round_small), and the eq table is expanded over all
+// variables, so nothing is multiplied after the block's sum. The table of the
+// next round (one variable fewer) is the sums of this one's neighbours, as
+// eq's two factors add up to one: one lane of each second pair writes it.
+// Rounds 0..5 of 2^8 compressions (2^15..2^10 pairs) through
+// zc_round_grp_kernel: 260 us, here 41 us; 2^10 pairs through zc_round_kernel:
+// 18 us, here 5.7 us; 2^17 pairs: 40 us and 30 us (beyond, the table products
+// of the other kernels win).
+constexpr int SR_MAX_THREADS = 256;
+template <bool SKIP>
+__global__ void __launch_bounds__(SR_MAX_THREADS)
+zc_round_small_kernel(const void* __restrict__ in0, const void* __restrict__ in1, size_t n_pairs, const gf128 rho,
+                      const gf128* __restrict__ lag, gf128* __restrict__ Aout, gf128* __restrict__ Bout,
+                      const gf128* __restrict__ eq, gf128* __restrict__ eq_next, gf128* __restrict__ partials) {
+  extern __shared__ gf128 tab[];  // SKIP: subset sums of the Lagrange weights, as in zc_round_grp_kernel
+  const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x, j = i >> 1;  // value i & 1 of pair j
+  const bool act = j < n_pairs;
+  gf128 a0 = gf_zero(), a1 = a0, b0 = a0, b1 = a0, e = a0;
+  if (act) {
+    e = gf_load(&eq[j]);
+    if (i < n_pairs / 2) eq_next[i] = gf_add(gf_load(&eq[2 * i]), gf_load(&eq[2 * i + 1]));
+  }
+  if constexpr (SKIP) {
+    uint64_t w[2] = {0, 0};
+    if (act) {
+      w[0] = reinterpret_cast<const uint64_t*>(in0)[i];
+      w[1] = reinterpret_cast<const uint64_t*>(in1)[i];
+    }
+    // item: byte position c = item & 7, entries v = 16 (item >> 3) .. + 15 by a Gray walk
+    for (int it = threadIdx.x; it < 128; it += blockDim.x) {
+      const int c = it & 7, g = it >> 3;
+      gf128 v = gf_zero();
+#pragma unroll
+      for (int k = 4; k < 8; k++)
+        if ((g >> (k - 4)) & 1) v = gf_add(v, gf_load(&lag[8 * c + k]));
+      const gf128 l[4] = {gf_load(&lag[8 * c]), gf_load(&lag[8 * c + 1]), gf_load(&lag[8 * c + 2]),
+                          gf_load(&lag[8 * c + 3])};
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        if (k) v = gf_add(v, l[gf_tab_ctz4(k)]);
+        tab[((16 * g + (k ^ (k >> 1))) << 3) + c] = v;
+      }
+    }
+    __syncthreads();
+    gf128 f[2];
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      gf128 r = gf_zero();
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const int c = (threadIdx.x + k) & 7;
+        r = gf_add(r, tab[((((uint32_t)(w[q] >> (8 * c))) & 255) << 3) + c]);
+      }
+      f[q] = r;
+    }
+    a0 = f[0];
+    b0 = f[1];
+  } else if (act) {
+    const gf128 *A = reinterpret_cast<const gf128*>(in0) + 2 * i, *B = reinterpret_cast<const gf128*>(in1) + 2 * i;
+    a0 = gf_load(A); a1 = gf_load(A + 1);
+    b0 = gf_load(B); b1 = gf_load(B + 1);
+  }
+  const gf128 p = gf_round_small<true, 0>(a0, a1, b0, b1, !SKIP, rho, e);
+  if (act) {
+    Aout[i] = a0;
+    Bout[i] = b0;
+  }
+  gf_block_sum_lanes(p, 1, partials + 2 * blockIdx.x);  // G(1) from the odd lanes, G(inf) from the even ones
+}
+
 // Final bind of the last round: out[j] = A0 + rho (A0 + A1).
 __global__ void bind_pairs_kernel(const gf128* __restrict__ A, const gf128* __restrict__ B, size_t n, gf128 rho,
                                   gf128* __restrict__ Aout, gf128* __restrict__ Bout) {
@@ -803,9 +904,7 @@ int flock_launch_reduce_rows(const void* in, size_t count, int width, void* out,
 int flock_launch_eq_split_multi(const FlockEqJob* d_jobs, int n_jobs, size_t max_entries, cudaStream_t st) {
   if (n_jobs <= 0) return FLOCK_OK;
   if (n_jobs > 65535) return FLOCK_ERR_SHAPE;
-  size_t gx = (max_entries + 2047) / 2048;  // >= 8 entries per thread, as in flock_launch_eq_split
-  if (gx < 1) gx = 1;
-  if (gx > 152) gx = 152;
+  const size_t gx = eq_grid(max_entries);
   eq_split_multi_kernel<<<dim3((unsigned)gx, (unsigned)n_jobs), 256, 0, st>>>(d_jobs); flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
@@ -813,9 +912,7 @@ int flock_launch_eq_split_multi(const FlockEqJob* d_jobs, int n_jobs, size_t max
 int flock_launch_eq_split(const void* r, int lo_bits, int hi_bits, void* lo, void* hi, cudaStream_t st) {
   if (lo_bits < 0 || hi_bits < 0 || lo_bits > EQ_CHUNK * EQ_MAX_CHUNKS || hi_bits > EQ_CHUNK * EQ_MAX_CHUNKS)
     return FLOCK_ERR_SHAPE;
-  size_t n = ((size_t)1 << lo_bits) + ((size_t)1 << hi_bits);
-  size_t grid = (n + 2047) / 2048;  // >= 8 entries per thread: the chunk tables are built per CTA
-  if (grid > 152) grid = 152;
+  const size_t grid = eq_grid(((size_t)1 << lo_bits) + ((size_t)1 << hi_bits));
   eq_split_kernel<<<(unsigned)grid, 256, 0, st>>>((const gf128*)r, lo_bits, hi_bits, (gf128*)lo, (gf128*)hi); flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
@@ -871,6 +968,27 @@ int flock_launch_zc_round_grp(const void* in0, const void* in1, size_t n_pairs, 
     zc_round_grp_kernel<false><<<grid, RND_THREADS, kTabSmem, st>>>(
         in0, in1, n_pairs, r, (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)eq_lo,
         (const gf128*)eq_hi, lo_bits, a_bits, m_bits, m_mul, (gf128*)partials);
+  flock_count_launch();
+  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+}
+
+int flock_zc_small_grid(size_t n_pairs) { return gf_small_grid(n_pairs); }
+
+int flock_launch_zc_round_small(const void* in0, const void* in1, size_t n_pairs, int skip, const uint64_t rho[2],
+                                const void* lag, void* Aout, void* Bout, const void* eq, void* eq_next,
+                                void* partials, cudaStream_t st) {
+  if (n_pairs < 1 || n_pairs > FLOCK_ZC_SMALL_PAIRS) return FLOCK_ERR_SHAPE;
+  gf128 r;
+  r.w[0] = (uint32_t)rho[0]; r.w[1] = (uint32_t)(rho[0] >> 32); r.w[2] = (uint32_t)rho[1]; r.w[3] = (uint32_t)(rho[1] >> 32);
+  const int grid = gf_small_grid(n_pairs), threads = gf_small_threads(n_pairs);
+  if (skip)
+    zc_round_small_kernel<true><<<grid, threads, 8 * 256 * sizeof(gf128), st>>>(
+        in0, in1, n_pairs, r, (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)eq, (gf128*)eq_next,
+        (gf128*)partials);
+  else
+    zc_round_small_kernel<false><<<grid, threads, 0, st>>>(
+        in0, in1, n_pairs, r, (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)eq, (gf128*)eq_next,
+        (gf128*)partials);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
