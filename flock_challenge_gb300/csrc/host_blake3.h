@@ -3,6 +3,7 @@
 // root output is extendable (XOF). Matches the device compression in
 // blake3.cuh word for word.
 #pragma once
+#include <array>
 #include <cstdint>
 #include <cstring>
 #include <vector>
@@ -13,40 +14,55 @@ static constexpr uint32_t IV[8] = {0x6a09e667, 0xbb67ae85, 0x3c6ef372, 0xa54ff53
                                    0x510e527f, 0x9b05688c, 0x1f83d9ab, 0x5be0cd19};
 enum : uint32_t { CHUNK_START = 1, CHUNK_END = 2, PARENT = 4, ROOT = 8 };
 
-inline uint32_t rotr(uint32_t x, int n) { return (x >> n) | (x << (32 - n)); }
+// The message word that column/diagonal step i of round r takes: the BLAKE3
+// permutation applied r times.
+constexpr int kPerm[16] = {2, 6, 3, 10, 7, 0, 4, 13, 1, 11, 12, 5, 9, 14, 15, 8};
+constexpr int msg_index(int r, int i) { return r == 0 ? i : msg_index(r - 1, kPerm[i]); }
 
-inline void compress(const uint32_t cv[8], const uint32_t m_in[16], uint64_t ctr, uint32_t len, uint32_t flags,
-                     uint32_t out[16]) {
-  static const int P[16] = {2, 6, 3, 10, 7, 0, 4, 13, 1, 11, 12, 5, 9, 14, 15, 8};
-  uint32_t v[16] = {cv[0], cv[1], cv[2], cv[3], cv[4], cv[5], cv[6], cv[7],
-                    IV[0], IV[1], IV[2], IV[3], (uint32_t)ctr, (uint32_t)(ctr >> 32), len, flags};
-  uint32_t m[16];
-  memcpy(m, m_in, 64);
-  auto g = [&](int a, int b, int c, int d, uint32_t x, uint32_t y) {
-    v[a] += v[b] + x; v[d] = rotr(v[d] ^ v[a], 16);
-    v[c] += v[d];     v[b] = rotr(v[b] ^ v[c], 12);
-    v[a] += v[b] + y; v[d] = rotr(v[d] ^ v[a], 8);
-    v[c] += v[d];     v[b] = rotr(v[b] ^ v[c], 7);
-  };
-  for (int r = 0; r < 7; r++) {
-    g(0, 4, 8, 12, m[0], m[1]); g(1, 5, 9, 13, m[2], m[3]);
-    g(2, 6, 10, 14, m[4], m[5]); g(3, 7, 11, 15, m[6], m[7]);
-    g(0, 5, 10, 15, m[8], m[9]); g(1, 6, 11, 12, m[10], m[11]);
-    g(2, 7, 8, 13, m[12], m[13]); g(3, 4, 9, 14, m[14], m[15]);
-    uint32_t t[16];
-    for (int i = 0; i < 16; i++) t[i] = m[P[i]];
-    memcpy(m, t, 64);
-  }
-  for (int i = 0; i < 8; i++) {
-    out[i] = v[i] ^ v[i + 8];
-    out[i + 8] = v[i + 8] ^ cv[i];
-  }
+// One round with its message order fixed at compile time: the sixteen state
+// words stay in registers and the schedule costs no moves (a transcript's
+// samples are chains of compressions: 650 ns a sample with the message permuted
+// in memory every round, 350 ns so, 75 ns a compression, on a Grace core).
+template <int R, class W>
+inline __attribute__((always_inline)) void round_fn(W v[16], const W* m) {
+#define HB3_G(a, b, c, d, i)                                                             \
+  v[a] += v[b] + m[msg_index(R, i)];     v[d] ^= v[a]; v[d] = (v[d] >> 16) | (v[d] << 16); \
+  v[c] += v[d];                          v[b] ^= v[c]; v[b] = (v[b] >> 12) | (v[b] << 20); \
+  v[a] += v[b] + m[msg_index(R, i + 1)]; v[d] ^= v[a]; v[d] = (v[d] >> 8) | (v[d] << 24);  \
+  v[c] += v[d];                          v[b] ^= v[c]; v[b] = (v[b] >> 7) | (v[b] << 25);
+  HB3_G(0, 4, 8, 12, 0)
+  HB3_G(1, 5, 9, 13, 2)
+  HB3_G(2, 6, 10, 14, 4)
+  HB3_G(3, 7, 11, 15, 6)
+  HB3_G(0, 5, 10, 15, 8)
+  HB3_G(1, 6, 11, 12, 10)
+  HB3_G(2, 7, 8, 13, 12)
+  HB3_G(3, 4, 9, 14, 14)
+#undef HB3_G
+}
+template <class W>
+inline __attribute__((always_inline)) void rounds(W v[16], const W* m) {
+  round_fn<0>(v, m);
+  round_fn<1>(v, m);
+  round_fn<2>(v, m);
+  round_fn<3>(v, m);
+  round_fn<4>(v, m);
+  round_fn<5>(v, m);
+  round_fn<6>(v, m);
 }
 
-inline void load_words(const uint8_t* b, size_t n, uint32_t w[16]) {
-  uint8_t t[64] = {0};
-  memcpy(t, b, n);
-  for (int i = 0; i < 16; i++) w[i] = t[4 * i] | (t[4 * i + 1] << 8) | (t[4 * i + 2] << 16) | ((uint32_t)t[4 * i + 3] << 24);
+// (host_hash.cpp, so that the host compiler alone sees the unrolled rounds)
+void compress(const uint32_t cv[8], const uint32_t m[16], uint64_t ctr, uint32_t len, uint32_t flags,
+              uint32_t out[16]);
+
+// Eight independent chaining values at a time, one per vector lane, with a
+// zero counter: cv[k] = compress(cv[k], block k of 64 bytes at p[k], len, flags)
+// (Merkle leaves and parents of one level; 51 ns each on a Grace core).
+void compress_lanes8(uint32_t cv[8][8], const uint8_t* const p[8], uint32_t len, uint32_t flags);
+
+inline void load_words(const uint8_t* b, size_t n, uint32_t w[16]) {  // little-endian hosts
+  if (n < 64) memset(w, 0, 64);
+  memcpy(w, b, n);
 }
 
 class Hasher {
@@ -98,14 +114,15 @@ class Hasher {
     uint32_t w[16], o[16];
     load_words(buf_, 64, w);
     compress(cv_, w, chunk_, 64, CHUNK_END, o);
-    std::vector<uint32_t> ncv(o, o + 8);
+    std::array<uint32_t, 8> ncv;
+    memcpy(ncv.data(), o, 32);
     for (uint64_t total = chunk_ + 1; (total & 1) == 0; total >>= 1) {
       uint32_t blk[16];
       memcpy(blk, stack_.back().data(), 32);
       memcpy(blk + 8, ncv.data(), 32);
       stack_.pop_back();
       compress(IV, blk, 0, 64, PARENT, o);
-      ncv.assign(o, o + 8);
+      memcpy(ncv.data(), o, 32);
     }
     stack_.push_back(ncv);
     chunk_++;
@@ -139,7 +156,7 @@ class Hasher {
   uint8_t buf_[64];
   size_t buf_len_ = 0, blocks_ = 0;
   uint64_t chunk_ = 0;
-  std::vector<std::vector<uint32_t>> stack_;
+  std::vector<std::array<uint32_t, 8>> stack_;
 };
 
 }  // namespace hb3

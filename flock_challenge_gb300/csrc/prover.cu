@@ -12,12 +12,12 @@
 #include <chrono>
 #include <cstring>
 #include <mutex>
-#include <set>
 #include <stdexcept>
 #include <string>
 #include <vector>
 
 #include "flock_internal.h"
+#include "host_bulk.h"
 #include "host_field.h"
 #include "prover.h"
 #include "r1cs_setup.h"
@@ -106,19 +106,9 @@ inline int ilog2(size_t n) {
 }
 
 // ---------------------------------------------------------------- host algebra
-std::vector<F> eq_table(const std::vector<F>& r) {
-  std::vector<F> t((size_t)1 << r.size());
-  t[0] = F::one();
-  for (size_t i = 0; i < r.size(); i++) {
-    size_t h = (size_t)1 << i;
-    for (size_t j = 0; j < h; j++) {
-      F vr = t[j] * r[i];
-      t[j + h] = vr;
-      t[j] = t[j] + vr;
-    }
-  }
-  return t;
-}
+using hf::dot;
+using hf::eq_table;
+using hf::transpose128;
 
 // Lagrange weights on 64 nodes phi8(off..off+63) (multilinear.rs:361-520),
 // prefix/suffix products with cached denominators.
@@ -166,25 +156,6 @@ const std::vector<F>& phi_ext_matrix() {
   return pm;
 }
 
-F dot(const F* a, const F* b, size_t n) {
-  F s;
-  for (size_t i = 0; i < n; i++) s += a[i] * b[i];
-  return s;
-}
-
-std::vector<F> transpose128(const std::vector<F>& v) {
-  std::vector<F> u(128);
-  for (int i = 0; i < 128; i++)
-    for (int b = 0; b < 128; b++) {
-      uint64_t bit = b < 64 ? (v[i].lo >> b) & 1 : (v[i].hi >> (b - 64)) & 1;
-      if (bit) {
-        if (i < 64) u[b].lo |= 1ULL << i;
-        else u[b].hi |= 1ULL << (i - 64);
-      }
-    }
-  return u;
-}
-
 // s_k(v_k) and inverses, ligerito.rs:1747-1774.
 struct Sks {
   std::vector<F> s, inv;
@@ -227,12 +198,20 @@ const Sks& sks_for(int n) {
 }
 
 std::vector<uint32_t> sample_queries(fs::Transcript& tr, size_t block_len, size_t count) {
-  std::set<uint32_t> seen;
+  constexpr uint32_t kNone = 0xFFFFFFFFu;  // block_len <= 2^30
+  size_t cap = 64;
+  while (cap < 4 * count) cap *= 2;
+  std::vector<uint32_t> seen(cap, kNone);  // open addressing
   std::vector<uint32_t> out;
+  out.reserve(count);
   while (out.size() < count) {
     F v = tr.sample();
-    uint32_t q = (uint32_t)(v.lo % block_len);
-    if (seen.insert(q).second) out.push_back(q);
+    const uint32_t q = (uint32_t)(v.lo % block_len);
+    size_t h = (q * 0x9E3779B1u) & (cap - 1);
+    while (seen[h] != kNone && seen[h] != q) h = (h + 1) & (cap - 1);
+    if (seen[h] == q) continue;
+    seen[h] = q;
+    out.push_back(q);
   }
   std::sort(out.begin(), out.end());
   return out;
@@ -919,7 +898,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       d2h(*S, tA.data(), curA, n_in * 16);
       d2h(*S, tB.data(), curB, n_in * 16);
       auto bind = [](std::vector<F>& v, F rr) {
-        for (size_t j = 0; j < v.size() / 2; j++) v[j] = v[2 * j] + rr * (v[2 * j] + v[2 * j + 1]);
+        hf::bind_pairs(v.data(), v.size() / 2, rr);
         v.resize(v.size() / 2);
       };
       for (int i = host_from; i < n_mlv; i++) {
@@ -928,11 +907,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         const std::vector<F> rr(r.begin() + 6 + i + 1, r.end());
         const std::vector<F> eq = eq_table(rr);
         F g1, gi;
-        for (size_t j = 0; j < tA.size() / 2; j++) {
-          const F a0 = tA[2 * j], a1 = tA[2 * j + 1], b0 = tB[2 * j], b1 = tB[2 * j + 1];
-          g1 += eq[j] * (a1 * b1);
-          gi += eq[j] * ((a0 + a1) * (b0 + b1));
-        }
+        hf::weighted_round(tA.data(), tB.data(), eq.data(), tA.size() / 2, &g1, &gi);
         g1 = g1 * qs[i].dinv;
         gi = gi * qs[i].dinv;
         zc_rounds.push_back({g1, gi});
@@ -1011,19 +986,14 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       d2h(*S, hW.data(), dcomb, len * 16);
       d2h(*S, hg.data(), dzv, len * 16);
       auto bind_top = [](std::vector<F>& v, F rr) {
-        const size_t h = v.size() / 2;
-        for (size_t i = 0; i < h; i++) v[i] = v[i] + rr * (v[i + h] + v[i]);
-        v.resize(h);
+        hf::bind_halves(v.data(), v.size() / 2, rr);
+        v.resize(v.size() / 2);
       };
       for (; t < inner_rest; t++) {
         bind_top(hW, lc_rr.back());
         bind_top(hg, lc_rr.back());
-        const size_t q = hW.size() / 2;
         F e1, ei;
-        for (size_t i = 0; i < q; i++) {
-          e1 += hW[i + q] * hg[i + q];
-          ei += (hW[i] + hW[i + q]) * (hg[i] + hg[i + q]);
-        }
+        hf::halves_round(hW.data(), hg.data(), hW.size() / 2, &e1, &ei);
         tr.observe(e1);
         tr.observe(ei);
         lc_rounds.push_back({e1, ei});
@@ -1151,8 +1121,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     {
       // w_k[b] = gamma_k eq(r''_k)[b]: the basis is sum_k sum_b bit_b(t_k) w_k[b]
       std::vector<F> wk(2 * 128);
-      for (int k = 0; k < 2; k++)
-        for (int bb = 0; bb < 128; bb++) wk[k * 128 + bb] = gam[k] * eqr[k][bb];
+      for (int k = 0; k < 2; k++) hf::scale(eqr[k].data(), gam[k], 128, &wk[k * 128]);
       void* dt = S->tables.get(wk.size() * 16);
       h2d(*S, dt, wk.data(), wk.size() * 16);
       if (chain) {
@@ -1513,28 +1482,40 @@ H32 cv_bytes(const uint32_t w[8]) {
   memcpy(h.data(), w, 32);  // little-endian words
   return h;
 }
-// Non-root chaining value of a single-chunk leaf (<= 1024 bytes): blocks with
-// counter 0, CHUNK_START on the first, CHUNK_END on the last (merkle.rs:200-210).
-H32 leaf_cv(const uint8_t* d, size_t len) {
-  uint32_t cv[8];
-  memcpy(cv, hb3::IV, 32);
-  size_t nb = len == 0 ? 1 : (len + 63) / 64;
-  for (size_t b = 0; b < nb; b++) {
-    size_t off = b * 64, bl = len - off < 64 ? len - off : 64;
-    uint32_t m[16], o[16];
-    hb3::load_words(d + off, bl, m);
-    uint32_t fl = (b == 0 ? hb3::CHUNK_START : 0) | (b + 1 == nb ? hb3::CHUNK_END : 0);
-    hb3::compress(cv, m, 0, (uint32_t)bl, fl, o);
-    memcpy(cv, o, 32);
+// Non-root chaining values of single-chunk leaves (<= 1024 bytes each, all of
+// one size): blocks with counter 0, CHUNK_START on the first, CHUNK_END on the
+// last (merkle.rs:200-210). Eight leaves at a time.
+std::vector<H32> leaf_cvs(const std::vector<const uint8_t*>& d, size_t len) {
+  std::vector<H32> out(d.size());
+  const size_t nb = len == 0 ? 1 : (len + 63) / 64;
+  for (size_t i = 0; i < d.size(); i += 8) {
+    const size_t cnt = std::min<size_t>(8, d.size() - i);
+    uint32_t cv[8][8];
+    for (int k = 0; k < 8; k++) memcpy(cv[k], hb3::IV, 32);
+    for (size_t b = 0; b < nb; b++) {
+      const uint8_t* p[8];
+      for (size_t k = 0; k < 8; k++) p[k] = d[i + std::min(k, cnt - 1)] + b * 64;
+      const size_t bl = len - b * 64 < 64 ? len - b * 64 : 64;
+      hb3::compress_lanes8(cv, p, (uint32_t)bl, (b == 0 ? hb3::CHUNK_START : 0) | (b + 1 == nb ? hb3::CHUNK_END : 0));
+    }
+    for (size_t k = 0; k < cnt; k++) out[i + k] = cv_bytes(cv[k]);
   }
-  return cv_bytes(cv);
+  return out;
 }
-H32 parent_cv(const H32& l, const H32& r) {
-  uint32_t m[16], o[16];
-  memcpy(m, l.data(), 32);
-  memcpy(m + 8, r.data(), 32);
-  hb3::compress(hb3::IV, m, 0, 64, hb3::PARENT, o);
-  return cv_bytes(o);
+// The parents of pairs (64 bytes each, left || right), eight at a time.
+void parent_cvs(const std::vector<std::array<uint8_t, 64>>& lr, std::vector<H32>& out) {
+  out.resize(lr.size());
+  for (size_t i = 0; i < lr.size(); i += 8) {
+    const size_t cnt = std::min<size_t>(8, lr.size() - i);
+    uint32_t cv[8][8];
+    const uint8_t* p[8];
+    for (size_t k = 0; k < 8; k++) {
+      memcpy(cv[k], hb3::IV, 32);
+      p[k] = lr[i + std::min(k, cnt - 1)].data();
+    }
+    hb3::compress_lanes8(cv, p, 64, hb3::PARENT);
+    for (size_t k = 0; k < cnt; k++) out[i + k] = cv_bytes(cv[k]);
+  }
 }
 // Octopus multi-proof check (merkle.rs:937-1004).
 bool merkle_multi_ok(const H32& root, size_t n_leaves, const std::vector<uint32_t>& pos, std::vector<H32> leaves,
@@ -1544,30 +1525,34 @@ bool merkle_multi_ok(const H32& root, size_t n_leaves, const std::vector<uint32_
   for (size_t i = 0; i < pos.size(); i++)
     if (pos[i] >= n_leaves || (i && pos[i - 1] >= pos[i])) return false;
   if (n_leaves == 1) return proof.empty() && leaves[0] == root;
-  std::vector<std::pair<size_t, H32>> act;
-  for (size_t i = 0; i < pos.size(); i++) act.push_back({pos[i], leaves[i]});
+  std::vector<size_t> act(pos.begin(), pos.end());
+  std::vector<H32> cvs(std::move(leaves));
+  std::vector<std::array<uint8_t, 64>> lr;
   size_t pi = 0;
   for (size_t ll = n_leaves; ll > 1; ll >>= 1) {
-    std::vector<std::pair<size_t, H32>> nxt;
+    std::vector<size_t> nxt;
+    lr.clear();
     for (size_t i = 0; i < act.size();) {
-      size_t p = act[i].first;
-      H32 l, r;
-      if (i + 1 < act.size() && act[i + 1].first == (p ^ 1)) {
-        l = act[i].second;
-        r = act[i + 1].second;
+      const size_t p = act[i];
+      std::array<uint8_t, 64> b;
+      if (i + 1 < act.size() && act[i + 1] == (p ^ 1)) {
+        memcpy(b.data(), cvs[i].data(), 32);
+        memcpy(b.data() + 32, cvs[i + 1].data(), 32);
         i += 2;
       } else {
         if (pi >= proof.size()) return false;
         const H32& sb = proof[pi++];
-        if (p & 1) { l = sb; r = act[i].second; }
-        else { l = act[i].second; r = sb; }
+        memcpy(b.data() + ((p & 1) ? 32 : 0), cvs[i].data(), 32);
+        memcpy(b.data() + ((p & 1) ? 0 : 32), sb.data(), 32);
         i += 1;
       }
-      nxt.push_back({p >> 1, parent_cv(l, r)});
+      lr.push_back(b);
+      nxt.push_back(p >> 1);
     }
+    parent_cvs(lr, cvs);
     act.swap(nxt);
   }
-  return pi == proof.size() && act.size() == 1 && act[0].second == root;
+  return pi == proof.size() && act.size() == 1 && cvs[0] == root;
 }
 
 // Proof of work (challenger.rs:1246-1310): BLAKE3(digest || nonce_le || 0^24)
@@ -1631,16 +1616,16 @@ std::vector<F> combined_weights(F z) {
 }
 
 void bind_top(std::vector<F>& v, F r) {
-  size_t half = v.size() / 2;
-  for (size_t i = 0; i < half; i++) v[i] = v[i] + r * (v[i + half] + v[i]);
-  v.resize(half);
+  hf::bind_halves(v.data(), v.size() / 2, r);
+  v.resize(v.size() / 2);
 }
 
 std::vector<F> what_at(int n, const Sks& sk, uint32_t q) {
   std::vector<F> w(n);
-  for (int k = 0; k < n; k++)
-    for (int b = 0; b < 32; b++)
-      if ((q >> b) & 1) w[k] += sk.lin[(size_t)k * 32 + b];
+  for (uint32_t left = q; left; left &= left - 1) {
+    const int b = __builtin_ctz(left);
+    for (int k = 0; k < n; k++) w[k] += sk.lin[(size_t)k * 32 + b];
+  }
   return w;
 }
 
@@ -1943,8 +1928,7 @@ static int verify_impl(ProverState* S, const uint8_t* data, size_t len, const ch
     void* dbc = S->bc.get(n128 * 16);
     {
       std::vector<F> wk(2 * 128);
-      for (int k = 0; k < 2; k++)
-        for (int bb = 0; bb < 128; bb++) wk[k * 128 + bb] = gam[k] * eqr[k][bb];
+      for (int k = 0; k < 2; k++) hf::scale(eqr[k].data(), gam[k], 128, &wk[k * 128]);
       void* dt = S->tables.get(wk.size() * 16);
       h2d(*S, dt, wk.data(), wk.size() * 16);
       FK(flock_launch_combined_basis(n128, S->tlo0.p, S->thi0.p, S->tlo1.p, S->thi1.p, rs_lo, dt, dbc, st));
@@ -1988,11 +1972,12 @@ static int verify_impl(ProverState* S, const uint8_t* data, size_t len, const ch
     auto opens_ok = [&](const H32& root, size_t block_len, const std::vector<uint32_t>& q, const VOpen& o,
                         size_t width) {
       if (q.size() != o.rows.size()) return false;
-      std::vector<H32> leaves;
+      std::vector<const uint8_t*> rows;
       for (auto& row : o.rows) {
         if (row.size() != width) return false;
-        leaves.push_back(leaf_cv((const uint8_t*)row.data(), row.size() * 16));
+        rows.push_back((const uint8_t*)row.data());
       }
+      std::vector<H32> leaves = leaf_cvs(rows, width * 16);
       std::vector<H32> nodes(o.nodes.begin(), o.nodes.end());
       return merkle_multi_ok(root, block_len, q, leaves, nodes);
     };
