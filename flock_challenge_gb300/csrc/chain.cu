@@ -54,13 +54,13 @@ __global__ void chain_weights_kernel(const gf128* __restrict__ lo, const gf128* 
 }
 
 // With bind: the 2h-entry tables W, g are bound at r in their top variable
-// (x' = x_lo + r (x_hi + x_lo)) into their first h entries, in place (thread i
-// owns entries i, i + h/2, i + h, i + 3h/2). Then the round message over the
+// (x' = x_lo + r (x_hi + x_lo)) into the first h entries of Wo, go, which may
+// be W, g (thread i owns entries i, i + h/2, i + h, i + 3h/2). Then the round message over the
 // h-entry tables: q(1) = sum W_hi g_hi, q(inf) = sum (W_lo + W_hi)(g_lo + g_hi),
 // halves split at h/2; per-block partials (q(1), q(inf)).
 __global__ void __launch_bounds__(CH_THREADS)
-chain_round_kernel(gf128* __restrict__ W, gf128* __restrict__ g, size_t h, int bind, const __grid_constant__ gf128p r,
-                   gf128* __restrict__ partials) {
+chain_round_kernel(const gf128* W, const gf128* g, size_t h, int bind, const __grid_constant__ gf128p r, gf128* Wo,
+                   gf128* go, gf128* __restrict__ partials) {
   const size_t q = h / 2;
   gf256 e1 = {{0, 0, 0, 0}}, ei = e1;
   for (size_t i = (size_t)blockIdx.x * CH_THREADS + threadIdx.x; i < q; i += (size_t)gridDim.x * CH_THREADS) {
@@ -70,7 +70,7 @@ chain_round_kernel(gf128* __restrict__ W, gf128* __restrict__ g, size_t h, int b
       wh = gf_add(wh, gf_mul_p(gf_add(W[i + q + h], wh), r));
       gl = gf_add(gl, gf_mul_p(gf_add(g[i + h], gl), r));
       gh = gf_add(gh, gf_mul_p(gf_add(g[i + q + h], gh), r));
-      W[i] = wl; W[i + q] = wh; g[i] = gl; g[i + q] = gh;
+      Wo[i] = wl; Wo[i + q] = wh; go[i] = gl; go[i + q] = gh;
     }
     gf256_acc(e1, gf_mul_wide(wh, gh));
     gf256_acc(ei, gf_mul_wide(gf_add(wl, wh), gf_add(gl, gh)));
@@ -98,7 +98,7 @@ chain_round_kernel(gf128* __restrict__ W, gf128* __restrict__ g, size_t h, int b
 // this 5.1 us.
 constexpr size_t CH_SMALL_PAIRS = (size_t)1 << 17;
 __global__ void __launch_bounds__(CH_THREADS)
-chain_round_small_kernel(gf128* __restrict__ W, gf128* __restrict__ g, size_t h, int bind, const gf128 r,
+chain_round_small_kernel(const gf128* W, const gf128* g, size_t h, int bind, const gf128 r, gf128* Wo, gf128* go,
                          gf128* __restrict__ partials) {
   const size_t q = h / 2, t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, j = t >> 1;
   const size_t i = (t & 1) ? j + q : j;  // the pair's entry of the lower or upper half
@@ -114,8 +114,8 @@ chain_round_small_kernel(gf128* __restrict__ W, gf128* __restrict__ g, size_t h,
   }
   const gf128 p = gf_round_small<false, 0>(w0, w1, g0, g1, bind, r, gf_zero());
   if (bind && act) {
-    W[i] = w0;
-    g[i] = g0;
+    Wo[i] = w0;
+    go[i] = g0;
   }
   gf_block_sum_lanes(p, 1, partials + 2 * blockIdx.x);  // q(1) from the odd lanes, q(inf) from the even ones
 }
@@ -159,18 +159,18 @@ int flock_chain_round_grid(size_t h) {
   return h / 2 <= CH_SMALL_PAIRS ? gf_small_grid(h / 2) : (int)grid_for(h / 2, CH_THREADS, 152 * 4);
 }
 
-int flock_launch_chain_round(void* W, void* g, size_t h, int bind, const uint64_t r[2], void* partials, int grid,
-                             cudaStream_t st) {
+int flock_launch_chain_round(void* W, void* g, size_t h, int bind, const uint64_t r[2], void* Wo, void* go,
+                             void* partials, int grid, cudaStream_t st) {
   if (h < 2) return FLOCK_ERR_SHAPE;
   if (h / 2 <= CH_SMALL_PAIRS) {
     if (grid != gf_small_grid(h / 2)) return FLOCK_ERR_SHAPE;
-    chain_round_small_kernel<<<grid, gf_small_threads(h / 2), 0, st>>>((gf128*)W, (gf128*)g, h, bind, to_gf(r),
-                                                                       (gf128*)partials);
+    chain_round_small_kernel<<<grid, gf_small_threads(h / 2), 0, st>>>(
+        (const gf128*)W, (const gf128*)g, h, bind, to_gf(r), (gf128*)Wo, (gf128*)go, (gf128*)partials);
     flock_count_launch();
     return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
   }
-  chain_round_kernel<<<grid, CH_THREADS, 0, st>>>((gf128*)W, (gf128*)g, h, bind, gf_prepare(to_gf(r)),
-                                                  (gf128*)partials);
+  chain_round_kernel<<<grid, CH_THREADS, 0, st>>>((const gf128*)W, (const gf128*)g, h, bind, gf_prepare(to_gf(r)),
+                                                  (gf128*)Wo, (gf128*)go, (gf128*)partials);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }

@@ -32,16 +32,21 @@ int flock_launch_zc_round1(const void* a, const void* b, const void* c, size_t n
 int flock_launch_zc1_eq_basis(const void* eq_out, size_t n_outer, const ZcRound1Tables* d_tables, void* out,
                               cudaStream_t st);
 int flock_launch_reduce_rows(const void* in, size_t count, int width, void* out, cudaStream_t st);
-int flock_launch_eq_split(const void* r, int lo_bits, int hi_bits, void* lo, void* hi, cudaStream_t st);
-// Several eq table pairs in one launch (device array of jobs; lo_bits and
-// hi_bits each at most 28; max_entries = the largest 2^lo_bits + 2^hi_bits).
+// Split eq tables: lo[i] = eq of lo_bits variables at the bits of i, hi[i] of the
+// next hi_bits. A batch holds up to FLOCK_EQ_VARS variables and FLOCK_EQ_JOBS
+// table pairs; a pair takes the variables from `first` on, leaving out skip_n of
+// them after the first skip_at. lo_bits and hi_bits at most 28.
+constexpr int FLOCK_EQ_VARS = 64, FLOCK_EQ_JOBS = 24;
 struct FlockEqJob {
-  const void* r;
-  void* lo;
-  void* hi;
-  int lo_bits, hi_bits;
+  void *lo, *hi;
+  int lo_bits, hi_bits, first, skip_at, skip_n;
 };
-int flock_launch_eq_split_multi(const FlockEqJob* d_jobs, int n_jobs, size_t max_entries, cudaStream_t st);
+struct FlockEqBatch {
+  uint64_t r[FLOCK_EQ_VARS][2];
+  FlockEqJob jobs[FLOCK_EQ_JOBS];
+  int n_jobs;
+};
+int flock_launch_eq_tables(const FlockEqBatch& q, cudaStream_t st);
 int flock_launch_zc_round(const void* A, const void* B, size_t n_pairs, int bind, const uint64_t rho[2], void* Aout,
                           void* Bout, const void* eq_lo, const void* eq_hi, int lo_bits, void* partials, int grid,
                           cudaStream_t st);
@@ -91,12 +96,15 @@ int flock_launch_glue(void* b, const void* add, size_t n, const uint64_t beta[2]
 size_t flock_induce_basis_rows_bytes(int n, int log_d, int nq);
 int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, int log_d, const void* what_lin,
                               const void* alpha_w, void* LO, void* basis, cudaStream_t st);
-int flock_launch_gather_rows(const void* mat, const uint32_t* rows, int n_rows, int width, void* out,
-                             cudaStream_t st);
-int flock_launch_gather_nodes(const void* tree, const uint32_t* idx, int n, void* out, cudaStream_t st);
+// Rows `rows` of mat (width F128 each) and 32-byte nodes `idx` of tree; the index
+// lists and both outputs may be pinned host memory.
+int flock_launch_gather_opening(const void* mat, const uint32_t* rows, int n_rows, int width, void* out_rows,
+                                const void* tree, const uint32_t* idx, int n_nodes, void* out_nodes, cudaStream_t st);
 // waits: the caller's count of host waits (nullptr: not counted).
+// h_best_atomic: h_best is pinned memory the device's atomics reach, so the
+// kernel lowers it directly.
 int flock_grind(const uint8_t digest[32], uint32_t bits, void* d_scratch, int* parity, uint64_t* h_best,
-                cudaStream_t st, WaitStats* waits, uint64_t* nonce);
+                bool h_best_atomic, cudaStream_t st, WaitStats* waits, uint64_t* nonce);
 
 // Launch counter of this library's kernels (read through flock_kernel_launches).
 int flock_launch_fold_lsb(const void* in, size_t n_out, const uint64_t r[2], void* out, cudaStream_t st);
@@ -126,8 +134,9 @@ int flock_launch_chain_fold_io(const void* z, size_t n_inst, const uint64_t e0[2
 int flock_launch_chain_weights(const void* lo, const void* hi, int lo_bits, size_t n_inst, const uint64_t alpha[2],
                                void* W, cudaStream_t st);
 int flock_chain_round_grid(size_t h);
-int flock_launch_chain_round(void* W, void* g, size_t h, int bind, const uint64_t r[2], void* partials, int grid,
-                             cudaStream_t st);
+// With bind, the bound tables go to Wo, go (W, g themselves, or others).
+int flock_launch_chain_round(void* W, void* g, size_t h, int bind, const uint64_t r[2], void* Wo, void* go,
+                             void* partials, int grid, cudaStream_t st);
 int flock_launch_chain_claim_basis(void* b, size_t n_inst, const void* lo, const void* hi, int lo_bits,
                                    const uint64_t c[8], cudaStream_t st);
 

@@ -37,7 +37,8 @@ struct Digest {
 // `other` (may be null): the other result slot, reset here for the next grind
 // (which runs after this launch in stream order), so no grind needs a memset.
 __global__ void grind_kernel(const __grid_constant__ Digest digest, uint64_t start, uint64_t count, uint32_t bits,
-                             unsigned long long* __restrict__ best, unsigned long long* __restrict__ other) {
+                             unsigned long long* __restrict__ best, unsigned long long* __restrict__ other,
+                             int best_on_host) {
   uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= count) return;
   if (other && i == 0) *other = ~0ull;
@@ -53,7 +54,10 @@ __global__ void grind_kernel(const __grid_constant__ Digest digest, uint64_t sta
 #pragma unroll
   for (int k = 0; k < 8; k++) cv[k] = b3::IV(k);
   b3::compress_cv(cv, m, 64, b3::CHUNK_START | b3::CHUNK_END | b3::ROOT);
-  if (leading_zeros_ok(cv, bits)) atomicMin(best, (unsigned long long)nonce);
+  if (leading_zeros_ok(cv, bits)) {
+    if (best_on_host) atomicMin_system(best, (unsigned long long)nonce);
+    else atomicMin(best, (unsigned long long)nonce);
+  }
 }
 
 // Grinds of at most this many bits run on the host: about 2^bits hashes of
@@ -89,7 +93,7 @@ bool host_pow(const uint32_t dg[8], uint64_t nonce, uint32_t bits) {
 // grinds alternate slots and each resets the other one for the next; without,
 // the slot is cleared by a memset first.
 int flock_grind(const uint8_t digest[32], uint32_t bits, void* d_scratch, int* parity, uint64_t* h_best,
-                cudaStream_t st, WaitStats* waits, uint64_t* nonce) {
+                bool h_best_atomic, cudaStream_t st, WaitStats* waits, uint64_t* nonce) {
   if (bits == 0) {
     *nonce = 0;
     return FLOCK_OK;
@@ -108,28 +112,38 @@ int flock_grind(const uint8_t digest[32], uint32_t bits, void* d_scratch, int* p
   }
   unsigned long long* d_best = (unsigned long long*)d_scratch;
   unsigned long long* d_other = nullptr;
+  if (h_best_atomic) {
+    d_best = reinterpret_cast<unsigned long long*>(h_best);  // reset here: nothing on the stream writes it any more
+    *reinterpret_cast<volatile uint64_t*>(h_best) = ~0ull;
+    parity = nullptr;
+  }
   if (parity) {
     d_best += *parity & 1;
     d_other = (unsigned long long*)d_scratch + ((*parity & 1) ^ 1);
     ++*parity;
   }
   const unsigned long long none = ~0ull;
-  if (!parity && cudaMemsetAsync(d_best, 0xFF, 8, st) != cudaSuccess) return FLOCK_ERR_CUDA;
-  // About two expected hits per window: a miss costs one more window, an
-  // oversized window wastes work on every grind (most grinds are 2..14 bits).
-  int wlog = (int)bits + 1;
+  if (!parity && !h_best_atomic && cudaMemsetAsync(d_best, 0xFF, 8, st) != cudaSuccess) return FLOCK_ERR_CUDA;
+  // A miss costs one more window and wait, an oversized window its hashes: up
+  // to 2^15 nonces (a quarter of a wave) cost nothing over the launch, so small
+  // grinds expect eight hits per window, larger ones two.
+  int wlog = (int)bits + 3;
+  if (wlog > 15) wlog = (int)bits + 1 > 15 ? (int)bits + 1 : 15;
   if (wlog < 12) wlog = 12;
   if (wlog > 26) wlog = 26;
   uint64_t window = (uint64_t)1 << wlog;
   for (uint64_t start = 0;; start += window) {
-    grind_kernel<<<(unsigned)((window + 255) / 256), 256, 0, st>>>(dg, start, window, bits, d_best, d_other);
+    grind_kernel<<<(unsigned)((window + 255) / 256), 256, 0, st>>>(dg, start, window, bits, d_best, d_other,
+                                                                     h_best_atomic);
     flock_count_launch();
     if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
-    if (cudaMemcpyAsync(h_best, d_best, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess) return FLOCK_ERR_CUDA;
+    if (!h_best_atomic && cudaMemcpyAsync(h_best, d_best, 8, cudaMemcpyDeviceToHost, st) != cudaSuccess)
+      return FLOCK_ERR_CUDA;
     const cudaError_t we = flock_stream_wait(st, waits);
     if (we != cudaSuccess) return we == cudaErrorTimeout ? FLOCK_ERR_TIMEOUT : FLOCK_ERR_CUDA;
-    if (*h_best != none) {
-      *nonce = *h_best;
+    const uint64_t found = *reinterpret_cast<volatile uint64_t*>(h_best);
+    if (found != none) {
+      *nonce = found;
       return FLOCK_OK;
     }
     if (start > ((uint64_t)1 << 62)) return FLOCK_ERR_TIMEOUT;

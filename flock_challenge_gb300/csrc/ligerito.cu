@@ -329,19 +329,20 @@ __global__ void fold_lsb_kernel(const gf128* __restrict__ in, size_t n_out, cons
   }
 }
 
-__global__ void gather_rows_kernel(const gf128* __restrict__ mat, const uint32_t* __restrict__ rows, int n_rows,
-                                   int width, gf128* __restrict__ out) {
-  size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (size_t)n_rows * width) return;
-  size_t r = e / width, c = e % width;
-  out[e] = mat[(size_t)rows[r] * width + c];
-}
-
-__global__ void gather_nodes_kernel(const uint4* __restrict__ tree, const uint32_t* __restrict__ idx, int n,
-                                    uint4* __restrict__ out) {
-  int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= 2 * n) return;
-  out[e] = tree[2 * (size_t)idx[e >> 1] + (e & 1)];
+// The opened rows, then the multiproof's nodes, in one launch. The index lists
+// are read from, and the values written to, pinned host memory: no copies
+// before or behind the kernel.
+__global__ void gather_opening_kernel(const gf128* __restrict__ mat, const uint32_t* __restrict__ rows, int n_rows,
+                                      int width, gf128* __restrict__ out_rows, const uint4* __restrict__ tree,
+                                      const uint32_t* __restrict__ idx, int n_nodes, uint4* __restrict__ out_nodes) {
+  const size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nr = (size_t)n_rows * width;
+  if (e < nr) {
+    const size_t r = e / width, c = e % width;
+    out_rows[e] = mat[(size_t)rows[r] * width + c];
+  } else if (e - nr < 2 * (size_t)n_nodes) {
+    const size_t k = e - nr;
+    out_nodes[k] = tree[2 * (size_t)idx[k >> 1] + (k & 1)];
+  }
 }
 
 inline gf128 to_gf(const uint64_t v[2]) {
@@ -448,17 +449,14 @@ int flock_launch_induce_basis(const uint32_t* d_queries, int nq, int n, int log_
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
-int flock_launch_gather_rows(const void* mat, const uint32_t* rows, int n_rows, int width, void* out,
-                             cudaStream_t st) {
-  size_t n = (size_t)n_rows * width;
-  gather_rows_kernel<<<grid_for(n, 256, 1u << 30), 256, 0, st>>>((const gf128*)mat, rows, n_rows, width,
-                                                                  (gf128*)out); flock_count_launch();
-  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
-}
-
-int flock_launch_gather_nodes(const void* tree, const uint32_t* idx, int n, void* out, cudaStream_t st) {
+int flock_launch_gather_opening(const void* mat, const uint32_t* rows, int n_rows, int width, void* out_rows,
+                                const void* tree, const uint32_t* idx, int n_nodes, void* out_nodes, cudaStream_t st) {
+  const size_t n = (size_t)n_rows * width + 2 * (size_t)n_nodes;
   if (n == 0) return FLOCK_OK;
-  gather_nodes_kernel<<<(2 * n + 255) / 256, 256, 0, st>>>((const uint4*)tree, idx, n, (uint4*)out); flock_count_launch();
+  gather_opening_kernel<<<grid_for(n, 256, 1u << 30), 256, 0, st>>>((const gf128*)mat, rows, n_rows, width,
+                                                                   (gf128*)out_rows, (const uint4*)tree, idx, n_nodes,
+                                                                   (uint4*)out_nodes);
+  flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 

@@ -263,7 +263,7 @@ struct Open {
   std::vector<F> rows;  // q x width
   size_t width = 0;
   std::vector<uint8_t> nodes;  // 32-byte hashes
-  // Copied into the pinned openings area by the stream (no wait of its own):
+  // Gathered into the pinned openings area (no wait of its own):
   // rows and nodes are filled from there by finish_open once a later wait
   // has passed. -1: already filled.
   ptrdiff_t pin_rows = -1, pin_nodes = -1;
@@ -280,9 +280,9 @@ struct ProverState {
   cudaStream_t st = nullptr;  // the stream in use: st_normal or st_high
   cudaStream_t st_normal = nullptr, st_high = nullptr;
   ZcRound1Tables* d_r1t = nullptr;
-  DBuf in, z, a, b, stripe, cw, tree, A0, B0, A1, B1, eqlo, eqhi, eqout, rdev, part, red, lag, small, eqin, comb,
-      zvec, zvec0, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, LO, basis, qbuf, abuf, rows, nidx, nodes,
-      grind, lvl_cw[2], lvl_tree[2], chW, chG, zceq, zcr, zcjobs;
+  DBuf in, z, a, b, stripe, cw, tree, A0, B0, A1, B1, eqlo, eqhi, eqout, part, red, lag, small, eqin, comb,
+      zvec, zvec1, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, LO, basis, qbuf, qopen, rows, nidx, nodes,
+      grind, lvl_cw[2], lvl_tree[2], chW, chG, zceq;
   DBuf csc_ap, csc_ai, csc_bp, csc_bi;
   bool csc_ready = false;
   DBuf skl[kSklMax];  // What_k(x^b) tables of the induced basis, per number of variables
@@ -300,23 +300,24 @@ struct ProverState {
   // copies asynchronous); device->host reads go through the last kPinD2H bytes.
   uint8_t* pin = nullptr;
   size_t pin_off = 0;
-  // Pinned area the opened rows and Merkle nodes of a proof are copied into
+  // Pinned area the opened rows and Merkle nodes of a proof are gathered into
   // (bump-allocated per proof): they are only serialized at the end of the
-  // proof, so their copies ride on the stream and need no wait of their own.
+  // proof, so they need no wait of their own.
   uint8_t* pin_open = nullptr;
   size_t pin_open_off = 0;
   // Mapped pinned area for round partials: kernels write them straight into
   // host memory, so reading a round's message needs only the stream sync.
   uint8_t* mapped = nullptr;
   void* mapped_dev = nullptr;
+  bool host_atomics = false;  // the device's atomics reach pinned host memory (cudaDevAttrHostNativeAtomicSupported)
   // The host's waits for the stream (flock_stream_wait) in the current proof.
   WaitStats waits;
 
   std::vector<DBuf*> bufs() {
-    std::vector<DBuf*> v = {&in, &z, &a, &b, &stripe, &cw, &tree, &A0, &B0, &A1, &B1, &eqlo, &eqhi, &eqout, &rdev, &part, &red,
-            &lag, &small, &eqin, &comb, &zvec, &zvec0, &tlo0, &thi0, &tlo1, &thi1, &tables, &bc, &f1, &b1,
-            &LO, &basis, &qbuf, &abuf, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
-            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &zcr, &zcjobs, &csc_ap, &csc_ai, &csc_bp, &csc_bi};
+    std::vector<DBuf*> v = {&in, &z, &a, &b, &stripe, &cw, &tree, &A0, &B0, &A1, &B1, &eqlo, &eqhi, &eqout, &part, &red,
+            &lag, &small, &eqin, &comb, &zvec, &zvec1, &tlo0, &thi0, &tlo1, &thi1, &tables, &bc, &f1, &b1,
+            &LO, &basis, &qbuf, &qopen, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
+            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &csc_ap, &csc_ai, &csc_bp, &csc_bi};
     for (DBuf& d : skl) v.push_back(&d);
     return v;
   }
@@ -330,6 +331,7 @@ namespace {
 
 constexpr size_t kPinH2D = (size_t)4 << 20, kPinD2H = (size_t)1 << 20, kMapped = (size_t)256 << 10;
 constexpr size_t kPinOpen = (size_t)4 << 20;
+constexpr size_t kGrindSlot = 64;  // the last bytes of the pinned read area: a grind's result
 // Zerocheck rounds of at most this many pairs run on the host (see the round loop).
 constexpr size_t kHostTailPairs = 512;
 // Lincheck product-sumcheck rounds over at most this many entries run on the host.
@@ -347,9 +349,29 @@ void h2d(ProverState& S, void* d, const void* h, size_t n) {
     CK(cudaMemcpyAsync(d, h, n, cudaMemcpyHostToDevice, S.st));
   }
 }
+// Small kernel inputs left in the pinned arena, where kernels read them; copied
+// to `dev` where the arena has no room.
+const void* staged(ProverState& S, DBuf& dev, const void* h, size_t n) {
+  const size_t need = (n + 255) & ~(size_t)255;
+  if (S.pin && S.pin_off + need <= kPinH2D) {
+    uint8_t* p = S.pin + S.pin_off;
+    S.pin_off += need;
+    std::memcpy(p, h, n);
+    return p;
+  }
+  void* d = dev.get(n);
+  h2d(S, d, h, n);
+  return d;
+}
+// A kernel's output for the host: in the upper half of the pinned read area
+// (the copies of d2h use the lower one), to be read after the next wait; nullptr
+// where it does not fit.
+void* host_out(ProverState& S, size_t off, size_t n) {
+  return S.pin && off + n <= kPinD2H / 2 - kGrindSlot ? S.pin + kPinH2D + kPinD2H / 2 + off : nullptr;
+}
 void d2h(ProverState& S, void* h, const void* d, size_t n) {
   if (n == 0) return;
-  if (S.pin && n <= kPinD2H) {
+  if (S.pin && n <= kPinD2H / 2) {
     uint8_t* p = S.pin + kPinH2D;
     CK(cudaMemcpyAsync(p, d, n, cudaMemcpyDeviceToHost, S.st));
     CK(flock_stream_wait(S.st, &S.waits));
@@ -362,7 +384,7 @@ void d2h(ProverState& S, void* h, const void* d, size_t n) {
 // Two device->host reads behind one wait.
 void d2h2(ProverState& S, void* h1, const void* d1, size_t n1, void* h2, const void* d2, size_t n2) {
   const size_t off2 = (n1 + 255) & ~(size_t)255;
-  if (!S.pin || off2 + n2 > kPinD2H) {
+  if (!S.pin || off2 + n2 > kPinD2H / 2) {
     d2h(S, h1, d1, n1);
     d2h(S, h2, d2, n2);
     return;
@@ -400,36 +422,31 @@ Open open_rows(ProverState& S, const void* cw, const void* tree, size_t block_le
                const std::vector<uint32_t>& q) {
   Open o;
   o.width = width;
-  uint32_t* dq = (uint32_t*)S.qbuf.get(q.size() * 4);
-  h2d(S, dq, q.data(), q.size() * 4);
-  void* dr = S.rows.get(q.size() * width * 16);
-  FK(flock_launch_gather_rows(cw, dq, (int)q.size(), width, dr, S.st));
-  // both gathers are queued before the first read: one wait for the two
-  auto idx = multiproof_nodes(block_len, q);
-  void* dn = nullptr;
-  if (!idx.empty()) {
-    uint32_t* di = (uint32_t*)S.nidx.get(idx.size() * 4);
-    h2d(S, di, idx.data(), idx.size() * 4);
-    dn = S.nodes.get(idx.size() * 32);
-    FK(flock_launch_gather_nodes(tree, di, (int)idx.size(), dn, S.st));
-  }
+  const uint32_t* dq = (const uint32_t*)staged(S, S.qopen, q.data(), q.size() * 4);
+  const auto idx = multiproof_nodes(block_len, q);
+  const uint32_t* di = idx.empty() ? nullptr : (const uint32_t*)staged(S, S.nidx, idx.data(), idx.size() * 4);
   o.rows.resize(q.size() * width);
   o.nodes.resize(idx.size() * 32);
-  const size_t nr = o.rows.size() * 16, nn = dn ? o.nodes.size() : 0;
+  const size_t nr = o.rows.size() * 16, nn = o.nodes.size();
   const size_t need = ((nr + 255) & ~(size_t)255) + ((nn + 255) & ~(size_t)255);
-  if (S.pin_open && S.pin_open_off + need <= kPinOpen) {
+  const bool pinned = S.pin_open && S.pin_open_off + need <= kPinOpen;
+  void *dr = nullptr, *dn = nullptr;
+  if (pinned) {
     o.pin_rows = (ptrdiff_t)S.pin_open_off;
     o.pin_nodes = (ptrdiff_t)(S.pin_open_off + ((nr + 255) & ~(size_t)255));
     S.pin_open_off += need;
-    if (nr) CK(cudaMemcpyAsync(S.pin_open + o.pin_rows, dr, nr, cudaMemcpyDeviceToHost, S.st));
-    if (nn) CK(cudaMemcpyAsync(S.pin_open + o.pin_nodes, dn, nn, cudaMemcpyDeviceToHost, S.st));
+    dr = S.pin_open + o.pin_rows;
+    dn = S.pin_open + o.pin_nodes;
   } else {
-    d2h2(S, o.rows.data(), dr, nr, o.nodes.data(), dn, nn);
+    dr = S.rows.get(nr);
+    dn = S.nodes.get(nn + 16);
   }
+  FK(flock_launch_gather_opening(cw, dq, (int)q.size(), width, dr, tree, di, (int)idx.size(), dn, S.st));
+  if (!pinned) d2h2(S, o.rows.data(), dr, nr, o.nodes.data(), dn, nn);
   return o;
 }
 
-// Fills an opening whose copies were queued by open_rows; the caller has
+// Fills an opening that open_rows had gathered into pinned memory; the caller has
 // waited for the stream since.
 void finish_open(ProverState& S, Open& o) {
   if (o.pin_rows < 0) return;
@@ -467,6 +484,12 @@ std::vector<F> reduce_partials(ProverState& S, const void* part, size_t count, i
       for (int k = 0; k < width; k++) out[k] += rows[c * width + k];
     return out;
   }
+  if (void* r = host_out(S, 0, (size_t)width * 16)) {
+    FK(flock_launch_reduce_rows(part, count, width, r, S.st));
+    CK(flock_stream_wait(S.st, &S.waits));
+    std::memcpy(out.data(), r, (size_t)width * 16);
+    return out;
+  }
   void* r = S.red.get((size_t)width * 16);
   FK(flock_launch_reduce_rows(part, count, width, r, S.st));
   d2h(S, out.data(), r, (size_t)width * 16);
@@ -480,11 +503,22 @@ void* part_buf(ProverState& S, size_t bytes) {
   return S.part.get(bytes);
 }
 
+// Adds to a batch the tables of r, split after lo_bits variables.
+void eq_job(FlockEqBatch& q, const std::vector<F>& r, int lo_bits, DBuf& lo, DBuf& hi) {
+  int first = 0;
+  for (int i = 0; i < q.n_jobs; i++)
+    first = std::max(first, q.jobs[i].first + q.jobs[i].lo_bits + q.jobs[i].hi_bits + q.jobs[i].skip_n);
+  const int hi_bits = (int)r.size() - lo_bits;
+  if (q.n_jobs >= FLOCK_EQ_JOBS || first + (int)r.size() > FLOCK_EQ_VARS) throw Fail(FLOCK_ERR_SHAPE, "eq tables");
+  for (size_t i = 0; i < r.size(); i++) u2(r[i], q.r[first + i]);
+  q.jobs[q.n_jobs++] = {lo.get((size_t)16 << lo_bits), hi.get((size_t)16 << hi_bits), lo_bits, hi_bits, first,
+                        (int)r.size(), 0};
+}
 void eq_split_dev(ProverState& S, const std::vector<F>& r, int lo_bits, DBuf& lo, DBuf& hi) {
-  int hi_bits = (int)r.size() - lo_bits;
-  void* dr = S.rdev.get(r.size() * 16 + 16);
-  h2d(S, dr, r.data(), r.size() * 16);
-  FK(flock_launch_eq_split(dr, lo_bits, hi_bits, lo.get((size_t)16 << lo_bits), hi.get((size_t)16 << hi_bits), S.st));
+  FlockEqBatch q;
+  q.n_jobs = 0;
+  eq_job(q, r, lo_bits, lo, hi);
+  FK(flock_launch_eq_tables(q, S.st));
 }
 
 }  // namespace
@@ -508,6 +542,9 @@ ProverState* flock_prover_create(int device) {
   void* pin = nullptr;
   if (cudaMallocHost(&pin, kPinH2D + kPinD2H) == cudaSuccess) S->pin = (uint8_t*)pin;
   else cudaGetLastError();
+  int native = 0;
+  S->host_atomics =
+      cudaDeviceGetAttribute(&native, cudaDevAttrHostNativeAtomicSupported, device) == cudaSuccess && native;
   void* po = nullptr;
   if (cudaMallocHost(&po, kPinOpen) == cudaSuccess) S->pin_open = (uint8_t*)po;
   else cudaGetLastError();
@@ -712,13 +749,15 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       const size_t rows = nbits / 64, n_outer = rows / 128;
       std::vector<F> rout(r.begin() + 13, r.end());
       int nv = (int)rout.size();
-      void* dr = S->rdev.get(rout.size() * 16 + 16);
-      h2d(*S, dr, rout.data(), rout.size() * 16);
       // eq_out, then round 1's per-block table basis phi8(2^k) eq_out(xo)
       // behind it in the same buffer
       void* deq = S->eqout.get(n_outer * 16 * 9);
       void* dbasis = (uint8_t*)deq + n_outer * 16;
-      FK(flock_launch_eq_split(dr, nv, 0, deq, S->eqhi.get(16), st));
+      FlockEqBatch eb;
+      eb.n_jobs = 1;
+      for (int i = 0; i < nv; i++) u2(rout[i], eb.r[i]);
+      eb.jobs[0] = {deq, S->eqhi.get(16), nv, 0, 0, nv, 0};
+      FK(flock_launch_eq_tables(eb, st));
       FK(flock_launch_zc1_eq_basis(deq, n_outer, S->d_r1t, dbasis, st));
       const int grid = 152;
       void* dpart = S->part.get((size_t)grid * 192 * 16);
@@ -767,12 +806,11 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       bool grp, small;
       int a_bits, m_bits, f0, lob;
       F dinv;
-      std::vector<F> vars;  // the variables of the split tables
+      int n_vars;  // variables of the split tables: the round's, less the m_bits after the first a_bits where grp
     };
     auto round_eq = [&](int i) {
-      std::vector<F> rr(r.begin() + 6 + i + 1, r.end());
-      const int nv = (int)rr.size();
-      // lowest variables of rr that are fixed challenges: phi8 ones (r7, r8)
+      const int nv = m - (6 + i + 1);
+      // lowest of the round's variables r[7 + i ..] that are fixed challenges: phi8 ones (r7, r8)
       // and shift ones (r9..r12); rounds 0..5 factor their eq weight
       RoundEq q;
       q.a_bits = std::max(0, 2 - i);
@@ -784,58 +822,55 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       q.dinv = F::one();
       if (q.grp) {
         for (int k = q.f0; k < 13; k++) q.dinv = q.dinv * (F::one() + r[k]);
-        std::vector<F> rg(rr.begin(), rr.begin() + q.a_bits);
-        rg.insert(rg.end(), rr.begin() + q.a_bits + q.m_bits, rr.end());
         q.lob = std::min(nv - q.m_bits, 8);
-        q.vars = std::move(rg);
+        q.n_vars = nv - q.m_bits;
       } else if (q.small) {
         q.lob = nv;  // one table over all variables
-        q.vars = std::move(rr);
+        q.n_vars = nv;
       } else {
         // a CTA takes whole rows of 2^lob pairs: rows of 2^(nv - 10) pairs,
         // at least 2^8 (one pair per thread) and at most 2^12, keep the grid
         // near 608 CTAs while the round has pairs for it (rows of 2^12 left
         // rounds 7..13 on 1..64 CTAs, ~90 us each)
         q.lob = std::min(nv, std::max(8, std::min(12, nv - 10)));
-        q.vars = std::move(rr);
+        q.n_vars = nv;
       }
       return q;
     };
     std::vector<RoundEq> qs;
     std::vector<std::pair<size_t, size_t>> eq_off;  // (lo, hi) F128 offsets in zceq
     {
-      std::vector<F> vars;
-      std::vector<size_t> var_off;
-      size_t tot = 0, max_entries = 0;
+      size_t tot = 0;
       for (int i = 0; i < n_mlv; i++) {
         qs.push_back(round_eq(i));
         const RoundEq& q = qs.back();
-        const int hb = (int)q.vars.size() - q.lob;
+        const int hb = q.n_vars - q.lob;
         if (q.lob > 28 || hb > 28) throw Fail(FLOCK_ERR_SHAPE, "eq split");
-        var_off.push_back(vars.size());
-        vars.insert(vars.end(), q.vars.begin(), q.vars.end());
         eq_off.push_back({tot, tot + ((size_t)1 << q.lob)});
         tot += ((size_t)1 << q.lob) + ((size_t)1 << hb);
-        max_entries = std::max(max_entries, ((size_t)1 << q.lob) + ((size_t)1 << hb));
       }
-      F* dvars = (F*)S->zcr.get(vars.size() * 16 + 16);
-      h2d(*S, dvars, vars.data(), vars.size() * 16);
       F* deq = (F*)S->zceq.get(tot * 16);
+      FlockEqBatch eb;
+      eb.n_jobs = 0;
+      for (int k = 6; k < m; k++) u2(r[k], eb.r[k - 6]);
       // a small round's table comes out of the small round before it
-      std::vector<FlockEqJob> jobs;
       for (int i = 0; i < n_mlv; i++)
-        if (i == 0 || !qs[i].small || !qs[i - 1].small)
-          jobs.push_back({dvars + var_off[i], deq + eq_off[i].first, deq + eq_off[i].second, qs[i].lob,
-                          (int)qs[i].vars.size() - qs[i].lob});
-      auto* djobs = (FlockEqJob*)S->zcjobs.get(jobs.size() * sizeof(FlockEqJob));
-      h2d(*S, djobs, jobs.data(), jobs.size() * sizeof(FlockEqJob));
-      FK(flock_launch_eq_split_multi(djobs, (int)jobs.size(), max_entries, st));
+        if (i == 0 || !qs[i].small || !qs[i - 1].small) {
+          if (eb.n_jobs >= FLOCK_EQ_JOBS) throw Fail(FLOCK_ERR_SHAPE, "eq tables");
+          const RoundEq& q = qs[i];
+          eb.jobs[eb.n_jobs++] = {deq + eq_off[i].first, deq + eq_off[i].second, q.lob, q.n_vars - q.lob, i + 1,
+                                  q.grp ? q.a_bits : q.n_vars, q.grp ? q.m_bits : 0};
+        }
+      FK(flock_launch_eq_tables(eb, st));
     }
     // The last rounds, from kHostTailPairs pairs down, run on the host: a GPU
     // round of a few hundred pairs is a latency-bound launch plus a round
     // trip (~20 us), the same round on the host a few microseconds.
     int host_from = n_mlv;
     while (host_from > 1 && (rows0 >> host_from) <= kHostTailPairs && !qs[host_from - 1].grp) host_from--;
+    // the last device round writes its tables where the host reads them
+    const size_t tail_n = host_from < n_mlv ? (rows0 >> host_from) * 2 : 0;
+    void* tail_out = tail_n && host_from > 0 && qs[host_from - 1].small ? host_out(*S, 0, 2 * tail_n * 16) : nullptr;
     for (int i = 0; i < host_from; i++) {
       const size_t n_pairs = rows0 >> (i + 1);  // pairs of the round-i table
       const RoundEq& q = qs[i];
@@ -855,8 +890,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       } else if (q.small) {
         grid = flock_zc_small_grid(n_pairs);
         dpart = part_buf(*S, (size_t)grid * 2 * 16);
-        FK(flock_launch_zc_round_small(i == 0 ? da : curA, i == 0 ? db : curB, n_pairs, i == 0, rp, dlag,
-                                       i == 0 ? dA0 : nxtA, i == 0 ? dB0 : nxtB, elo,
+        void *oa = i == 0 ? dA0 : nxtA, *ob = i == 0 ? dB0 : nxtB;
+        if (tail_out && i == host_from - 1) {
+          oa = tail_out;
+          ob = (F*)tail_out + tail_n;
+        }
+        FK(flock_launch_zc_round_small(i == 0 ? da : curA, i == 0 ? db : curB, n_pairs, i == 0, rp, dlag, oa, ob, elo,
                                        (F*)S->zceq.p + eq_off[std::min(i + 1, n_mlv - 1)].first, dpart, st));
       } else {
         grid = (int)std::max<size_t>(std::min<size_t>(n_pairs >> q.lob, 152 * 4), 1);
@@ -895,8 +934,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       // remaining variables
       const size_t n_in = (rows0 >> host_from) * 2;
       std::vector<F> tA(n_in), tB(n_in);
-      d2h(*S, tA.data(), curA, n_in * 16);
-      d2h(*S, tB.data(), curB, n_in * 16);
+      if (tail_out) {  // that round's wait has passed
+        std::memcpy(tA.data(), tail_out, n_in * 16);
+        std::memcpy(tB.data(), (const F*)tail_out + n_in, n_in * 16);
+      } else {
+        d2h2(*S, tA.data(), curA, n_in * 16, tB.data(), curB, n_in * 16);
+      }
       auto bind = [](std::vector<F>& v, F rr) {
         hf::bind_pairs(v.data(), v.size() / 2, rr);
         v.resize(v.size() / 2);
@@ -941,8 +984,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     std::vector<std::pair<F, F>> lc_rounds;
     std::vector<F> z_partial(64);
     {
-      void* dxr = S->small.get(inner_rest * 16);
-      h2d(*S, dxr, x_in.data(), inner_rest * 16);
+      const void* dxr = staged(*S, S->small, x_in.data(), inner_rest * 16);
       void* deqin = S->eqin.get(FLOCK_K * 16);
       FK(flock_launch_lc_quirky_eq(dlag, dxr, inner_rest, deqin, st));
       void* dcomb = S->comb.get(FLOCK_K * 16);
@@ -959,13 +1001,15 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       FK(flock_launch_lc_partial_fold(ds, n_stripes, S->eqlo.p, S->eqhi.p, lob, dpart, grid, st));
       void* dzv = S->zvec.get(FLOCK_K * 16);
       FK(flock_launch_reduce_rows(dpart, grid, FLOCK_K, dzv, st));
-      CK(cudaMemcpyAsync(S->zvec0.get(FLOCK_K * 16), dzv, FLOCK_K * 16, cudaMemcpyDeviceToDevice, st));
       // product sumcheck on (comb, z_vec) binding the top variable
       // (lincheck.rs:1242-1300): the same round as the chain shift sumcheck
       // Rounds over at most kHostTailLincheck entries (and the final bind)
       // run on the host from the tables the last device round left, as
       // chain_round_kernel computes them: bind the top variable, then
       // q(1) = sum W_hi g_hi, q(inf) = sum (W_lo + W_hi)(g_lo + g_hi).
+      // the first bind leaves z_vec as it is (the ring switch reads it), the
+      // last device round leaves its tables where the host reads them
+      void *curW = dcomb, *curg = dzv;
       size_t len = FLOCK_K;
       int t = 0;
       for (; t < inner_rest; t++) {
@@ -975,7 +1019,19 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         if (t > 0) len /= 2;
         const int grid = flock_chain_round_grid(len);
         void* dpart = part_buf(*S, (size_t)grid * 2 * 16);
-        FK(flock_launch_chain_round(dcomb, dzv, len, t > 0, rp, dpart, grid, st));
+        void *oW = curW, *og = t == 1 ? S->zvec1.get(FLOCK_K / 2 * 16) : curg;
+        if (t > 0 && (t + 1 == inner_rest || len / 2 <= kHostTailLincheck)) {
+          void* out = host_out(*S, 0, 2 * len * 16);
+          if (out) {
+            oW = out;
+            og = (F*)out + len;
+          }
+        }
+        FK(flock_launch_chain_round(curW, curg, len, t > 0, rp, oW, og, dpart, grid, st));
+        if (t > 0) {
+          curW = oW;
+          curg = og;
+        }
         auto msg = reduce_partials(*S, dpart, grid, 2);
         tr.observe(msg[0]);
         tr.observe(msg[1]);
@@ -983,8 +1039,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         lc_rr.push_back(tr.sample());
       }
       std::vector<F> hW(len), hg(len);  // the tables bound up to round t - 1 (2 x the next length)
-      d2h(*S, hW.data(), dcomb, len * 16);
-      d2h(*S, hg.data(), dzv, len * 16);
+      if (curW == host_out(*S, 0, 2 * len * 16)) {  // that round's wait has passed
+        std::memcpy(hW.data(), curW, len * 16);
+        std::memcpy(hg.data(), curg, len * 16);
+      } else {
+        d2h2(*S, hW.data(), curW, len * 16, hg.data(), curg, len * 16);
+      }
       auto bind_top = [](std::vector<F>& v, F rr) {
         hf::bind_halves(v.data(), v.size() / 2, rr);
         v.resize(v.size() / 2);
@@ -1062,7 +1122,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         void* dpart = part_buf(*S, (size_t)grid * 2 * 16);
         uint64_t rp[2] = {0, 0};
         if (k > 0) u2(rs.back(), rp);
-        FK(flock_launch_chain_round(dW, dg, h, k > 0, rp, dpart, grid, st));
+        FK(flock_launch_chain_round(dW, dg, h, k > 0, rp, dW, dg, dpart, grid, st));
         auto sm = reduce_partials(*S, dpart, grid, 2);
         tr.observe(sm[0]);
         tr.observe(sm[1]);
@@ -1095,18 +1155,27 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       // ab claim: from the pre-sumcheck z_vec; c claim: from zerocheck round 1.
       std::vector<F> tail(r_inner_rest.begin() + 1, r_inner_rest.end());
       auto eq_tail = eq_table(tail);
-      void* det = S->small.get(128 * 16);
-      h2d(*S, det, eq_tail.data(), 128 * 16);
-      void* dsh = S->red.get(128 * 16);
-      FK(flock_launch_shv_from_zvec(S->zvec0.p, det, S->part.get(32 * 128 * 16), dsh, st));
+      const void* det = staged(*S, S->small, eq_tail.data(), 128 * 16);
+      void* hsh = host_out(*S, 0, 128 * 16);
+      void* dsh = hsh ? hsh : S->red.get(128 * 16);
+      FK(flock_launch_shv_from_zvec(S->zvec.p, det, S->part.get(32 * 128 * 16), dsh, st));
       s_hat[0].resize(128);
-      d2h(*S, s_hat[0].data(), dsh, 128 * 16);
+      // the basis tables need nothing of the wait below: both pairs are queued before it
+      FlockEqBatch eb;
+      eb.n_jobs = 0;
+      for (int k = 0; k < 2; k++)
+        eq_job(eb, std::vector<F>(xs[k]->begin() + 1, xs[k]->end()), rs_lo, *tlo[k], *thi[k]);
+      FK(flock_launch_eq_tables(eb, st));
+      if (hsh) {
+        CK(flock_stream_wait(st, &S->waits));
+        std::memcpy(s_hat[0].data(), hsh, 128 * 16);
+      } else {
+        d2h(*S, s_hat[0].data(), dsh, 128 * 16);
+      }
       s_hat[1] = shv_c;
     }
     for (int k = 0; k < 2; k++) {
       tr.label("flock-ring-switch-v0");
-      std::vector<F> suffix(xs[k]->begin() + 1, xs[k]->end());
-      eq_split_dev(*S, suffix, rs_lo, *tlo[k], *thi[k]);
       tr.observe_slice(s_hat[k].data(), 128);
       auto rpp = tr.sample_vec(7);
       eqr[k] = eq_table(rpp);
@@ -1163,14 +1232,14 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     std::vector<F> ood_vals;
     void* dgr = S->grind.get(64);
     int grind_parity = 0;  // the grinds alternate two result slots, both cleared here once
-    CK(cudaMemsetAsync(dgr, 0xFF, 16, st));
+    if (!(S->pin && S->host_atomics)) CK(cudaMemsetAsync(dgr, 0xFF, 16, st));
     auto grind = [&](uint32_t bits) {
       uint8_t dg[32];
       tr.digest(dg);
       uint64_t nonce = 0;
       uint64_t local_best = 0;
-      uint64_t* h_best = S->pin ? reinterpret_cast<uint64_t*>(S->pin + kPinH2D) : &local_best;
-      FK(flock_grind(dg, bits, dgr, &grind_parity, h_best, st, &S->waits, &nonce));
+      uint64_t* h_best = S->pin ? reinterpret_cast<uint64_t*>(S->pin + kPinH2D + kPinD2H - kGrindSlot) : &local_best;
+      FK(flock_grind(dg, bits, dgr, &grind_parity, h_best, S->pin && S->host_atomics, st, &S->waits, &nonce));
       tr.absorb_nonce(nonce);
       return nonce;
     };
@@ -1246,10 +1315,13 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         dsk = S->skl[nvars].get((size_t)nvars * 32 * 16);
         h2d(*S, dsk, sk.lin.data(), (size_t)nvars * 32 * 16);
       }
-      uint32_t* dq = (uint32_t*)S->qbuf.get(q.size() * 4);
-      h2d(*S, dq, q.data(), q.size() * 4);
-      void* dal = S->abuf.get(q.size() * 16);
-      h2d(*S, dal, aw.data(), q.size() * 16);
+      // the queries behind their weights, in one copy
+      std::vector<uint8_t> qa(q.size() * 20);
+      std::memcpy(qa.data(), aw.data(), q.size() * 16);
+      std::memcpy(qa.data() + q.size() * 16, q.data(), q.size() * 4);
+      void* dal = S->qbuf.get(qa.size());
+      h2d(*S, dal, qa.data(), qa.size());
+      const uint32_t* dq = (const uint32_t*)((const uint8_t*)dal + q.size() * 16);
       const int log_d = ilog2(block_len);
       void* dLO = S->LO.get(flock_induce_basis_rows_bytes(nvars, log_d, (int)q.size()));
       void* dbs = S->basis.get(((size_t)16) << nvars);
@@ -1825,8 +1897,7 @@ static int verify_impl(ProverState* S, const uint8_t* data, size_t len, const ch
       auto lag_z = LG.at(z, 0);
       void* dlag = S->lag.get(64 * 16);
       h2d(*S, dlag, lag_z.data(), 64 * 16);
-      void* dxr = S->small.get(inner_rest * 16);
-      h2d(*S, dxr, x_in.data(), inner_rest * 16);
+      const void* dxr = staged(*S, S->small, x_in.data(), inner_rest * 16);
       void* deqin = S->eqin.get(FLOCK_K * 16);
       FK(flock_launch_lc_quirky_eq(dlag, dxr, inner_rest, deqin, st));
       void* dcomb = S->comb.get(FLOCK_K * 16);

@@ -450,10 +450,16 @@ reduce_rows_kernel(const gf128* __restrict__ in, size_t count, int width, gf128*
 // to some 2^16 entries (13 + 1 variables: 18 us with up to seven products a
 // chunk entry and eight entries a thread, 7.4 us here), by the products beyond.
 constexpr int EQ_CHUNK = 7, EQ_MAX_CHUNKS = 4, EQ_HALF = 4;
-// One table pair, CTA `blk` of `nblk` (the calling kernel's grid slice).
-__device__ __forceinline__ void eq_split_body(const gf128* __restrict__ r, int lo_bits, int hi_bits,
-                                              gf128* __restrict__ lo, gf128* __restrict__ hi, size_t blk,
-                                              size_t nblk) {
+// Table pair blockIdx.y of the batch, CTA blockIdx.x of gridDim.x. The
+// variables and jobs are kernel arguments: no copy precedes the launch.
+__global__ void __launch_bounds__(256) eq_tables_kernel(const __grid_constant__ FlockEqBatch q) {
+  const FlockEqJob& job = q.jobs[blockIdx.y];
+  const int lo_bits = job.lo_bits, hi_bits = job.hi_bits;
+  gf128 *lo = (gf128*)job.lo, *hi = (gf128*)job.hi;
+  auto var = [&](int k) {
+    const uint64_t* v = q.r[job.first + k + (k >= job.skip_at ? job.skip_n : 0)];
+    return gf128{{(uint32_t)v[0], (uint32_t)(v[0] >> 32), (uint32_t)v[1], (uint32_t)(v[1] >> 32)}};
+  };
   __shared__ gf128 half_t[2 * EQ_MAX_CHUNKS][2][1 << EQ_HALF];
   __shared__ gf128 t[2 * EQ_MAX_CHUNKS][1 << EQ_CHUNK];
   const int nc_lo = (lo_bits + EQ_CHUNK - 1) / EQ_CHUNK, nc = nc_lo + (hi_bits + EQ_CHUNK - 1) / EQ_CHUNK;
@@ -473,7 +479,7 @@ __device__ __forceinline__ void eq_split_body(const gf128* __restrict__ r, int l
     gf128 acc = gf_one();
 #pragma unroll 1
     for (int k = 0; k < hv; k++) {
-      gf128 rk = gf_load(&r[v0 + (h ? EQ_HALF : 0) + k]);
+      gf128 rk = var(v0 + (h ? EQ_HALF : 0) + k);
       if (!((v >> k) & 1)) rk.w[0] ^= 1;
       acc = k == 0 ? rk : gf_mul(acc, rk);
     }
@@ -492,7 +498,7 @@ __device__ __forceinline__ void eq_split_body(const gf128* __restrict__ r, int l
   __syncthreads();
   const size_t nlo = (size_t)1 << lo_bits, nhi = (size_t)1 << hi_bits;
 #pragma unroll 1
-  for (size_t e = blk * blockDim.x + threadIdx.x; e < nlo + nhi; e += nblk * blockDim.x) {
+  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < nlo + nhi; e += (size_t)gridDim.x * blockDim.x) {
     const bool is_lo = e < nlo;
     const size_t idx = is_lo ? e : e - nlo;
     const int c0 = is_lo ? 0 : nc_lo, c1 = is_lo ? nc_lo : nc;
@@ -510,20 +516,6 @@ __device__ __forceinline__ void eq_split_body(const gf128* __restrict__ r, int l
 size_t eq_grid(size_t n) {
   const size_t g = (n + 255) / 256;
   return g < 1 ? 1 : g > 304 ? 304 : g;
-}
-
-__global__ void __launch_bounds__(256)
-eq_split_kernel(const gf128* __restrict__ r, int lo_bits, int hi_bits, gf128* __restrict__ lo,
-                gf128* __restrict__ hi) {
-  eq_split_body(r, lo_bits, hi_bits, lo, hi, blockIdx.x, gridDim.x);
-}
-
-// Many table pairs in one launch: job blockIdx.y, its tables split over the
-// x dimension.
-__global__ void __launch_bounds__(256)
-eq_split_multi_kernel(const FlockEqJob* __restrict__ jobs) {
-  const FlockEqJob j = jobs[blockIdx.y];
-  eq_split_body((const gf128*)j.r, j.lo_bits, j.hi_bits, (gf128*)j.lo, (gf128*)j.hi, blockIdx.x, gridDim.x);
 }
 
 // One multilinear round (zerocheck.rs:690-760, multilinear.rs:632-675), with
@@ -901,19 +893,18 @@ int flock_launch_reduce_rows(const void* in, size_t count, int width, void* out,
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
-int flock_launch_eq_split_multi(const FlockEqJob* d_jobs, int n_jobs, size_t max_entries, cudaStream_t st) {
-  if (n_jobs <= 0) return FLOCK_OK;
-  if (n_jobs > 65535) return FLOCK_ERR_SHAPE;
-  const size_t gx = eq_grid(max_entries);
-  eq_split_multi_kernel<<<dim3((unsigned)gx, (unsigned)n_jobs), 256, 0, st>>>(d_jobs); flock_count_launch();
-  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
-}
-
-int flock_launch_eq_split(const void* r, int lo_bits, int hi_bits, void* lo, void* hi, cudaStream_t st) {
-  if (lo_bits < 0 || hi_bits < 0 || lo_bits > EQ_CHUNK * EQ_MAX_CHUNKS || hi_bits > EQ_CHUNK * EQ_MAX_CHUNKS)
-    return FLOCK_ERR_SHAPE;
-  const size_t grid = eq_grid(((size_t)1 << lo_bits) + ((size_t)1 << hi_bits));
-  eq_split_kernel<<<(unsigned)grid, 256, 0, st>>>((const gf128*)r, lo_bits, hi_bits, (gf128*)lo, (gf128*)hi); flock_count_launch();
+int flock_launch_eq_tables(const FlockEqBatch& q, cudaStream_t st) {
+  if (q.n_jobs < 1) return FLOCK_OK;
+  size_t most = 0;
+  for (int i = 0; i < q.n_jobs; i++) {
+    const FlockEqJob& j = q.jobs[i];
+    if (j.lo_bits < 0 || j.hi_bits < 0 || j.lo_bits > EQ_CHUNK * EQ_MAX_CHUNKS || j.hi_bits > EQ_CHUNK * EQ_MAX_CHUNKS ||
+        j.first + j.lo_bits + j.hi_bits + j.skip_n > FLOCK_EQ_VARS)
+      return FLOCK_ERR_SHAPE;
+    most = std::max(most, ((size_t)1 << j.lo_bits) + ((size_t)1 << j.hi_bits));
+  }
+  eq_tables_kernel<<<dim3((unsigned)eq_grid(most), (unsigned)q.n_jobs), 256, 0, st>>>(q);
+  flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
