@@ -62,8 +62,13 @@ int flock_launch_zc_round_small(const void* in0, const void* in1, size_t n_pairs
 int flock_launch_bind_pairs(const void* A, const void* B, size_t n, const uint64_t rho[2], void* Aout, void* Bout,
                             cudaStream_t st);
 
-int flock_launch_lc_partial_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi,
-                                 int lo_bits, void* partials, int grid, cudaStream_t st);
+// z_vec[i] = sum over the outer indices o < 8 n_stripes of z[i, o] eq(o) (2^14
+// entries; n_stripes a multiple of 32, at most 2^19). scratch:
+// flock_lc_fold_scratch_bytes(n_stripes). fault: set to one if a wait inside
+// the kernel gave up (the result is then unusable).
+size_t flock_lc_fold_scratch_bytes(size_t n_stripes);
+int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi, int lo_bits,
+                         void* scratch, void* z_vec, int* fault, cudaStream_t st);
 int flock_launch_lc_comb(const uint32_t* a_ptr, const uint32_t* a_idx, const uint32_t* b_ptr,
                          const uint32_t* b_idx, const void* eq, const uint64_t alpha[2], const uint64_t beta[2],
                          int pin, void* comb, cudaStream_t st);

@@ -1,94 +1,191 @@
 // Lincheck kernels (crates/flock-core/src/lincheck.rs:1480-1660).
 //
 //  * partial fold: z_vec[i] = sum_outer z[i, outer] eq(x_outer, outer), read
-//    from the byte stripe (byte (outer/8)*2^14 + i holds 8 outer bits), one
-//    256-entry subset-sum table of eq per stripe, eight stripes per round
-//    (lincheck.rs:655-720);
+//    from the byte stripe (byte (outer/8)*2^14 + i holds 8 outer bits), as a
+//    bit-matrix product on the tensor cores (lincheck.rs:655-720);
 //  * comb: alpha * A0^T eq_inner + B0^T eq_inner (+ beta at the constant
 //    column) gathered column-wise from a CSC copy of the base matrices;
 //  (the product sumcheck rounds over (comb, z_vec), binding the top variable
 //  (lincheck.rs:1242-1300), run on flock_launch_chain_round).
 #include "flock_internal.h"
 #include "gf128.cuh"
+#include "tc.cuh"
 
 namespace {
 
-constexpr int PF_THREADS = 256;
-constexpr int PF_PER_THREAD = 16;                                    // bytes (columns) per thread
-constexpr int PF_SLICES = FLOCK_K / (PF_THREADS * PF_PER_THREAD);  // column slices: 4
+// The stripe fold as a bit-matrix product on the tensor cores (tc.cuh):
+// z_vec[i], bit e = parity over the outer indices o of eq(o)[e] z[i, o], so
+// M = 128 (the bits of eq), N = 2^14 columns, and the outer index is summed.
+//
+// A: the eq weights' bits as fp4, written once by eq_bits_kernel in the
+// operand layout, a plane (32 outer indices) being [128 rows e][16 bytes]: word
+// m of a row holds in its nibbles the bits 4 n + m of the plane. B: a thread
+// takes four stripes of four columns, gathers each column's four bytes with
+// byte permutations and masks them the same way, which expands 32 bits in five
+// operations. The bits of mask m stand for 0.5, 1, 2, 0.5 in B and for 2, 1,
+// 0.5, 2 in A, so every product is one or zero.
+//
+// A CTA owns FM_COLS columns and a range of the outer indices, in stages of
+// FM_STAGE indices and FM_BUFS buffers. Sixteen warps load, expand and store B
+// (words loaded FM_AHEAD stages before they are expanded) and count in on a
+// barrier; one thread of a further warp has the copy engine fetch A and issues
+// one MMA per 64 indices, so no expanding warp waits for another (one warp
+// doing both, with a block barrier per stage, took 352 us at 2^18 outer
+// indices: the tensor and shared-memory pipes at 29% and 22%). Subset-sum
+// tables of eight eq weights per stripe with a lookup per byte took 422 us;
+// this takes 241 us, and 28 us against 40 us at 2^14.
+constexpr int FM_PRODUCERS = 512, FM_THREADS = FM_PRODUCERS + 32;
+constexpr int FM_COLS = 256, FM_STAGE = 256, FM_BUFS = 4, FM_PLANES = FM_STAGE / 32, FM_AHEAD = 4;
+constexpr int FM_A_PLANE = 128 * 16, FM_B_PLANE = FM_COLS * 16;
+constexpr size_t FM_SMEM = (size_t)FM_BUFS * FM_PLANES * (FM_A_PLANE + FM_B_PLANE);
+constexpr int FM_MAX_PARTS = 7;  // 64 column tiles x 7 = 2.95 waves of one CTA per SM
+static_assert(FM_SMEM <= 232448, "fold shared memory above the 227 KB per-block limit");
+static_assert(FM_PRODUCERS == 64 * FM_PLANES, "a producer takes one column word of one plane");
 
-constexpr int PF_GROUP = 8;  // stripes per table round (64 outer indices)
-
-// CTA (slice, part): columns [slice * 4096, +4096) of the stripe groups
-// part, part + parts, ... Per round: 64 eq weights (one product each, 64
-// threads), PF_GROUP subset-sum tables of 256 entries, then every thread folds
-// its 16 bytes of each stripe. Grouping amortises the barriers and the table
-// build over eight stripes; the four column slices keep 64 accumulator
-// registers per thread affordable.
-__global__ void __launch_bounds__(PF_THREADS, 2)
-lc_partial_fold_kernel(const uint8_t* __restrict__ stripe, size_t n_stripes, const gf128* __restrict__ eq_lo,
-                       const gf128* __restrict__ eq_hi, int lo_bits, gf128* __restrict__ partials) {
-  // t8[v][q]: subset sums of stripe q's eight eq weights; entry (v, q) sits in
-  // bank group q, and lane l starts at stripe l mod 8, so eight consecutive
-  // lanes read eight distinct bank groups. e8v[r][q]: weight of bit r of stripe q.
-  __shared__ gf128 t8[256][PF_GROUP];
-  __shared__ gf128 e8v[8][PF_GROUP];
-  const int lane8 = threadIdx.x & 7;
-  gf128 acc[PF_PER_THREAD];
+// One warp per plane: lane = outer index, then lane = bit row.
+__global__ void __launch_bounds__(256)
+eq_bits_kernel(const gf128* __restrict__ eq_lo, const gf128* __restrict__ eq_hi, int lo_bits, size_t n_planes,
+               uint4* __restrict__ out) {
+  const size_t plane = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
+  if (plane >= n_planes) return;
+  const size_t o = plane * 32 + lane;
+  const gf128 e = gf_mul(gf_load(&eq_lo[o & (((size_t)1 << lo_bits) - 1)]), gf_load(&eq_hi[o >> lo_bits]));
 #pragma unroll
-  for (int k = 0; k < PF_PER_THREAD; k++) acc[k] = gf_zero();
-  const int slice = blockIdx.x % PF_SLICES;
-  const size_t part = blockIdx.x / PF_SLICES, parts = gridDim.x / PF_SLICES;
-  const size_t col0 = (size_t)slice * PF_THREADS * PF_PER_THREAD + (size_t)threadIdx.x * PF_PER_THREAD;
-  const size_t lo_mask = ((size_t)1 << lo_bits) - 1;
-  const size_t n_groups = n_stripes / PF_GROUP;
-  for (size_t g = part; g < n_groups; g += parts) {
-    const size_t s0 = g * PF_GROUP;
-    if (threadIdx.x < PF_GROUP * 8) {
-      size_t o = 8 * s0 + threadIdx.x;  // stripe threadIdx.x / 8, bit threadIdx.x % 8
-      e8v[threadIdx.x & 7][threadIdx.x >> 3] = gf_mul(eq_lo[o & lo_mask], eq_hi[o >> lo_bits]);
+  for (int k = 0; k < 4; k++) {
+    uint32_t row = 0;
+#pragma unroll 8
+    for (int b = 0; b < 32; b++) {
+      const uint32_t v = __ballot_sync(0xffffffffu, (e.w[k] >> b) & 1);
+      if (lane == b) row = v;
     }
-    // this thread's bytes of the group's stripes (loads overlap the table build)
-    uint4 bytes[PF_GROUP];
-#pragma unroll
-    for (int q = 0; q < PF_GROUP; q++)
-      bytes[q] = *reinterpret_cast<const uint4*>(stripe + (s0 + q) * FLOCK_K + col0);
-    __syncthreads();
-    // subset sums by a Gray walk: thread (c, q) owns t8[8c .. 8c+7][q], starts
-    // from the sum over the bits of 8c and adds one weight per entry
-    static_assert(PF_THREADS == 32 * PF_GROUP, "one thread per (8-entry run, stripe)");
-    {
-      const int q = threadIdx.x & 7, c = threadIdx.x >> 3;
-      gf128 acc8 = gf_zero();
-#pragma unroll
-      for (int r = 3; r < 8; r++)
-        if ((c >> (r - 3)) & 1) acc8 = gf_add(acc8, e8v[r][q]);
-#pragma unroll
-      for (int i = 0; i < 8; i++) {
-        if (i) acc8 = gf_add(acc8, e8v[(i & 1) ? 0 : (i & 2) ? 1 : 2][q]);
-        t8[8 * c + (i ^ (i >> 1))][q] = acc8;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int st = 0; st < PF_GROUP; st++) {
-      const int q = (lane8 + st) & (PF_GROUP - 1);  // rotated stripe
-      uint4 bq = bytes[0];
-#pragma unroll
-      for (int qq = 1; qq < PF_GROUP; qq++)
-        if (q == qq) bq = bytes[qq];
-      const uint32_t wds[4] = {bq.x, bq.y, bq.z, bq.w};
-#pragma unroll
-      for (int k = 0; k < PF_PER_THREAD; k++) {
-        uint32_t b = (wds[k >> 2] >> (8 * (k & 3))) & 255;
-        if (b) acc[k] = gf_add(acc[k], t8[b][q]);
-      }
-    }
-    __syncthreads();
+    out[plane * 128 + 32 * k + lane] = make_uint4((row & 0x11111111u) << 2, row & 0x22222222u, (row >> 2) & 0x11111111u,
+                                                  (row >> 1) & 0x44444444u);
   }
-  gf128* out = partials + part * FLOCK_K + col0;
+}
+
+// The bytes of one column of four stripes, expanded: a row of one B plane.
+__device__ __forceinline__ uint4 fm_expand(uint32_t w) {
+  return make_uint4(w & 0x11111111u, w & 0x22222222u, w & 0x44444444u, (w >> 3) & 0x11111111u);
+}
+
+__global__ void __launch_bounds__(FM_THREADS, 1)
+lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict__ eq_bits, int n_stages, int parts,
+                   uint32_t* __restrict__ partials, volatile int* fault) {
+  extern __shared__ __align__(128) uint8_t fm_smem[];  // A buffers, then B buffers
+  __shared__ uint64_t a_full[FM_BUFS], b_full[FM_BUFS], done[FM_BUFS];
+  __shared__ uint32_t tmem_slot;
+  constexpr uint32_t kABytes = FM_PLANES * FM_A_PLANE, kBBytes = FM_PLANES * FM_B_PLANE;
+  uint8_t* sa = fm_smem;
+  uint8_t* sb = fm_smem + FM_BUFS * kABytes;
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int tile = blockIdx.x % (FLOCK_K / FM_COLS), part = blockIdx.x / (FLOCK_K / FM_COLS);
+  const int s_begin = (int)((long long)n_stages * part / parts), s_end = (int)((long long)n_stages * (part + 1) / parts);
+  const int n = s_end - s_begin;  // at least one: parts <= n_stages
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
+  if (t == 0) {
+    for (int k = 0; k < FM_BUFS; k++) {
+      tc::mbar_init(&a_full[k], 1);
+      tc::mbar_init(&b_full[k], FM_PRODUCERS / 32);
+      tc::mbar_init(&done[k], 1);
+    }
+    tc::mbar_fence_init();
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  // columns 0..255: the counts; 256..287: the operands' scales, all one
+  const uint32_t tmem = tmem_slot, sf = tmem + 256;
+  if (warp < 4) tc::tmem_fill32(sf + ((uint32_t)(32 * warp) << 16), 0x7f7f7f7fu);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  bool ok = true;
+  if (t < FM_PRODUCERS) {
+    // column word cw (four columns) of plane g: stripes 4 g .. 4 g + 3 of a stage
+    const int cw = t & 63, g = t >> 6;
+    const uint8_t* src = stripe + (size_t)tile * FM_COLS + 4 * cw + (size_t)(s_begin * (FM_STAGE / 8) + 4 * g) * FLOCK_K;
+    uint32_t x[FM_AHEAD][4];
+    auto load = [&](int it, uint32_t (&v)[4]) {
 #pragma unroll
-  for (int k = 0; k < PF_PER_THREAD; k++) out[k] = acc[k];
+      for (int k = 0; k < 4; k++)
+        v[k] = *reinterpret_cast<const uint32_t*>(src + ((size_t)it * (FM_STAGE / 8) + k) * FLOCK_K);
+    };
+#pragma unroll
+    for (int k = 0; k < FM_AHEAD; k++)
+      if (k < n) load(k, x[k]);
+    for (int it0 = 0; it0 < n && ok; it0 += FM_AHEAD) {
+#pragma unroll
+      for (int k = 0; k < FM_AHEAD; k++) {
+        const int it = it0 + k, b = it % FM_BUFS;
+        if (it >= n) break;
+        if (it >= FM_BUFS) ok = tc::mbar_wait(&done[b], (it / FM_BUFS - 1) & 1);
+        if (!ok) break;
+        const uint32_t l01 = __byte_perm(x[k][0], x[k][1], 0x5140), h01 = __byte_perm(x[k][0], x[k][1], 0x7362);
+        const uint32_t l23 = __byte_perm(x[k][2], x[k][3], 0x5140), h23 = __byte_perm(x[k][2], x[k][3], 0x7362);
+        uint4* row = reinterpret_cast<uint4*>(sb + b * kBBytes + g * FM_B_PLANE) + cw;
+        row[0] = fm_expand(__byte_perm(l01, l23, 0x5410));
+        row[64] = fm_expand(__byte_perm(l01, l23, 0x7632));
+        row[128] = fm_expand(__byte_perm(h01, h23, 0x5410));
+        row[192] = fm_expand(__byte_perm(h01, h23, 0x7632));
+        if (it + FM_AHEAD < n) load(it + FM_AHEAD, x[k]);
+        tc::fence_smem_for_mma();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&b_full[b]);
+      }
+    }
+  } else if (lane == 0) {
+    auto load_a = [&](int it) {
+      uint64_t* bar = &a_full[it % FM_BUFS];
+      tc::mbar_expect(bar, kABytes);
+      tc::bulk_load(sa + (it % FM_BUFS) * kABytes, eq_bits + (size_t)(s_begin + it) * kABytes, kABytes, bar);
+    };
+    for (int it = 0; it < FM_BUFS - 1 && it < n; it++) load_a(it);
+    for (int it = 0; it < n && ok; it++) {
+      const int b = it % FM_BUFS, j = it + FM_BUFS - 1;
+      ok = tc::mbar_wait(&a_full[b], (it / FM_BUFS) & 1) && tc::mbar_wait(&b_full[b], (it / FM_BUFS) & 1);
+      if (!ok) break;
+      tc::fence_after();
+      const uint32_t a0 = tc::smem_addr(sa + b * kABytes), b0 = tc::smem_addr(sb + b * kBBytes);
+#pragma unroll
+      for (int q = 0; q < FM_PLANES / 2; q++)
+        tc::mma_mxf4(tmem, tc::operand(a0 + 2 * q * FM_A_PLANE, FM_A_PLANE, 128),
+                     tc::operand(b0 + 2 * q * FM_B_PLANE, FM_B_PLANE, 128), tc::mxf4_desc(128, FM_COLS), sf, sf + 16,
+                     it > 0 || q > 0);
+      tc::mma_commit(&done[b]);
+      // the buffer of stage j: its last MMAs (stage j - FM_BUFS = it - 1)
+      if (j < n) {
+        if (j >= FM_BUFS) ok = tc::mbar_wait(&done[j % FM_BUFS], (j / FM_BUFS - 1) & 1);
+        if (ok) load_a(j);
+      }
+    }
+  }
+  // every MMA is done when the last stage's commit has arrived
+  ok = tc::mbar_wait(&done[(n - 1) % FM_BUFS], ((n - 1) / FM_BUFS) & 1) && ok;
+  if (!ok) *fault = 1;
+  __syncwarp();
+  tc::fence_after();
+  // counts -> parities: lane = row e of quadrant warp & 3, a ballot per column
+  if (t < FM_PRODUCERS) {
+    const int quad = warp & 3, c_begin = (warp >> 2) * (FM_COLS / 4);
+    for (int c0 = c_begin; c0 < c_begin + FM_COLS / 4; c0 += 32) {
+      uint32_t r[32];
+      tc::tmem_load32(tmem + ((uint32_t)(32 * quad) << 16) + c0, r);
+      uint32_t keep = 0;
+#pragma unroll
+      for (int j = 0; j < 32; j++) {
+        // counts below 2^23: the sum's low mantissa bit is the parity
+        const uint32_t v = __ballot_sync(0xffffffffu, __float_as_uint(__uint_as_float(r[j]) + 8388608.0f) & 1);
+        if (lane == j) keep = v;
+      }
+      // row r of B holds column 4 (r mod 64) + r / 64 of the tile
+      const int rr = c0 + lane, col = tile * FM_COLS + 4 * (rr & 63) + (rr >> 6);
+      partials[((size_t)part * FLOCK_K + col) * 4 + quad] = keep;
+    }
+  }
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
 // comb[c] = alpha * sum_{r in colA(c)} eq[r] + sum_{r in colB(c)} eq[r] (+ beta at pin).
@@ -141,15 +238,31 @@ inline gf128 to_gf(const uint64_t v[2]) {
 
 }  // namespace
 
-// grid = number of partial rows (stripe-group partitions); partials: grid x 2^14.
-int flock_launch_lc_partial_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi,
-                                 int lo_bits, void* partials, int grid, cudaStream_t st) {
-  if (n_stripes % PF_GROUP != 0) return FLOCK_ERR_SHAPE;
-  lc_partial_fold_kernel<<<grid * PF_SLICES, PF_THREADS, 0, st>>>((const uint8_t*)stripe, n_stripes,
-                                                                  (const gf128*)eq_lo, (const gf128*)eq_hi, lo_bits,
-                                                                  (gf128*)partials);
+size_t flock_lc_fold_scratch_bytes(size_t n_stripes) {
+  return n_stripes / 4 * FM_A_PLANE + (size_t)FM_MAX_PARTS * FLOCK_K * 16;
+}
+
+int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi, int lo_bits,
+                         void* scratch, void* z_vec, int* fault, cudaStream_t st) {
+  constexpr size_t kPerStage = FM_STAGE / 8;
+  if (n_stripes == 0 || n_stripes % kPerStage != 0 || n_stripes > ((size_t)1 << 19)) return FLOCK_ERR_SHAPE;
+  const size_t n_planes = n_stripes / 4;
+  uint8_t* bits = (uint8_t*)scratch;
+  void* partials = bits + n_planes * FM_A_PLANE;
+  eq_bits_kernel<<<(unsigned)((n_planes + 7) / 8), 256, 0, st>>>((const gf128*)eq_lo, (const gf128*)eq_hi, lo_bits,
+                                                                n_planes, (uint4*)bits);
   flock_count_launch();
-  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+  if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
+  flock_once_per_device((const void*)lc_fold_mma_kernel, [] {
+    cudaFuncSetAttribute(lc_fold_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FM_SMEM);
+  });
+  const int n_stages = (int)(n_stripes / kPerStage);
+  const int parts = n_stages < FM_MAX_PARTS ? n_stages : FM_MAX_PARTS;
+  lc_fold_mma_kernel<<<(unsigned)(FLOCK_K / FM_COLS * parts), FM_THREADS, FM_SMEM, st>>>(
+      (const uint8_t*)stripe, bits, n_stages, parts, (uint32_t*)(parts > 1 ? partials : z_vec), fault);
+  flock_count_launch();
+  if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
+  return parts > 1 ? flock_launch_reduce_rows(partials, parts, FLOCK_K, z_vec, st) : FLOCK_OK;
 }
 
 int flock_launch_lc_comb(const uint32_t* a_ptr, const uint32_t* a_idx, const uint32_t* b_ptr, const uint32_t* b_idx,

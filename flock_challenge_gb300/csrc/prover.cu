@@ -272,6 +272,9 @@ struct Open {
 }  // namespace
 
 // ============================================================================
+constexpr size_t kPinH2D = (size_t)4 << 20, kPinD2H = (size_t)1 << 20, kMapped = (size_t)256 << 10;
+constexpr size_t kPinOpen = (size_t)4 << 20;
+constexpr size_t kGrindSlot = 64;  // the last bytes of the pinned read area: a grind's result, the fault word
 constexpr int kSklMax = 40;  // induced-basis variable counts below this
 constexpr int kKernelSpans = 4;  // witness, L0 NTT, L0 Merkle tree, zerocheck round 1
 
@@ -309,6 +312,12 @@ struct ProverState {
   // host memory, so reading a round's message needs only the stream sync.
   uint8_t* mapped = nullptr;
   void* mapped_dev = nullptr;
+  // A word kernels set when a wait inside them gave up (bounded, tc.cuh); read
+  // with the next result. Host memory, or device memory nobody reads without it.
+  int* fault() {
+    return pin ? reinterpret_cast<int*>(pin + kPinH2D + kPinD2H - kGrindSlot / 2) : reinterpret_cast<int*>(grind.get(64)) + 8;
+  }
+  bool faulted() { return pin && *reinterpret_cast<volatile int*>(fault()) != 0; }
   bool host_atomics = false;  // the device's atomics reach pinned host memory (cudaDevAttrHostNativeAtomicSupported)
   // The host's waits for the stream (flock_stream_wait) in the current proof.
   WaitStats waits;
@@ -329,9 +338,6 @@ struct ProverState {
 
 namespace {
 
-constexpr size_t kPinH2D = (size_t)4 << 20, kPinD2H = (size_t)1 << 20, kMapped = (size_t)256 << 10;
-constexpr size_t kPinOpen = (size_t)4 << 20;
-constexpr size_t kGrindSlot = 64;  // the last bytes of the pinned read area: a grind's result
 // Zerocheck rounds of at most this many pairs run on the host (see the round loop).
 constexpr size_t kHostTailPairs = 512;
 // Lincheck product-sumcheck rounds over at most this many entries run on the host.
@@ -640,6 +646,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     CK(flock_stream_wait(S->st, &S->waits, false));
     S->pin_off = 0;
     S->pin_open_off = 0;
+    if (S->pin) *S->fault() = 0;
     const int m = 14 + n_log;
     LigCfg cfg;
     if (!lig_config(m, 0, cfg)) return FLOCK_ERR_SHAPE;
@@ -996,11 +1003,9 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       int lob = n_outer_log / 2;
       eq_split_dev(*S, x_out, lob, S->eqlo, S->eqhi);
       size_t n_stripes = ((size_t)1 << n_outer_log) / 8;
-      int grid = (int)std::min<size_t>(n_stripes / 8, 152);  // partial rows (stripe-group partitions)
-      void* dpart = S->part.get((size_t)grid * FLOCK_K * 16);
-      FK(flock_launch_lc_partial_fold(ds, n_stripes, S->eqlo.p, S->eqhi.p, lob, dpart, grid, st));
       void* dzv = S->zvec.get(FLOCK_K * 16);
-      FK(flock_launch_reduce_rows(dpart, grid, FLOCK_K, dzv, st));
+      FK(flock_launch_lc_fold(ds, n_stripes, S->eqlo.p, S->eqhi.p, lob,
+                              S->part.get(flock_lc_fold_scratch_bytes(n_stripes)), dzv, S->fault(), st));
       // product sumcheck on (comb, z_vec) binding the top variable
       // (lincheck.rs:1242-1300): the same round as the chain shift sumcheck
       // Rounds over at most kHostTailLincheck entries (and the final bind)
@@ -1064,6 +1069,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       bind_top(hg, lc_rr.back());
       std::copy(hg.begin(), hg.begin() + 64, z_partial.begin());
     }
+    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "stripe fold");
     tr.observe_slice(z_partial.data(), 64);
     const F lc_skip = tr.sample();  // lincheck's skip challenge: the ab claim's z_skip
     std::vector<F> r_inner_rest(lc_rr.rbegin(), lc_rr.rend());
