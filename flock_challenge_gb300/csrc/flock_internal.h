@@ -25,7 +25,8 @@ int flock_launch_merkle(const void* d_data, size_t n_leaves, size_t leaf_bytes, 
 
 // ---- protocol kernels ------------------------------------------------------
 struct ZcRound1Tables;
-// eq_basis: n_outer x 8 F128 from flock_launch_zc1_eq_basis.
+// eq_basis: n_outer x 8 F128 from flock_launch_zc1_eq_basis. Rows of partials: 64
+// P^AB sums, then with c (may be null) the 128 sums of the c statistic.
 int flock_launch_zc_round1(const void* a, const void* b, const void* c, size_t n_outer, const void* eq_basis,
                            const ZcRound1Tables* d_tables, void* partials, int grid, cudaStream_t st);
 // out[8 xo + k] = phi8(2^k) eq_out[xo] for xo < n_outer (round 1's table basis).

@@ -30,10 +30,9 @@
 
 namespace {
 
-#ifndef ZC1_THREADS
-#define ZC1_THREADS 384
-#endif
-constexpr int R1_THREADS = ZC1_THREADS;  // 12 warps, one block per SM
+// One block per SM: 12 warps with the c statistic (168 registers), 16 without.
+template <bool WITH_C>
+constexpr int kR1Threads = WITH_C ? 384 : 512;
 #ifndef ZC1_PAR_UNROLL
 #define ZC1_PAR_UNROLL 1
 #endif
@@ -227,16 +226,23 @@ __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
 // of the points to bytes, and each lane then handles two of the 64 points.
 constexpr int R1_ROW = 20;
 constexpr int R1_XCH = 16 * R1_ROW;
-constexpr int R1_WARPS = R1_THREADS / 32;
-constexpr size_t R1_SMEM = (size_t)8 * 4 * 256 * 16 + (size_t)R1_WARPS * 256 * 16 + (size_t)R1_WARPS * R1_XCH * 4;
-static_assert(R1_SMEM <= 232448, "round-1 shared memory above the 227 KB per-block limit");
+template <bool WITH_C>
+constexpr size_t kR1Smem = (size_t)8 * 4 * 256 * 16 + (size_t)(kR1Threads<WITH_C> / 32) * (256 * 16 + R1_XCH * 4);
+static_assert(kR1Smem<true> <= 232448 && kR1Smem<false> <= 232448,
+              "round-1 shared memory above the 227 KB per-block limit");
 
 // grid: each warp walks outer blocks; lane: xm = lane & 15 (producer row
 // group, then point quad), h = lane >> 4 (row half, then point pair).
-__global__ void __launch_bounds__(R1_THREADS, 1)
+// WITH_C: the c statistic S too (128 more sums). Without it, S comes out of a
+// stripe fold (flock_launch_lc_fold) at eq(r[14..m)): the fold costs 0.27 ms at
+// 2^18 compressions where S costs this kernel 1.24 ms (3.96 -> 2.72: two of its three plane sets
+// and the registers that allow 16 warps), and about as much as S at 2^13.
+template <bool WITH_C>
+__global__ void __launch_bounds__(kR1Threads<WITH_C>, 1)
 zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B, const uint64_t* __restrict__ C,
                  size_t n_outer, const uint4* __restrict__ eq_basis, const ZcRound1Tables* __restrict__ T,
                  gf128* __restrict__ partials) {
+  constexpr int R1_THREADS = kR1Threads<WITH_C>, R1_WARPS = R1_THREADS / 32, kSets = WITH_C ? 3 : 1;
   extern __shared__ uint4 sm[];
   uint4* ext = sm;                                                   // [4][256][8]
   uint4* t8 = ext + 8 * 4 * 256;                                     // per warp T8[256]
@@ -272,7 +278,8 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
 #pragma unroll kZc1ParUnroll
       for (int par = 0; par < 2; par++) {
         const int xs = 4 * h + 2 * xs2 + par;
-        const uint64_t ra = A[row0 + 2 * xs2 + par], rb = B[row0 + 2 * xs2 + par], rc = C[row0 + 2 * xs2 + par];
+        const uint64_t ra = A[row0 + 2 * xs2 + par], rb = B[row0 + 2 * xs2 + par];
+        const uint64_t rc = WITH_C ? C[row0 + 2 * xs2 + par] : 0;
         uint64_t ea[8], eb[8];
 #pragma unroll
         for (int j = 0; j < 8; j++) { ea[j] = 0; eb[j] = 0; }
@@ -303,6 +310,7 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
           case 2: f8_mul_const_planes<f8_mul_c(f8_eq_factor(0, 0), f8_eq_factor(1, 1)), true>(y, w); break;
           default: f8_mul_const_planes<f8_mul_c(f8_eq_factor(0, 1), f8_eq_factor(1, 1)), true>(y, w); break;
         }
+        if constexpr (!WITH_C) continue;
         const uint8_t e8c = T->e8c[xs >> 1];
         // c goes to the parity-par half of t; with the parity a runtime value
         // (one loop body for both parities) the halves take rc or 0
@@ -326,8 +334,10 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
     // the two halves' row sums of producer group xm: add them
 #pragma unroll
     for (int j = 0; j < 8; j++) w[j] ^= shfl_xor64(w[j], 16);
+    if constexpr (WITH_C) {
 #pragma unroll
-    for (int j = 0; j < 16; j++) t[j] ^= shfl_xor64(t[j], 16);
+      for (int j = 0; j < 16; j++) t[j] ^= shfl_xor64(t[j], 16);
+    }
     // eq-weighted phi8 table of this block (see the layout above)
     {
       // lane l writes T8[l + 32 i], i < 8: the part of bits 0..4 (l) once,
@@ -357,7 +367,7 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
     // lanes of point quad xm read word xm of every producer row, half h
     // taking points 4 xm + 2 h, 4 xm + 2 h + 1.
 #pragma unroll 1
-    for (int set = 0; set < 3; set++) {
+    for (int set = 0; set < kSets; set++) {
       uint64_t pl[8];
 #pragma unroll
       for (int j = 0; j < 8; j++) pl[j] = set == 0 ? w[j] : set == 1 ? t[j] : t[8 + j];
@@ -398,15 +408,17 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
 #pragma unroll
     for (int q = 0; q < 2; q++) {
       o[q] = sum_ab[q];
-      o[64 + q] = sum_c[q];
-      o[128 + q] = sum_c[2 + q];
+      if constexpr (WITH_C) {
+        o[64 + q] = sum_c[q];
+        o[128 + q] = sum_c[2 + q];
+      }
     }
   }
   __syncthreads();
-  for (int col = threadIdx.x; col < 192; col += R1_THREADS) {
+  for (int col = threadIdx.x; col < 64 * kSets; col += R1_THREADS) {
     gf128 acc = gf_zero();
     for (int w2 = 0; w2 < R1_WARPS; w2++) acc = gf_add(acc, red[w2 * 192 + col]);
-    partials[(size_t)blockIdx.x * 192 + col] = acc;
+    partials[(size_t)blockIdx.x * (64 * kSets) + col] = acc;
   }
 }
 
@@ -867,17 +879,23 @@ __global__ void bind_pairs_kernel(const gf128* __restrict__ A, const gf128* __re
 
 }  // namespace
 
-int flock_launch_zc_round1(const void* a, const void* b, const void* c, size_t n_outer, const void* eq_basis,
-                           const ZcRound1Tables* d_tables, void* partials, int grid, cudaStream_t st) {
-  const size_t smem = R1_SMEM;
-  flock_once_per_device((const void*)zc_round1_kernel, [] {
-    cudaFuncSetAttribute(zc_round1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)R1_SMEM);
+template <bool WITH_C>
+static int launch_zc_round1(const void* a, const void* b, const void* c, size_t n_outer, const void* eq_basis,
+                            const ZcRound1Tables* d_tables, void* partials, int grid, cudaStream_t st) {
+  flock_once_per_device((const void*)zc_round1_kernel<WITH_C>, [] {
+    cudaFuncSetAttribute(zc_round1_kernel<WITH_C>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kR1Smem<WITH_C>);
   });
-  zc_round1_kernel<<<grid, R1_THREADS, smem, st>>>((const uint64_t*)a, (const uint64_t*)b, (const uint64_t*)c,
-                                                   n_outer, (const uint4*)eq_basis, d_tables, (gf128*)partials); flock_count_launch();
+  zc_round1_kernel<WITH_C><<<grid, kR1Threads<WITH_C>, kR1Smem<WITH_C>, st>>>(
+      (const uint64_t*)a, (const uint64_t*)b, (const uint64_t*)c, n_outer, (const uint4*)eq_basis, d_tables,
+      (gf128*)partials);
+  flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
-
+int flock_launch_zc_round1(const void* a, const void* b, const void* c, size_t n_outer, const void* eq_basis,
+                           const ZcRound1Tables* d_tables, void* partials, int grid, cudaStream_t st) {
+  return c ? launch_zc_round1<true>(a, b, c, n_outer, eq_basis, d_tables, partials, grid, st)
+           : launch_zc_round1<false>(a, b, c, n_outer, eq_basis, d_tables, partials, grid, st);
+}
 
 int flock_launch_zc1_eq_basis(const void* eq_out, size_t n_outer, const ZcRound1Tables* d_tables, void* out,
                               cudaStream_t st) {
