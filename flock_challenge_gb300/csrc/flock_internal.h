@@ -86,9 +86,11 @@ int flock_launch_combined_basis_msg(size_t n, const void* t0_lo, const void* t0_
 int flock_launch_combined_basis(size_t n, const void* t0_lo, const void* t0_hi, const void* t1_lo,
                                 const void* t1_hi, int lo_bits, const void* tables, void* b, cudaStream_t st);
 
-int flock_lig_grid(size_t n_pairs);
+int flock_lig_grid(size_t n_pairs);       // blocks of lig_intro_eq
+int flock_lig_fold_grid(size_t n_pairs);  // blocks of lig_fold_msg (n_pairs = n_out / 2)
+// fault: set to one if a wait inside the kernel gave up.
 int flock_launch_lig_fold_msg(const void* f, const void* b, size_t n_out, int fold, const uint64_t r[2], void* fo,
-                              void* bo, void* partials, int grid, cudaStream_t st);
+                              void* bo_out, void* partials, int grid, int* fault, cudaStream_t st);
 int flock_launch_lig_intro_eq(const void* f, size_t n, const void* lo, const void* hi, int lo_bits, void* partials,
                               int grid, cudaStream_t st);
 int flock_launch_glue_eq(void* b, size_t n, const void* lo, const void* hi, int lo_bits, const uint64_t beta[2],

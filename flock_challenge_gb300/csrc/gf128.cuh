@@ -34,6 +34,14 @@ __device__ __forceinline__ gf128 gf_load(const void* p) {
   gf128 r; r.w[0] = v.x; r.w[1] = v.y; r.w[2] = v.z; r.w[3] = v.w;
   return r;
 }
+// Two neighbouring elements, 32-byte aligned, in one 256-bit load (of memory the
+// kernel does not write).
+__device__ __forceinline__ void gf_load2(const gf128* p, gf128& a, gf128& b) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(a.w[0]), "=r"(a.w[1]), "=r"(a.w[2]), "=r"(a.w[3]), "=r"(b.w[0]), "=r"(b.w[1]), "=r"(b.w[2]),
+                 "=r"(b.w[3])
+               : "l"(p));
+}
 __device__ __forceinline__ void gf_store(void* p, gf128 a) {
   *reinterpret_cast<uint4*>(p) = make_uint4(a.w[0], a.w[1], a.w[2], a.w[3]);
 }

@@ -12,14 +12,12 @@
 //  * glue b += beta * basis, row and tree-node gathers for openings.
 #include "flock_internal.h"
 #include "gf128.cuh"
+#include "bit_outer.cuh"
 #include "gf_tab.cuh"
 
 namespace {
 
 constexpr int LG_THREADS = 256;
-#ifndef LG_MIN_BLOCKS
-#define LG_MIN_BLOCKS 2  // resident blocks per SM of the fold/message kernels
-#endif
 
 __device__ __forceinline__ void block_reduce_write(gf256 a, gf256 b, gf256 c, gf128* out) {
   __shared__ gf256 red[3][LG_THREADS / 32];
@@ -42,50 +40,141 @@ __device__ __forceinline__ void block_reduce_write(gf256 a, gf256 b, gf256 c, gf
   }
 }
 
-// If fold: in has 2 * n_out elements, bound at r into out (n_out elements);
-// message over the n_out-element state. Partials: (u0, u2, 0) per block.
-// use_tab: the fold multiplies through r's byte tables (gf_tab.cuh, dynamic
-// shared memory), worth their build when a CTA folds hundreds of pairs.
-__global__ void __launch_bounds__(LG_THREADS, LG_MIN_BLOCKS)
-lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, size_t n_out, int fold,
-                    const __grid_constant__ gf128p r, const gf128 r_plain, int use_tab,
-                    gf128* __restrict__ fo, gf128* __restrict__ bo, gf128* __restrict__ partials) {
-  extern __shared__ uint4 rtab[];
-  const uint32_t rot = threadIdx.x & 15;
-  if (use_tab) gf_tab_build(r_plain, rtab);
-  gf256 u0 = {{0, 0, 0, 0}}, u2 = u0, zz = u0;
-  size_t pairs = n_out / 2;
-  for (size_t j = (size_t)blockIdx.x * LG_THREADS + threadIdx.x; j < pairs; j += (size_t)gridDim.x * LG_THREADS) {
-    gf128 f0, f1, b0, b1;
-    if (fold) {
-      gf128 x0 = f[4 * j], x1 = f[4 * j + 1], x2 = f[4 * j + 2], x3 = f[4 * j + 3];
-      gf128 y0 = b[4 * j], y1 = b[4 * j + 1], y2 = b[4 * j + 2], y3 = b[4 * j + 3];
-      if (use_tab) {
-        f0 = gf_add(x0, gf_mul_tab(rtab, gf_add(x0, x1), rot));
-        f1 = gf_add(x2, gf_mul_tab(rtab, gf_add(x2, x3), rot));
-        b0 = gf_add(y0, gf_mul_tab(rtab, gf_add(y0, y1), rot));
-        b1 = gf_add(y2, gf_mul_tab(rtab, gf_add(y2, y3), rot));
-      } else {
-        f0 = gf_add(x0, gf_mul_p(gf_add(x0, x1), r));
-        f1 = gf_add(x2, gf_mul_p(gf_add(x2, x3), r));
-        b0 = gf_add(y0, gf_mul_p(gf_add(y0, y1), r));
-        b1 = gf_add(y2, gf_mul_p(gf_add(y2, y3), r));
-      }
-      fo[2 * j] = f0; fo[2 * j + 1] = f1;
-      bo[2 * j] = b0; bo[2 * j + 1] = b1;
-    } else {
-      f0 = f[2 * j]; f1 = f[2 * j + 1]; b0 = b[2 * j]; b1 = b[2 * j + 1];
-    }
-    gf256_acc(u0, gf_mul_wide(f0, b0));
-    gf256_acc(u2, gf_mul_wide(gf_add(f0, f1), gf_add(b0, b1)));
+// FOLD: in has 2 * n_out elements, bound at r into out (n_out elements); the
+// message u0 = sum f0 b0, u2 = sum (f0 + f1)(b0 + b1) over the n_out-element
+// state's pairs. Partials: (u0, u2, 0) per block. n_out / 2 a multiple of
+// bo::TILE.
+//
+// The two sums run on the tensor cores (bit_outer.cuh): warps 0..7 take tiles of
+// 128 pairs of f, warps 8..15 the same tiles of b (bind through r's byte tables,
+// gf_tab.cuh, write, and expand the values' bits into the tile's slot), and
+// one thread of a further warp issues the MMAs in tile order. Four slots are
+// shared by the eight tiles in work. Bound by the shared-memory data path: 1 KB
+// of table lookups and 512 bytes of operands, written and read, per pair. With both
+// products as carry-less ones in the folding threads 580 us for 2^23 pairs (ALU
+// 58%, issue 47%), so 391 us (the data path 76% busy); without a fold 19 us and
+// 14 us for 2^18 pairs, 357 us for 2^24 (0.44 of the measured HBM rate: a tile's
+// MMAs and their commit, about 500 clocks, bound it). (One lane a pair, its four
+// values 64 bytes apart from the next lane's: 552 us, the uncoalesced loads taking
+// a third of the data path; loads without the four steps ahead: 451 us.)
+constexpr int LM_PRODUCERS = 512, LM_THREADS = LM_PRODUCERS + 32;
+template <bool FOLD>
+constexpr int kLmSlots = FOLD ? 4 : 6;
+template <bool FOLD>
+constexpr size_t kLmSmem = (FOLD ? (size_t)GF_TAB_ENTRIES * 16 : 0) + (size_t)kLmSlots<FOLD> * bo::SLOT;
+static_assert(kLmSmem<true> <= 232448 && kLmSmem<false> <= 232448, "fold shared memory above the 227 KB per-block limit");
+
+template <bool FOLD>
+__global__ void __launch_bounds__(LM_THREADS, 1)
+lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, size_t n_tiles, const gf128 r,
+                    gf128* __restrict__ fo, gf128* __restrict__ bo_out, gf128* __restrict__ partials,
+                    volatile int* fault) {
+  constexpr int LM_SLOTS = kLmSlots<FOLD>, LM_AHEAD = FOLD ? 4 : 8;
+  extern __shared__ __align__(128) uint8_t lm_smem[];
+  // done[tau mod 8]: the MMAs of tile tau of the CTA's sequence. A tile's warps
+  // come back to the same one of them every eight tiles, so nobody skips a phase
+  // (a wait tells a phase from its neighbours only).
+  __shared__ uint64_t full[LM_SLOTS], done[8], all_done;
+  __shared__ uint32_t tmem_slot, poly[2][4][5];
+  uint8_t* slots = lm_smem;
+  uint4* rtab = reinterpret_cast<uint4*>(lm_smem + (size_t)kLmSlots<FOLD> * bo::SLOT);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const size_t t0 = n_tiles * blockIdx.x / gridDim.x, t1 = n_tiles * (blockIdx.x + 1) / gridDim.x;
+  const int n = (int)(t1 - t0);  // at least one: gridDim.x <= n_tiles
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
+  if (t == 0) {
+    for (int k = 0; k < LM_SLOTS; k++) tc::mbar_init(&full[k], 2);
+    for (int k = 0; k < 8; k++) tc::mbar_init(&done[k], 1);
+    tc::mbar_init(&all_done, 1);
+    tc::mbar_fence_init();
   }
-  block_reduce_write(u0, u2, zz, partials);
+  if constexpr (FOLD) {
+    for (int it = t; it < 256; it += LM_THREADS) gf_tab_row_direct(r, rtab, it);
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  // columns 0..127, 128..255: the two sums' counts; 256..287: the scales, all one
+  const uint32_t tmem = tmem_slot, sf = tmem + 256;
+  if (warp < 4) tc::tmem_fill32(sf + ((uint32_t)(32 * warp) << 16), 0x7f7f7f7fu);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  bool ok = true;
+  if (t < LM_PRODUCERS) {
+    const bool is_b = warp >= 8;
+    const gf128* in = is_b ? b : f;
+    gf128* out = is_b ? bo_out : fo;
+    const uint32_t rot = t & 15;
+    // the loads run LM_AHEAD steps ahead, into the next tile
+    gf128 y0[LM_AHEAD], y1[LM_AHEAD];
+    auto load = [&](int tau, int k) {
+      const size_t i = (t0 + tau) * (2 * bo::TILE) + lane + 32 * k;
+      if constexpr (FOLD) gf_load2(&in[2 * i], y0[k % LM_AHEAD], y1[k % LM_AHEAD]);
+      else y0[k % LM_AHEAD] = gf_load(&in[i]);
+    };
+    if ((warp & 7) < n) {
+#pragma unroll
+      for (int k = 0; k < LM_AHEAD; k++) load(warp & 7, k);
+    }
+    for (int tau = warp & 7; tau < n && ok; tau += 8) {
+      // value i & 1 of pair i / 2: i = 2 pair + (lane & 1), 32 consecutive i per k
+      const size_t i0 = (t0 + tau) * (2 * bo::TILE) + lane;
+      gf128 v[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const size_t i = i0 + 32 * k;
+        if constexpr (FOLD) {
+          v[k] = gf_add(y0[k % LM_AHEAD], gf_mul_tab(rtab, gf_add(y0[k % LM_AHEAD], y1[k % LM_AHEAD]), rot));
+          gf_store(&out[i], v[k]);
+        } else {
+          v[k] = y0[k % LM_AHEAD];
+        }
+        if (k + LM_AHEAD < 8) load(tau, k + LM_AHEAD);
+        else if (tau + 8 < n) load(tau + 8, k + LM_AHEAD - 8);
+      }
+      // the odd lane takes the sum
+#pragma unroll
+      for (int k = 0; k < 8; k++) {
+        const gf128 o = gf_shfl_xor(v[k], 1);
+        if (lane & 1) v[k] = gf_add(v[k], o);
+      }
+      const int slot = tau % LM_SLOTS;
+      if (tau >= LM_SLOTS)
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(tau - LM_SLOTS) % 8], ((tau - LM_SLOTS) / 8) & 1));
+      if (ok) bo::put_tile(v, slots + slot * bo::SLOT + (is_b ? bo::SIDE : 0), lane & 1);
+      tc::fence_smem_for_mma();
+      __syncwarp();
+      if (lane == 0) tc::mbar_arrive(&full[slot]);
+    }
+  } else if (lane == 0) {
+    for (int tau = 0; tau < n && ok; tau++) {
+      const int slot = tau % LM_SLOTS;
+      ok = tc::mbar_wait(&full[slot], (tau / LM_SLOTS) & 1);
+      if (!ok) break;
+      tc::fence_after();
+      bo::mma_slot(tc::smem_addr(slots + slot * bo::SLOT), tmem, sf, tau == 0);
+      tc::mma_commit(&done[tau % 8]);
+    }
+    tc::mma_commit(&all_done);
+  }
+  __syncwarp();  // the issuing warp's other lanes stay out of its way: a lane's wait holds up the whole warp
+  ok = tc::mbar_wait(&all_done, 0) && ok;
+  if (!ok) *fault = 1;
+  __syncwarp();
+  tc::fence_after();
+  if (warp < 8) bo::read_quadrant(tmem + 128 * (warp >> 2), poly[warp >> 2][warp & 3]);
+  tc::fence_before();
+  __syncthreads();
+  if (t < 2) partials[3 * blockIdx.x + t] = bo::combine(poly[t]);
+  if (t == 2) partials[3 * blockIdx.x + 2] = gf_zero();
+  if (warp == 0) tc::tmem_free(tmem, 512);
 }
 
 // The same for small states (at most LG_SMALL_PAIRS pairs), bound by a
-// thread's chain: two lanes a pair (gf_round_small). One pair:
-// lig_fold_msg_kernel 9.3 us, this 5.2 us; 2^17 pairs: 25.6 us and 23.6 us
-// (beyond, the table products win).
+// thread's chain: two lanes a pair (gf_round_small). One pair: 5.2 us (one
+// thread a pair, its products unrolled: 9.3 us); 2^17 pairs: 23.4 us, beyond
+// which lig_fold_msg_kernel wins (2^18 pairs: 21.8 us).
 constexpr size_t LG_SMALL_PAIRS = (size_t)1 << 17;
 constexpr int LGS_MAX_THREADS = 256;
 __global__ void __launch_bounds__(LGS_MAX_THREADS)
@@ -361,24 +450,31 @@ inline unsigned grid_for(size_t work, size_t threads, size_t cap) {
 int flock_lig_grid(size_t n_pairs) {
   return n_pairs <= LG_SMALL_PAIRS ? gf_small_grid(n_pairs) : (int)grid_for(n_pairs, LG_THREADS, 152 * 4);
 }
+int flock_lig_fold_grid(size_t n_pairs) {
+  return n_pairs <= LG_SMALL_PAIRS ? gf_small_grid(n_pairs) : (int)grid_for(n_pairs, bo::TILE, 152);
+}
 
 int flock_launch_lig_fold_msg(const void* f, const void* b, size_t n_out, int fold, const uint64_t r[2], void* fo,
-                              void* bo, void* partials, int grid, cudaStream_t st) {
+                              void* bo_out, void* partials, int grid, int* fault, cudaStream_t st) {
   if (n_out / 2 <= LG_SMALL_PAIRS) {
     if (grid != gf_small_grid(n_out / 2)) return FLOCK_ERR_SHAPE;
     lig_fold_msg_small_kernel<<<grid, gf_small_threads(n_out / 2), 0, st>>>(
-        (const gf128*)f, (const gf128*)b, n_out / 2, fold, to_gf(r), (gf128*)fo, (gf128*)bo, (gf128*)partials);
+        (const gf128*)f, (const gf128*)b, n_out / 2, fold, to_gf(r), (gf128*)fo, (gf128*)bo_out, (gf128*)partials);
     flock_count_launch();
     return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
   }
-  constexpr size_t kTabSmem = (size_t)GF_TAB_ENTRIES * 16;
-  flock_once_per_device((const void*)lig_fold_msg_kernel, [] {
-    cudaFuncSetAttribute(lig_fold_msg_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTabSmem);
+  const size_t n_tiles = n_out / 2 / bo::TILE;
+  if ((n_out / 2) % bo::TILE || grid < 1 || (size_t)grid > n_tiles) return FLOCK_ERR_SHAPE;
+  flock_once_per_device((const void*)lig_fold_msg_kernel<true>, [] {
+    cudaFuncSetAttribute(lig_fold_msg_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLmSmem<true>);
+    cudaFuncSetAttribute(lig_fold_msg_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLmSmem<false>);
   });
-  const int use_tab = fold && (n_out / 2) / (size_t)grid >= 512;
-  lig_fold_msg_kernel<<<grid, LG_THREADS, use_tab ? kTabSmem : 0, st>>>(
-      (const gf128*)f, (const gf128*)b, n_out, fold, gf_prepare(to_gf(r)), to_gf(r), use_tab, (gf128*)fo, (gf128*)bo,
-      (gf128*)partials);
+  if (fold)
+    lig_fold_msg_kernel<true><<<grid, LM_THREADS, kLmSmem<true>, st>>>(
+        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), (gf128*)fo, (gf128*)bo_out, (gf128*)partials, fault);
+  else
+    lig_fold_msg_kernel<false><<<grid, LM_THREADS, kLmSmem<false>, st>>>(
+        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), nullptr, nullptr, (gf128*)partials, fault);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }

@@ -160,6 +160,7 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
       }
     }
   }
+  __syncwarp();  // the issuing warp's other lanes stay out of its way: a lane's wait holds up the whole warp
   // every MMA is done when the last stage's commit has arrived
   ok = tc::mbar_wait(&done[(n - 1) % FM_BUFS], ((n - 1) / FM_BUFS) & 1) && ok;
   if (!ok) *fault = 1;

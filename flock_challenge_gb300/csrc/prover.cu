@@ -344,6 +344,9 @@ constexpr size_t kHostTailPairs = 512;
 // fold instead of zerocheck round 1 (2^14: round 1 0.26 ms with it; 0.19 ms
 // without, and the fold 0.05 ms).
 constexpr int kFoldCLog = 14;
+// Proofs of at least 2^kSplitMsgLog compressions compute the combined basis and
+// the first Ligerito message in two launches, the message on the tensor cores.
+constexpr int kSplitMsgLog = 13;
 // Lincheck product-sumcheck rounds over at most this many entries run on the host.
 constexpr size_t kHostTailLincheck = 1024;
 
@@ -1232,7 +1235,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       for (int k = 0; k < 2; k++) hf::scale(eqr[k].data(), gam[k], 128, &wk[k * 128]);
       void* dt = S->tables.get(wk.size() * 16);
       h2d(*S, dt, wk.data(), wk.size() * 16);
-      if (chain) {
+      if (chain || n_log >= kSplitMsgLog) {
         FK(flock_launch_combined_basis(n128, S->tlo0.p, S->thi0.p, S->tlo1.p, S->thi1.p, rs_lo, dt, dbc, st));
       } else {
         // the first Ligerito message over (z, b) comes out of the same pass;
@@ -1291,17 +1294,17 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     size_t len = n128;
     auto run_msg = [&](int fold, F rr) {
       size_t n_out = fold ? len / 2 : len;
-      int grid = flock_lig_grid(n_out / 2);
+      int grid = flock_lig_fold_grid(n_out / 2);
       void* dpart = part_buf(*S, (size_t)grid * 3 * 16);
       uint64_t rp[2];
       u2(rr, rp);
       if (fold) {
-        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 1, rp, falt, balt, dpart, grid, st));
+        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 1, rp, falt, balt, dpart, grid, S->fault(), st));
         std::swap(fcur, falt);
         std::swap(bcur, balt);
         len = n_out;
       } else {
-        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 0, rp, nullptr, nullptr, dpart, grid, st));
+        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 0, rp, nullptr, nullptr, dpart, grid, S->fault(), st));
       }
       auto s = reduce_partials(*S, dpart, grid, 3);
       msgs.push_back({s[0], s[1]});
@@ -1309,10 +1312,10 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       tr.observe(s[1]);
     };
     auto introduce = [&](const void* dbasis) {
-      int grid = flock_lig_grid(len / 2);
+      int grid = flock_lig_fold_grid(len / 2);
       void* dpart = part_buf(*S, (size_t)grid * 3 * 16);
       uint64_t rp[2] = {0, 0};
-      FK(flock_launch_lig_fold_msg(fcur, dbasis, len, 0, rp, nullptr, nullptr, dpart, grid, st));
+      FK(flock_launch_lig_fold_msg(fcur, dbasis, len, 0, rp, nullptr, nullptr, dpart, grid, S->fault(), st));
       auto s = reduce_partials(*S, dpart, grid, 3);
       msgs.push_back({s[0], s[1]});
       tr.observe(s[0]);
@@ -1448,6 +1451,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     // one wait for the openings' queued copies (the final opening's gathers
     // are the last work of the phase)
     CK(flock_stream_wait(st, &S->waits));
+    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "Ligerito fold");
     finish_open(*S, open0);
     for (Open& o : rec_opens) finish_open(*S, o);
     finish_open(*S, final_open);

@@ -29,16 +29,11 @@ __device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
 }
-__device__ __forceinline__ uint64_t now_ns() {
-  uint64_t t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
-// Waits for the completion of phase `parity`; false when it gave up after a
-// second (no wait of a healthy kernel comes near it).
+// Waits for the completion of phase `parity`; false when it gave up after 2^31
+// clocks, a second (no wait of a healthy kernel comes near it).
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
   const uint32_t a = smem_addr(b);
-  uint64_t t0 = 0;
+  long long t0 = 0;
   for (;;) {
     uint32_t ok;
     asm volatile(
@@ -49,9 +44,9 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
         : "r"(a), "r"(parity)
         : "memory");
     if (ok) return true;
-    const uint64_t t = now_ns();
+    const long long t = clock64();
     if (t0 == 0) t0 = t;
-    else if (t - t0 > 1000000000ull) return false;
+    else if (t - t0 > (1ll << 31)) return false;
   }
 }
 // Contiguous copy into shared memory by the copy engine (16-byte aligned both
