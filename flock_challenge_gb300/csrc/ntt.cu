@@ -19,6 +19,7 @@
 // first pass of a rate-1/2^r code reads the message directly, position p
 // taking row p mod 2^(log_d - r), which is the replicated state after the r
 // copy layers (pcs/commit.rs:451-473).
+#include <algorithm>
 #include <cstdio>
 #include <cuda.h>
 
@@ -535,6 +536,117 @@ int launch_tab2(gf128* dst, const gf128* src, size_t mask, const gf128* tw, int 
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
+// ---- stage passes (8-lane codes) -------------------------------------------
+//
+// The level codes of the recursive opening have 8 lanes and 2^8..2^21 positions:
+// too few products per twiddle for byte tables to pay early on, and too few
+// elements for the multiply passes' eight positions a thread to fill the GPU
+// (2^16 positions: 13 warps per SM, the six-layer pass at 35% of the issue
+// slots, an eighth of them waiting for instructions). A stage pass gives a
+// thread four positions of one lane and applies two layers per stage to them,
+// up to SP_MAX_LAYERS layers on a tile of 2^F positions with one exchange
+// through shared memory between stages. Plain twiddles (16 bytes, masked in
+// registers; the two products of a stage's upper layer share one), one loop
+// body of two products for every layer of a width class. Bound by the
+// carry-less products (ALU and multiplier pipes). 2^12 positions from layer 3:
+// 25.5 us with table and multiply passes, 18.9 us so; 2^8: 18.8 us and 10.2 us.
+// At 2^16 positions stage passes of all layers lose (106 us: byte tables do the
+// upper layers at twice the rate), but take the last layers (87.5 -> 82.5 us).
+constexpr int kStageVariant = 4;
+constexpr int SP_MIN_BLOCKS = 3;  // 80 registers; 2 and 4 measured the same within 3%
+constexpr int SP_LANES = 8, SP_MAX_LAYERS = 7, SP_MAX_THREADS = (1 << (SP_MAX_LAYERS - 2)) * SP_LANES;
+
+// The four masked parts of a twiddle's word.
+__device__ __forceinline__ uint4 sp_masks(uint32_t w) {
+  return make_uint4(w & 0x11111111u, w & 0x22222222u, w & 0x44444444u, w & 0x88888888u);
+}
+
+__global__ void __launch_bounds__(SP_MAX_THREADS, SP_MIN_BLOCKS)
+ntt_stage_kernel(gf128* __restrict__ dst, const gf128* __restrict__ src, size_t src_pos_mask,
+                 const gf128* __restrict__ tw, int log_d, int l0, int F, int narrow) {
+  extern __shared__ gf128 sp_tile[];  // [2^F positions][SP_LANES]
+  const int lane = threadIdx.x % SP_LANES, pt = threadIdx.x / SP_LANES;
+  const int lo_bits = log_d - l0 - F;
+  const size_t lo = blockIdx.x & (((size_t)1 << lo_bits) - 1), hi = blockIdx.x >> lo_bits;
+  auto gpos = [&](int i) { return (hi << (log_d - l0)) | ((size_t)i << lo_bits) | lo; };
+  // stage of tile bits (hb, hb - 1): positions i = (upper of pt), j, (lower of
+  // pt). With F odd the last stage takes bit 0 only (bit 1 is done).
+  for (int hb = F - 1; hb >= 0; hb -= 2) {
+    const bool half = hb == 0;
+    const int b1 = half ? 1 : hb, up = pt >> (b1 - 1);
+    const int base = (up << (b1 + 1)) | (pt & ((1 << (b1 - 1)) - 1));
+    gf128 y[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = base | (j << (b1 - 1));
+      y[j] = hb == F - 1 ? gf_load(&src[(gpos(i) & src_pos_mask) * SP_LANES + lane]) : sp_tile[i * SP_LANES + lane];
+    }
+    // layer of bit b1: pairs (0, 2), (1, 3); of bit b1 - 1: (0, 1), (2, 3)
+    gf128 u0 = y[0], v0 = y[2], u1 = y[1], v1 = y[3];
+    if (half) {
+      v0 = y[1];
+      u1 = y[2];
+    }
+#pragma unroll 1
+    for (int k = half ? 1 : 0; k < 2; k++) {
+      const int t = F - 1 - b1 + k, layer = l0 + t;
+      const gf128* twl = tw + ((((size_t)1) << layer) - 1 + (hi << t));
+      const gf128 t0 = gf_load(&twl[k ? 2 * up : up]), t1 = k ? gf_load(&twl[2 * up + 1]) : t0;
+      gf128 p0, p1;
+      if (layer >= (narrow & 255)) {
+        p0 = gf_mul_p32(v0, sp_masks(t0.w[0]));
+        p1 = gf_mul_p32(v1, sp_masks(t1.w[0]));
+      } else if (layer >= ((narrow >> 16) & 255)) {
+        p0 = gf_mul_p64(v0, sp_masks(t0.w[0]), sp_masks(t0.w[1]), sp_masks(t0.w[0] ^ t0.w[1]));
+        p1 = gf_mul_p64(v1, sp_masks(t1.w[0]), sp_masks(t1.w[1]), sp_masks(t1.w[0] ^ t1.w[1]));
+      } else {
+        p0 = gf_mul(v0, t0);
+        p1 = gf_mul(v1, t1);
+      }
+      u0 = gf_add(u0, p0);
+      v0 = gf_add(v0, u0);
+      u1 = gf_add(u1, p1);
+      v1 = gf_add(v1, u1);
+      if (k == 0) {  // to the lower layer's pairs
+        const gf128 x = v0;
+        v0 = u1;
+        u1 = x;
+      }
+    }
+    y[0] = u0; y[1] = v0; y[2] = u1; y[3] = v1;
+    const bool last = hb <= 1;
+    if (!last && hb != F - 1) __syncthreads();  // the tile's reads are done
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+      const int i = base | (j << (b1 - 1));
+      if (last) gf_store(&dst[gpos(i) * SP_LANES + lane], y[j]);
+      else sp_tile[i * SP_LANES + lane] = y[j];
+    }
+    if (!last) __syncthreads();
+  }
+}
+
+// Layers [from, log_d) in stage passes of 2..SP_MAX_LAYERS layers, split evenly;
+// 8-lane codes with at least two layers left.
+bool stage_applies(int log_d, int log_lanes, int from) { return (1 << log_lanes) == SP_LANES && log_d - from >= 2; }
+int run_stage_passes(gf128* dst, const gf128* src, size_t mask, const gf128* twp, int log_d, int from,
+                     cudaStream_t st) {
+  const int narrow = flock_ntt_narrow_layers(log_d);
+  const int remaining = log_d - from, passes = (remaining + SP_MAX_LAYERS - 1) / SP_MAX_LAYERS;
+  int l = from;
+  for (int q = 0; q < passes; q++) {
+    const int f = (remaining - (l - from) + (passes - q) - 1) / (passes - q);
+    ntt_stage_kernel<<<(unsigned)((size_t)1 << (log_d - f)), (1 << (f - 2)) * SP_LANES,
+                       ((size_t)16 * SP_LANES) << f, st>>>(dst, src, mask, twp, log_d, l, f, narrow);
+    flock_count_launch();
+    if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
+    src = dst;
+    mask = ~(size_t)0;
+    l += f;
+  }
+  return FLOCK_OK;
+}
+
 // ---- deep-table pass ------------------------------------------------------
 //
 // The twiddles of the last three layers are narrow (layer d-1 below 2^d,
@@ -759,12 +871,13 @@ const void* flock_ntt_twiddles_prepared(int log_d) {
 // and two timed runs per candidate): the table passes for each table depth of
 // kTabMinLogs, and the multiply passes of every pass shape from each depth's
 // end layer, plus the deep-table pass where a depth leaves exactly the last
-// three layers of a 64-lane code; it keeps the pair with the smallest sum for
-// later calls. All candidates compute identical results; only speed differs.
-// FLOCK_NTT_TUNE=0 in the environment turns tuning off (the default depth and
-// shape everywhere); FLOCK_NTT_VARIANT=0|1|2|3 fixes the multiply-pass shape
-// (with the default depth; 3 falls back to shape 1 where the deep-table pass
-// does not apply).
+// three layers of a 64-lane code and, for 8-lane codes, the stage passes from
+// every depth's end (up to 2^15 positions from every smaller one); it keeps the
+// pair with the smallest sum for later calls. All candidates compute identical results; only
+// speed differs. FLOCK_NTT_TUNE=0 in the environment turns tuning off (the
+// default depth and shape everywhere); FLOCK_NTT_VARIANT=0..4 fixes the
+// multiply-pass shape (with the default depth; 4: stage passes of all layers; 3
+// and 4 fall back to shape 1 where they do not apply).
 namespace {
 
 struct TuneKey {
@@ -821,8 +934,14 @@ TunedShape tune_shape(const TuneKey& k, const void* tw, const gf128* twp, cudaSt
   std::map<int, float> tab_ms;                    // per table end layer
   std::map<std::pair<int, int>, float> mult_ms;  // per (table end layer, shape)
   float best_ms = 1e30f;
-  for (int ml : kTabMinLogs) {
-    const int te = tab_layers_end(k.log_d, k.log_lanes, k.start, ml);
+  // table depths; for the small codes that stage passes may take further, fewer
+  // table passes too
+  std::vector<int> ends;
+  for (int ml : kTabMinLogs) ends.push_back(tab_layers_end(k.log_d, k.log_lanes, k.start, ml));
+  if (k.log_d <= 15 && stage_applies(k.log_d, k.log_lanes, k.start))
+    for (int te = k.start; te < ends[0]; te += 2)
+      if (std::find(ends.begin(), ends.end(), te) == ends.end()) ends.push_back(te);
+  for (int te : ends) {
     if (te > k.start && !twp) continue;
     if (!tab_ms.count(te))
       tab_ms[te] = te == k.start ? 0.f
@@ -837,6 +956,17 @@ TunedShape tune_shape(const TuneKey& k, const void* tw, const gf128* twp, cudaSt
       if (t < best_ms) {
         best_ms = t;
         best = TunedShape{te, v};
+      }
+    }
+    // stage passes behind the table passes
+    if (twp && stage_applies(k.log_d, k.log_lanes, te)) {
+      const auto key = std::make_pair(te, kStageVariant);
+      if (!mult_ms.count(key))
+        mult_ms[key] = time_of([&] { return run_stage_passes(d, d, ~(size_t)0, twp, k.log_d, te, st); });
+      const float t = tab_ms[te] + mult_ms[key];
+      if (t < best_ms) {
+        best_ms = t;
+        best = TunedShape{te, kStageVariant};
       }
     }
     // the deep-table pass, where the multiply part is exactly the last three layers
@@ -863,6 +993,7 @@ TunedShape pick_shape(int log_d, int log_lanes, int start, const void* tw, const
   if (const char* f = std::getenv("FLOCK_NTT_VARIANT")) {  // a fixed shape, for measurements
     const int v = f[0] - '0';
     if ((v >= 0 && v < kVariants) || v == kDeepVariant) return TunedShape{dflt.tab_end, v};
+    if (v == kStageVariant) return TunedShape{stage_applies(log_d, log_lanes, start) ? start : dflt.tab_end, v};
   }
   if (!tuning_enabled()) return dflt;
   TuneKey k{0, log_d, log_lanes, start};
@@ -937,6 +1068,10 @@ int flock_launch_ntt(void* d_data, const void* d_src, int log_d, int log_lanes, 
     }
   }
   if (l == log_d) return FLOCK_OK;
+  if (sh.variant == kStageVariant) {
+    if (stage_applies(log_d, log_lanes, l)) return run_stage_passes(data, src, mask, twp, log_d, l, stream);
+    return run_passes<true>(kDefaultVariant, data, src, mask, tw, log_d, log_lanes, l, stream);
+  }
   if (sh.variant == kDeepVariant) {
     if (src == data && deep3_applies(log_d, log_lanes, l)) return run_deep3(data, twp, tw, log_d, stream);
     return run_passes<true>(kDefaultVariant, data, src, mask, tw, log_d, log_lanes, l, stream);
