@@ -488,6 +488,45 @@ ntt_tab2_kernel(gf128* __restrict__ dst, const gf128* __restrict__ src, size_t s
   }
 }
 
+// Layer l alone, where the layers before the deep-table pass are odd in number:
+// one table, so two blocks share an SM, and a thread's items are pairs of
+// positions. Bound by the codeword's traffic (a layer per read and write) where
+// it exceeds L2.
+constexpr size_t TAB1_SMEM = (size_t)TAB_ENTRIES * 16;
+__global__ void __launch_bounds__(TAB_THREADS, 2)
+ntt_tab1_kernel(gf128* dst, const gf128* src, size_t src_pos_mask, const gf128* __restrict__ tw, int log_d,
+                int log_lanes, int l, int cph) {
+  extern __shared__ uint4 tabs[];
+  const size_t hi = blockIdx.x / cph;
+  const int part = blockIdx.x % cph;
+  gf_tab_build(gf_load(&tw[((size_t)1 << l) - 1 + hi]), tabs);
+  const int lo_bits = log_d - l - 1;
+  const size_t nl = (size_t)1 << log_lanes, items = nl << lo_bits;
+  const uint32_t rot = threadIdx.x & 15;
+  for (size_t it = (size_t)part * TAB_THREADS + threadIdx.x; it < items; it += (size_t)cph * TAB_THREADS) {
+    const size_t lane = it & (nl - 1), p0 = (hi << (lo_bits + 1)) | (it >> log_lanes), p1 = p0 | ((size_t)1 << lo_bits);
+    gf128 u = gf_load(&src[(p0 & src_pos_mask) * nl + lane]);
+    const gf128 v = gf_load(&src[(p1 & src_pos_mask) * nl + lane]);
+    u = gf_add(u, gf_mul_tab(tabs, v, rot));
+    gf_store(&dst[p0 * nl + lane], u);
+    gf_store(&dst[p1 * nl + lane], gf_add(v, u));
+  }
+}
+
+int launch_tab1(gf128* dst, const gf128* src, size_t mask, const gf128* tw, int log_d, int log_lanes, int l,
+                cudaStream_t st) {
+  flock_once_per_device((const void*)ntt_tab1_kernel, [] {
+    cudaFuncSetAttribute(ntt_tab1_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAB1_SMEM);
+  });
+  const size_t n_hi = (size_t)1 << l, items = ((size_t)1 << (log_d - l - 1)) << log_lanes;
+  size_t cph = 1;  // about two waves of two blocks per SM, at least two items a thread
+  while (n_hi * cph < 608 && items / (2 * cph) >= 2 * (size_t)TAB_THREADS) cph *= 2;
+  ntt_tab1_kernel<<<(unsigned)(n_hi * cph), TAB_THREADS, TAB1_SMEM, st>>>(dst, src, mask, tw, log_d, log_lanes, l,
+                                                                          (int)cph);
+  flock_count_launch();
+  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+}
+
 // Layers [start, end) handled by table passes: pairs of layers while a block
 // of the pass's first layer l holds at least 2^min_log quad-lanes (its three
 // tables are then built for at least 4 x 2^min_log products; deeper blocks are
@@ -663,9 +702,14 @@ int run_stage_passes(gf128* dst, const gf128* src, size_t mask, const gf128* twp
 // three layers measured 6.29 ms for the 2^20-position L0 set, this split
 // 6.07, the multiply passes 6.65: the random lookups conflict on ~60% of
 // shared wavefronts, so the load/store data path binds the all-table form).
-// Used for the last three layers of a 64-lane code whose twiddles there fit
-// 88, 56 and 24 bits, when the autotuner measures it faster than the
-// multiply passes.
+// A code of more than 64 lanes has its block walk the groups of 64 lanes, one
+// table build for all of them (a kernel of its own: the loop costs the 64-lane
+// form 1%). Used for the last three layers of a code of 64 lanes or more whose
+// twiddles there fit 88, 56 and 24 bits, when the autotuner measures it faster
+// than the multiply passes. Where pairs of table layers would end a layer off, a
+// one-layer table pass goes first. 2^17 positions x 256 lanes from layer 2: 2,370 us
+// with the three layers in a multiply pass, 2,216 us so; 2^15 x 64 from layer 1:
+// 209.9 us with four layers in a multiply pass, 200.5 us so.
 constexpr int kDeepVariant = 3;
 constexpr int D3_LANES = 64;
 constexpr int D3_C_STRIDE = 256 + 16;  // words per layer d-1 table: the skew keeps the build's stores conflict-free
@@ -678,7 +722,7 @@ struct Deep3Tabs {
 // The deep-table pass applies to the layers [from, log_d) of a code of
 // 2^log_lanes lanes.
 bool deep3_applies(int log_d, int log_lanes, int from) {
-  return log_d >= 4 && log_d <= 30 && from == log_d - 3 && (1 << log_lanes) == D3_LANES &&
+  return log_d >= 4 && log_d <= 30 && from == log_d - 3 && (1 << log_lanes) >= D3_LANES &&
          twiddle_layer_width(log_d, log_d - 1) <= 24 && twiddle_layer_width(log_d, log_d - 2) <= 56 &&
          twiddle_layer_width(log_d, log_d - 3) <= 88;
 }
@@ -726,8 +770,10 @@ __device__ __forceinline__ gf128 d3_mul(const E* __restrict__ T, const gf128& y)
 // Layers log_d-3 .. log_d-1 in place for position group blockIdx.x
 // (positions 8 q .. 8 q + 7), thread = lane. tw: the plain twiddle table;
 // twq: the prepared one (layer d-2's products).
+template <bool ONE>
 __global__ void __launch_bounds__(D3_LANES, 8) ntt_deep3_kernel(gf128* __restrict__ data, const gf128* __restrict__ tw,
-                                                             const gf128p* __restrict__ twq, int log_d) {
+                                                             const gf128p* __restrict__ twq, int log_d,
+                                                             int lanes) {
   __shared__ Deep3Tabs T;
   const size_t q = blockIdx.x;
   const int lane = threadIdx.x;
@@ -773,42 +819,49 @@ __global__ void __launch_bounds__(D3_LANES, 8) ntt_deep3_kernel(gf128* __restric
     }
   }
   __syncthreads();
-  gf128 y[8];
+#pragma unroll 1
+  for (int lane0 = lane; lane0 < (ONE ? D3_LANES : lanes); lane0 += D3_LANES) {
+    gf128 y[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) y[j] = gf_load(&data[((q << 3) | (size_t)j) * D3_LANES + lane]);
-  // layer d-3: pairs (j, j + 4), one twiddle
+    for (int j = 0; j < 8; j++) y[j] = gf_load(&data[((q << 3) | (size_t)j) * (ONE ? D3_LANES : lanes) + lane0]);
+    // layer d-3: pairs (j, j + 4), one twiddle
 #pragma unroll
-  for (int j = 0; j < 4; j++) {
-    y[j] = gf_add(y[j], d3_mul<3>(T.a, y[j + 4]));
-    y[j + 4] = gf_add(y[j + 4], y[j]);
-  }
-  // layer d-2: pairs (j, j + 2) in each half h, the prepared twiddle of half h
-  // (below 2^56: its low word's four masked parts, then one shifted copy of
-  // y per set bit of its high word)
-#pragma unroll
-  for (int h = 0; h < 2; h++) {
-    const gf128p* qq = &twq[i18 + h];
-    const uint4 m0 = qq->m[0], m1 = qq->m[1];
-    const uint32_t thi = m1.x | m1.y | m1.z | m1.w;
-#pragma unroll
-    for (int j = 4 * h; j < 4 * h + 2; j++) {
-      y[j] = gf_add(y[j], gf_mul_p40(y[j + 2], m0, thi));
-      y[j + 2] = gf_add(y[j + 2], y[j]);
+    for (int j = 0; j < 4; j++) {
+      y[j] = gf_add(y[j], d3_mul<3>(T.a, y[j + 4]));
+      y[j + 4] = gf_add(y[j + 4], y[j]);
     }
-  }
-  // layer d-1: pairs (2 i, 2 i + 1), twiddle c[i]
+    // layer d-2: pairs (j, j + 2) in each half h, the prepared twiddle of half h
+    // (below 2^56: its low word's four masked parts, then one shifted copy of
+    // y per set bit of its high word)
 #pragma unroll
-  for (int i = 0; i < 4; i++) {
-    y[2 * i] = gf_add(y[2 * i], d3_mul<1>(T.c[i], y[2 * i + 1]));
-    y[2 * i + 1] = gf_add(y[2 * i + 1], y[2 * i]);
-  }
+    for (int h = 0; h < 2; h++) {
+      const gf128p* qq = &twq[i18 + h];
+      const uint4 m0 = qq->m[0], m1 = qq->m[1];
+      const uint32_t thi = m1.x | m1.y | m1.z | m1.w;
 #pragma unroll
-  for (int j = 0; j < 8; j++) gf_store(&data[((q << 3) | (size_t)j) * D3_LANES + lane], y[j]);
+      for (int j = 4 * h; j < 4 * h + 2; j++) {
+        y[j] = gf_add(y[j], gf_mul_p40(y[j + 2], m0, thi));
+        y[j + 2] = gf_add(y[j + 2], y[j]);
+      }
+    }
+    // layer d-1: pairs (2 i, 2 i + 1), twiddle c[i]
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      y[2 * i] = gf_add(y[2 * i], d3_mul<1>(T.c[i], y[2 * i + 1]));
+      y[2 * i + 1] = gf_add(y[2 * i + 1], y[2 * i]);
+    }
+#pragma unroll
+    for (int j = 0; j < 8; j++) gf_store(&data[((q << 3) | (size_t)j) * (ONE ? D3_LANES : lanes) + lane0], y[j]);
+  }
 }
 
 // The deep-table pass in place on data (the caller checked deep3_applies).
-int run_deep3(gf128* data, const gf128* twp, const void* twq, int log_d, cudaStream_t st) {
-  ntt_deep3_kernel<<<(unsigned)((size_t)1 << (log_d - 3)), D3_LANES, 0, st>>>(data, twp, (const gf128p*)twq, log_d);
+int run_deep3(gf128* data, const gf128* twp, const void* twq, int log_d, int log_lanes, cudaStream_t st) {
+  const unsigned grid = (unsigned)((size_t)1 << (log_d - 3));
+  if ((1 << log_lanes) == D3_LANES)
+    ntt_deep3_kernel<true><<<grid, D3_LANES, 0, st>>>(data, twp, (const gf128p*)twq, log_d, D3_LANES);
+  else
+    ntt_deep3_kernel<false><<<grid, D3_LANES, 0, st>>>(data, twp, (const gf128p*)twq, log_d, 1 << log_lanes);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
@@ -871,7 +924,8 @@ const void* flock_ntt_twiddles_prepared(int log_d) {
 // and two timed runs per candidate): the table passes for each table depth of
 // kTabMinLogs, and the multiply passes of every pass shape from each depth's
 // end layer, plus the deep-table pass where a depth leaves exactly the last
-// three layers of a 64-lane code and, for 8-lane codes, the stage passes from
+// three layers of a code of 64 lanes or more (a one-layer table pass first where
+// the depths would be a layer off) and, for 8-lane codes, the stage passes from
 // every depth's end (up to 2^15 positions from every smaller one); it keeps the
 // pair with the smallest sum for later calls. All candidates compute identical results; only
 // speed differs. FLOCK_NTT_TUNE=0 in the environment turns tuning off (the
@@ -898,11 +952,18 @@ bool tuning_enabled() {
   return !(e && e[0] == '0');
 }
 
-// Table passes of layers [from, to) in place on d.
-int run_tab_passes(gf128* d, const gf128* twp, int log_d, int log_lanes, int from, int to, cudaStream_t st) {
-  for (int l = from; l + 2 <= to; l += 2) {
-    const int rc = launch_tab2(d, d, ~(size_t)0, twp, log_d, log_lanes, l, st);
+// Table passes of layers [from, to) of src's positions (by mask) into d: pairs
+// of layers, after a single one where they are odd in number.
+int run_tab_passes(gf128* d, const gf128* src, size_t mask, const gf128* twp, int log_d, int log_lanes, int from, int to,
+                   cudaStream_t st) {
+  for (int l = from; l < to;) {
+    const bool one = (to - l) & 1;
+    const int rc = one ? launch_tab1(d, src, mask, twp, log_d, log_lanes, l, st)
+                       : launch_tab2(d, src, mask, twp, log_d, log_lanes, l, st);
     if (rc != FLOCK_OK) return rc;
+    src = d;
+    mask = ~(size_t)0;
+    l += one ? 1 : 2;
   }
   return FLOCK_OK;
 }
@@ -938,6 +999,9 @@ TunedShape tune_shape(const TuneKey& k, const void* tw, const gf128* twp, cudaSt
   // table passes too
   std::vector<int> ends;
   for (int ml : kTabMinLogs) ends.push_back(tab_layers_end(k.log_d, k.log_lanes, k.start, ml));
+  // a depth that leaves the deep-table pass its three layers, a layer off the pairs
+  if ((k.log_d - 3 - k.start) % 2 && k.log_d - 3 > k.start && deep3_applies(k.log_d, k.log_lanes, k.log_d - 3))
+    ends.push_back(k.log_d - 3);
   if (k.log_d <= 15 && stage_applies(k.log_d, k.log_lanes, k.start))
     for (int te = k.start; te < ends[0]; te += 2)
       if (std::find(ends.begin(), ends.end(), te) == ends.end()) ends.push_back(te);
@@ -945,7 +1009,9 @@ TunedShape tune_shape(const TuneKey& k, const void* tw, const gf128* twp, cudaSt
     if (te > k.start && !twp) continue;
     if (!tab_ms.count(te))
       tab_ms[te] = te == k.start ? 0.f
-                                 : time_of([&] { return run_tab_passes(d, twp, k.log_d, k.log_lanes, k.start, te, st); });
+                                 : time_of([&] {
+                                     return run_tab_passes(d, d, ~(size_t)0, twp, k.log_d, k.log_lanes, k.start, te, st);
+                                   });
     for (int v = 0; v < kVariants; v++) {
       const auto key = std::make_pair(te, v);
       if (!mult_ms.count(key))
@@ -972,7 +1038,7 @@ TunedShape tune_shape(const TuneKey& k, const void* tw, const gf128* twp, cudaSt
     // the deep-table pass, where the multiply part is exactly the last three layers
     if (twp && deep3_applies(k.log_d, k.log_lanes, te)) {
       const auto key = std::make_pair(te, kDeepVariant);
-      if (!mult_ms.count(key)) mult_ms[key] = time_of([&] { return run_deep3(d, twp, tw, k.log_d, st); });
+      if (!mult_ms.count(key)) mult_ms[key] = time_of([&] { return run_deep3(d, twp, tw, k.log_d, k.log_lanes, st); });
       const float t = tab_ms[te] + mult_ms[key];
       if (t < best_ms) {
         best_ms = t;
@@ -1058,14 +1124,12 @@ int flock_launch_ntt(void* d_data, const void* d_src, int log_d, int log_lanes, 
   const gf128* twp = (const gf128*)flock_ntt_twiddles(log_d);
   if (!twp) return FLOCK_ERR_OOM;
   const TunedShape sh = pick_shape(log_d, log_lanes, start_layer, tw, twp, stream);
-  const int tab_end = sh.tab_end;
-  if (tab_end > l) {
-    for (; l + 2 <= tab_end; l += 2) {
-      int rc = launch_tab2(data, src, mask, twp, log_d, log_lanes, l, stream);
-      if (rc != FLOCK_OK) return rc;
-      src = data;
-      mask = ~(size_t)0;
-    }
+  if (sh.tab_end > l) {
+    const int rc = run_tab_passes(data, src, mask, twp, log_d, log_lanes, l, sh.tab_end, stream);
+    if (rc != FLOCK_OK) return rc;
+    src = data;
+    mask = ~(size_t)0;
+    l = sh.tab_end;
   }
   if (l == log_d) return FLOCK_OK;
   if (sh.variant == kStageVariant) {
@@ -1073,7 +1137,7 @@ int flock_launch_ntt(void* d_data, const void* d_src, int log_d, int log_lanes, 
     return run_passes<true>(kDefaultVariant, data, src, mask, tw, log_d, log_lanes, l, stream);
   }
   if (sh.variant == kDeepVariant) {
-    if (src == data && deep3_applies(log_d, log_lanes, l)) return run_deep3(data, twp, tw, log_d, stream);
+    if (src == data && deep3_applies(log_d, log_lanes, l)) return run_deep3(data, twp, tw, log_d, log_lanes, stream);
     return run_passes<true>(kDefaultVariant, data, src, mask, tw, log_d, log_lanes, l, stream);
   }
   return run_passes<true>(sh.variant, data, src, mask, tw, log_d, log_lanes, l, stream);
