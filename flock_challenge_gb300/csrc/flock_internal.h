@@ -70,8 +70,12 @@ int flock_launch_bind_pairs(const void* A, const void* B, size_t n, const uint64
 size_t flock_lc_fold_scratch_bytes(size_t n_stripes);
 int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi, int lo_bits,
                          void* scratch, void* z_vec, int* fault, cudaStream_t st);
-int flock_launch_lc_comb(const uint32_t* a_ptr, const uint32_t* a_idx, const uint32_t* b_ptr,
-                         const uint32_t* b_idx, const void* eq, const uint64_t alpha[2], const uint64_t beta[2],
+// The base matrices' device copies (HostCsc, r1cs_setup.h).
+struct FlockLcMatrices {
+  const uint32_t *a_ptr, *a_mid, *b_ptr, *b_mid, *order, *g_ptr;
+  const uint16_t *a_idx, *b_idx;
+};
+int flock_launch_lc_comb(const FlockLcMatrices& M, const void* eq, const uint64_t alpha[2], const uint64_t beta[2],
                          int pin, void* comb, cudaStream_t st);
 int flock_launch_lc_quirky_eq(const void* lag, const void* x_rest, int n_rest, void* out, cudaStream_t st);
 

@@ -4,11 +4,13 @@
 //    from the byte stripe (byte (outer/8)*2^14 + i holds 8 outer bits), as a
 //    bit-matrix product on the tensor cores (lincheck.rs:655-720);
 //  * comb: alpha * A0^T eq_inner + B0^T eq_inner (+ beta at the constant
-//    column) gathered column-wise from a CSC copy of the base matrices;
+//    column) gathered column-wise from a CSC copy of the base matrices
+//    (r1cs_setup.h);
 //  (the product sumcheck rounds over (comb, z_vec), binding the top variable
 //  (lincheck.rs:1242-1300), run on flock_launch_chain_round).
 #include "flock_internal.h"
 #include "gf128.cuh"
+#include "r1cs_setup.h"
 #include "tc.cuh"
 
 namespace {
@@ -190,45 +192,95 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
 }
 
 // comb[c] = alpha * sum_{r in colA(c)} eq[r] + sum_{r in colB(c)} eq[r] (+ beta at pin).
-// One warp per column: the lanes stride over the column's row indices
-// (coalesced index reads, independent gathers of eq from L2) and XOR-reduce;
-// columns hold 0..7.4 K entries (930 + 355 on average).
-constexpr int LC_COMB_THREADS = 256;
-__global__ void __launch_bounds__(LC_COMB_THREADS)
-lc_comb_kernel(const uint32_t* __restrict__ a_ptr, const uint32_t* __restrict__ a_idx,
-               const uint32_t* __restrict__ b_ptr, const uint32_t* __restrict__ b_idx,
-               const gf128* __restrict__ eq, gf128 alpha, gf128 beta, int pin, gf128* __restrict__ comb) {
-  const int c = (int)((blockIdx.x * (size_t)LC_COMB_THREADS + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-  if (c >= FLOCK_K) return;
-  gf128 sa = gf_zero(), sb = gf_zero();
-  for (uint32_t k = a_ptr[c] + lane, e = a_ptr[c + 1]; k < e; k += 32) sa = gf_add(sa, eq[a_idx[k]]);
-  for (uint32_t k = b_ptr[c] + lane, e = b_ptr[c + 1]; k < e; k += 32) sb = gf_add(sb, eq[b_idx[k]]);
-  for (int off = 16; off > 0; off >>= 1)
+// Columns hold 0..7.4 K entries (930 + 355 on average): 21 M gathers of 16 bytes.
+// Half the eq table (8192 rows, 128 KB) sits in shared memory at a time, and a
+// CTA takes its columns, longest first, a warp each: random 16-byte lookups
+// there take about ten clocks a warp, from L1 (the form before: a warp per
+// column over the whole table in global memory, 57 us) one line each. Row indices
+// are 16 bits. 48 us: the data path is 80% busy while an SM works, but each half
+// waits for its longest column, a third of the time. (The next eight index loads
+// in flight under the lookups: 55 us, their bounds checks cost more.)
+constexpr int LCC_THREADS = 1024, LCC_ROWS = FLOCK_K / 2;
+constexpr int LCC_MAX_COLS = (FLOCK_K + kLcGroups - 1) / kLcGroups + 1;
+constexpr size_t LCC_SMEM = ((size_t)LCC_ROWS + 1) * 16 + (size_t)LCC_MAX_COLS * 2 * 16;
+__global__ void __launch_bounds__(LCC_THREADS, 1)
+lc_comb_kernel(const FlockLcMatrices M, const gf128* __restrict__ eq, gf128 alpha, gf128 beta, int pin,
+               gf128* __restrict__ comb) {
+  extern __shared__ gf128 lcc[];  // half the eq table, then the columns' sums (a, b)
+  __shared__ int next[2];
+  gf128* sums = lcc + LCC_ROWS + 1;
+  const int t = threadIdx.x, lane = t & 31;
+  const uint32_t g0 = M.g_ptr[blockIdx.x], n = M.g_ptr[blockIdx.x + 1] - g0;
+  if (t < 2) next[t] = 0;
+  if (t == 2) lcc[LCC_ROWS] = gf_zero();
+  for (int half = 0; half < 2; half++) {
+    __syncthreads();
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      sa.w[q] ^= __shfl_xor_sync(0xffffffffu, sa.w[q], off);
-      sb.w[q] ^= __shfl_xor_sync(0xffffffffu, sb.w[q], off);
+    for (int k = 0; k < LCC_ROWS / LCC_THREADS; k++)
+      lcc[k * LCC_THREADS + t] = gf_load(&eq[half * LCC_ROWS + k * LCC_THREADS + t]);
+    __syncthreads();
+    for (;;) {
+      uint32_t i = 0;
+      if (lane == 0) i = (uint32_t)atomicAdd(&next[half], 1);
+      i = __shfl_sync(0xffffffffu, i, 0);
+      if (i >= n) break;
+      const uint32_t c = M.order[g0 + i];
+#pragma unroll
+      for (int m = 0; m < 2; m++) {
+        const uint32_t *ptr = m ? M.b_ptr : M.a_ptr, *mid = m ? M.b_mid : M.a_mid;
+        const uint16_t* idx = m ? M.b_idx : M.a_idx;
+        const uint32_t begin = half ? mid[c] : ptr[c], end = half ? ptr[c + 1] : mid[c];
+        gf128 s = gf_zero();
+        // eight index loads in flight; past the end the entry behind the table, zero
+        for (uint32_t k0 = begin; k0 < end; k0 += 8 * 32) {
+          uint32_t r[8];
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            const uint32_t k = k0 + 32 * q + lane;
+            r[q] = k < end ? idx[k] : LCC_ROWS;
+          }
+#pragma unroll
+          for (int q = 0; q < 8; q++)
+            if (k0 + 32 * q < end) s = gf_add(s, lcc[r[q]]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; q++) s.w[q] = __reduce_xor_sync(0xffffffffu, s.w[q]);
+        if (lane == 0) sums[2 * i + m] = half ? gf_add(sums[2 * i + m], s) : s;
+      }
     }
-  if (lane == 0) {
-    gf128 v = gf_add(gf_mul(alpha, sa), sb);
+  }
+  __syncthreads();
+  for (uint32_t i = t; i < n; i += LCC_THREADS) {
+    const int c = (int)M.order[g0 + i];
+    gf128 v = gf_add(gf_mul(alpha, sums[2 * i]), sums[2 * i + 1]);
     if (c == pin) v = gf_add(v, beta);
     comb[c] = v;
   }
 }
 
 // Quirky eq table (lincheck.rs:1127-1143): out[s + 64 * j] = lag[s] * eq(x_inner_rest)[j].
-__global__ void lc_quirky_eq_kernel(const gf128* __restrict__ lag, const gf128* __restrict__ x_rest, int n_rest,
-                                    gf128* __restrict__ out) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= (64 << n_rest)) return;
-  int s = i & 63, j = i >> 6;
-  gf128 e = gf_one();
-  for (int k = 0; k < n_rest; k++) {
-    gf128 r = x_rest[k];
-    if (!((j >> k) & 1)) r.w[0] ^= 1;
-    e = gf_mul(e, r);
+// A block takes four j: their eq values by eight lanes each, multiplied up in
+// three steps, then one product per entry.
+constexpr int LQ_MAX_REST = 8;
+__global__ void __launch_bounds__(256)
+lc_quirky_eq_kernel(const gf128* __restrict__ lag, const gf128* __restrict__ x_rest, int n_rest,
+                    gf128* __restrict__ out) {
+  __shared__ gf128 ej[4];
+  const int t = threadIdx.x, i = blockIdx.x * 256 + t;
+  const gf128 l = gf_load(&lag[t & 63]);
+  if (t < 32) {
+    const int j = blockIdx.x * 4 + (t >> 3), k = t & 7;
+    gf128 e = gf_one();
+    if (k < n_rest) {
+      e = gf_load(&x_rest[k]);
+      if (!((j >> k) & 1)) e.w[0] ^= 1;
+    }
+#pragma unroll 1
+    for (int off = 1; off < LQ_MAX_REST; off <<= 1) e = gf_mul(e, gf_shfl_xor(e, off));
+    if (k == 0) ej[t >> 3] = e;
   }
-  out[i] = gf_mul(lag[s], e);
+  __syncthreads();
+  if (i < (64 << n_rest)) out[i] = gf_mul(l, ej[t >> 6]);
 }
 
 inline gf128 to_gf(const uint64_t v[2]) {
@@ -266,16 +318,19 @@ int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo
   return parts > 1 ? flock_launch_reduce_rows(partials, parts, FLOCK_K, z_vec, st) : FLOCK_OK;
 }
 
-int flock_launch_lc_comb(const uint32_t* a_ptr, const uint32_t* a_idx, const uint32_t* b_ptr, const uint32_t* b_idx,
-                         const void* eq, const uint64_t alpha[2], const uint64_t beta[2], int pin, void* comb,
-                         cudaStream_t st) {
-  lc_comb_kernel<<<FLOCK_K * 32 / LC_COMB_THREADS, LC_COMB_THREADS, 0, st>>>(a_ptr, a_idx, b_ptr, b_idx,
-                                                                            (const gf128*)eq, to_gf(alpha),
-                                                to_gf(beta), pin, (gf128*)comb); flock_count_launch();
+int flock_launch_lc_comb(const FlockLcMatrices& M, const void* eq, const uint64_t alpha[2], const uint64_t beta[2],
+                         int pin, void* comb, cudaStream_t st) {
+  flock_once_per_device((const void*)lc_comb_kernel, [] {
+    cudaFuncSetAttribute(lc_comb_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)LCC_SMEM);
+  });
+  lc_comb_kernel<<<kLcGroups, LCC_THREADS, LCC_SMEM, st>>>(M, (const gf128*)eq, to_gf(alpha), to_gf(beta), pin,
+                                                           (gf128*)comb);
+  flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
 
 int flock_launch_lc_quirky_eq(const void* lag, const void* x_rest, int n_rest, void* out, cudaStream_t st) {
+  if (n_rest < 0 || n_rest > LQ_MAX_REST) return FLOCK_ERR_SHAPE;
   int n = 64 << n_rest;
   lc_quirky_eq_kernel<<<(n + 255) / 256, 256, 0, st>>>((const gf128*)lag, (const gf128*)x_rest, n_rest,
                                                        (gf128*)out); flock_count_launch();

@@ -286,7 +286,8 @@ struct ProverState {
   DBuf in, z, a, b, stripe, cw, tree, A0, B0, A1, B1, eqlo, eqhi, eqout, part, red, lag, small, eqin, comb,
       zvec, zvec1, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, LO, basis, qbuf, qopen, rows, nidx, nodes,
       grind, lvl_cw[2], lvl_tree[2], chW, chG, zceq;
-  DBuf csc_ap, csc_ai, csc_bp, csc_bi;
+  DBuf csc_meta, csc_ai, csc_bi;  // the base matrices (HostCsc): pointers and order, row indices
+  FlockLcMatrices lcm = {};
   bool csc_ready = false;
   DBuf skl[kSklMax];  // What_k(x^b) tables of the induced basis, per number of variables
   FlockPhaseTimes times;
@@ -326,7 +327,7 @@ struct ProverState {
     std::vector<DBuf*> v = {&in, &z, &a, &b, &stripe, &cw, &tree, &A0, &B0, &A1, &B1, &eqlo, &eqhi, &eqout, &part, &red,
             &lag, &small, &eqin, &comb, &zvec, &zvec1, &tlo0, &thi0, &tlo1, &thi1, &tables, &bc, &f1, &b1,
             &LO, &basis, &qbuf, &qopen, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
-            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &csc_ap, &csc_ai, &csc_bp, &csc_bi};
+            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &csc_meta, &csc_ai, &csc_bi};
     for (DBuf& d : skl) v.push_back(&d);
     return v;
   }
@@ -516,6 +517,29 @@ void* part_buf(ProverState& S, size_t bytes) {
   return S.part.get(bytes);
 }
 
+// The base matrices' device copies, once per prover state.
+void upload_matrices(ProverState& S) {
+  if (S.csc_ready) return;
+  const HostCsc& c = flock_host_csc();
+  const std::vector<uint32_t>* parts[] = {&c.a_ptr, &c.a_mid, &c.b_ptr, &c.b_mid, &c.order, &c.g_ptr};
+  const uint32_t** ptrs[] = {&S.lcm.a_ptr, &S.lcm.a_mid, &S.lcm.b_ptr, &S.lcm.b_mid, &S.lcm.order, &S.lcm.g_ptr};
+  std::vector<uint32_t> meta;
+  size_t off[6];
+  for (int k = 0; k < 6; k++) {
+    off[k] = meta.size();
+    meta.insert(meta.end(), parts[k]->begin(), parts[k]->end());
+  }
+  uint32_t* d = (uint32_t*)S.csc_meta.get(meta.size() * 4);
+  for (int k = 0; k < 6; k++) *ptrs[k] = d + off[k];
+  h2d(S, d, meta.data(), meta.size() * 4);
+  S.lcm.a_idx = (const uint16_t*)S.csc_ai.get(c.a_idx.size() * 2);
+  S.lcm.b_idx = (const uint16_t*)S.csc_bi.get(c.b_idx.size() * 2);
+  h2d(S, S.csc_ai.p, c.a_idx.data(), c.a_idx.size() * 2);
+  h2d(S, S.csc_bi.p, c.b_idx.data(), c.b_idx.size() * 2);
+  CK(flock_stream_wait(S.st, &S.waits, false));
+  S.csc_ready = true;
+}
+
 // Adds to a batch the tables of r, split after lo_bits variables.
 void eq_job(FlockEqBatch& q, const std::vector<F>& r, int lo_bits, DBuf& lo, DBuf& hi) {
   int first = 0;
@@ -684,15 +708,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       CK(cudaMemcpy(S->d_r1t, h, sizeof(ZcRound1Tables), cudaMemcpyHostToDevice));
       delete h;
     }
-    if (!S->csc_ready) {
-      const HostCsc& c = flock_host_csc();
-      h2d(*S, S->csc_ap.get(c.a_ptr.size() * 4), c.a_ptr.data(), c.a_ptr.size() * 4);
-      h2d(*S, S->csc_ai.get(c.a_idx.size() * 4), c.a_idx.data(), c.a_idx.size() * 4);
-      h2d(*S, S->csc_bp.get(c.b_ptr.size() * 4), c.b_ptr.data(), c.b_ptr.size() * 4);
-      h2d(*S, S->csc_bi.get(c.b_idx.size() * 4), c.b_idx.data(), c.b_idx.size() * 4);
-      CK(flock_stream_wait(st, &S->waits, false));
-      S->csc_ready = true;
-    }
+    upload_matrices(*S);
     const Lagrange& LG = lagrange();
     T.setup_ms = clk.lap();
     snap_waits(0);
@@ -1034,8 +1050,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       uint64_t al[2], be[2];
       u2(alpha, al);
       u2(beta, be);
-      FK(flock_launch_lc_comb((const uint32_t*)S->csc_ap.p, (const uint32_t*)S->csc_ai.p, (const uint32_t*)S->csc_bp.p,
-                              (const uint32_t*)S->csc_bi.p, deqin, al, be, 512, dcomb, st));
+      FK(flock_launch_lc_comb(S->lcm, deqin, al, be, 512, dcomb, st));
       int lob = n_outer_log / 2;
       eq_split_dev(*S, x_out, lob, S->eqlo, S->eqhi);
       size_t n_stripes = ((size_t)1 << n_outer_log) / 8;
@@ -1928,15 +1943,7 @@ static int verify_impl(ProverState* S, const uint8_t* data, size_t len, const ch
     F beta = tr.sample();
     std::vector<F> comb(FLOCK_K);
     {
-      if (!S->csc_ready) {
-        const HostCsc& c = flock_host_csc();
-        h2d(*S, S->csc_ap.get(c.a_ptr.size() * 4), c.a_ptr.data(), c.a_ptr.size() * 4);
-        h2d(*S, S->csc_ai.get(c.a_idx.size() * 4), c.a_idx.data(), c.a_idx.size() * 4);
-        h2d(*S, S->csc_bp.get(c.b_ptr.size() * 4), c.b_ptr.data(), c.b_ptr.size() * 4);
-        h2d(*S, S->csc_bi.get(c.b_idx.size() * 4), c.b_idx.data(), c.b_idx.size() * 4);
-        CK(flock_stream_wait(st, &S->waits, false));
-        S->csc_ready = true;
-      }
+      upload_matrices(*S);
       auto lag_z = LG.at(z, 0);
       void* dlag = S->lag.get(64 * 16);
       h2d(*S, dlag, lag_z.data(), 64 * 16);
@@ -1947,8 +1954,7 @@ static int verify_impl(ProverState* S, const uint8_t* data, size_t len, const ch
       uint64_t al[2], be[2];
       u2(alpha, al);
       u2(beta, be);
-      FK(flock_launch_lc_comb((const uint32_t*)S->csc_ap.p, (const uint32_t*)S->csc_ai.p, (const uint32_t*)S->csc_bp.p,
-                              (const uint32_t*)S->csc_bi.p, deqin, al, be, 512, dcomb, st));
+      FK(flock_launch_lc_comb(S->lcm, deqin, al, be, 512, dcomb, st));
       d2h(*S, comb.data(), dcomb, FLOCK_K * 16);
     }
     running = alpha * fa + fb + beta;

@@ -158,15 +158,19 @@ void absorb_rows(hb3::Hasher& h, const std::vector<Lin>& rows) {
   }
 }
 
-void to_csc(const std::vector<Lin>& rows, std::vector<uint32_t>& ptr, std::vector<uint32_t>& idx) {
+void to_csc(const std::vector<Lin>& rows, std::vector<uint32_t>& ptr, std::vector<uint32_t>& mid,
+            std::vector<uint16_t>& idx) {
   ptr.assign(K + 1, 0);
   for (const auto& r : rows)
     for (uint32_t c : r) ptr[c + 1]++;
   for (int c = 0; c < K; c++) ptr[c + 1] += ptr[c];
   idx.assign(ptr[K], 0);
+  mid.assign(K, 0);
   std::vector<uint32_t> fill(ptr.begin(), ptr.end() - 1);
-  for (int r = 0; r < K; r++)
-    for (uint32_t c : rows[r]) idx[fill[c]++] = (uint32_t)r;
+  for (int r = 0; r < K; r++) {
+    if (r == K / 2) mid = fill;
+    for (uint32_t c : rows[r]) idx[fill[c]++] = (uint16_t)(r % (K / 2));
+  }
 }
 
 std::mutex g_mu;
@@ -211,8 +215,23 @@ const HostCsc& flock_host_csc() {
   if (!g_csc) {
     const Mats& M = mats();
     g_csc = new HostCsc;
-    to_csc(M.A, g_csc->a_ptr, g_csc->a_idx);
-    to_csc(M.B, g_csc->b_ptr, g_csc->b_idx);
+    HostCsc& h = *g_csc;
+    to_csc(M.A, h.a_ptr, h.a_mid, h.a_idx);
+    to_csc(M.B, h.b_ptr, h.b_mid, h.b_idx);
+    auto len = [&](uint32_t c) { return h.a_ptr[c + 1] - h.a_ptr[c] + h.b_ptr[c + 1] - h.b_ptr[c]; };
+    std::vector<uint32_t> by_len(K);
+    for (int c = 0; c < K; c++) by_len[c] = (uint32_t)c;
+    std::stable_sort(by_len.begin(), by_len.end(), [&](uint32_t x, uint32_t y) { return len(x) > len(y); });
+    std::vector<std::vector<uint32_t>> groups(kLcGroups);
+    for (int i = 0; i < K; i++) {
+      const int turn = i / kLcGroups, g = i % kLcGroups;
+      groups[turn & 1 ? kLcGroups - 1 - g : g].push_back(by_len[i]);
+    }
+    h.g_ptr.push_back(0);
+    for (const auto& g : groups) {
+      h.order.insert(h.order.end(), g.begin(), g.end());
+      h.g_ptr.push_back((uint32_t)h.order.size());
+    }
   }
   return *g_csc;
 }
