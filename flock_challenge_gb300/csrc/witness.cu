@@ -239,6 +239,187 @@ witness_kernel(const flock_compression* __restrict__ in, size_t n_in, size_t n_t
   while (k.word < KWORDS) k.emit(c, 0, 0, 0);
 }
 
+// ---- few compressions ------------------------------------------------------
+//
+// With a thread per compression a small batch is one thread's chain of about ten
+// thousand instructions, unrolled and fetched once (60..70 us whatever the size). Here
+// four lanes take a compression, a column (then diagonal) each: a G's 250
+// witness bits are packed in registers, shifted to their place in the block and
+// joined into the block's image in shared memory (the words a G shares with its
+// neighbours by atomic ORs), the rounds in one loop body. The block then leaves
+// in 16-byte vectors, the stripe bytes by the same 8x8 transposes. 2^8
+// compressions: 70 us through witness_kernel, 11 us so; 2^13: 61 us and 27 us;
+// 2^14: 62 us and 46 us; 2^15: 84 us so (half the threads idle in a G's serial part, so the
+// bandwidth-bound form wins beyond).
+constexpr int WS_COMPS = 16, WS_THREADS = 128, WS_STRIDE = 512 + 4;  // 32-bit words of a block's image, padded
+constexpr size_t WS_SMEM = ((size_t)3 * WS_COMPS * WS_STRIDE + WS_COMPS * 17) * 4;
+constexpr size_t kSmallWitness = (size_t)1 << 14;  // slots
+constexpr int kGBits = 250, kGFirst = 1153, kOutHi = 15153;
+
+__constant__ uint8_t ws_msg[7][16] = {
+    {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15}, {2, 6, 3, 10, 7, 0, 4, 13, 1, 11, 12, 5, 9, 14, 15, 8},
+    {3, 4, 10, 12, 13, 2, 7, 14, 6, 5, 9, 0, 11, 15, 8, 1}, {10, 7, 12, 9, 14, 3, 13, 15, 4, 0, 11, 2, 5, 8, 1, 6},
+    {12, 13, 9, 11, 15, 10, 14, 8, 7, 2, 5, 3, 0, 1, 6, 4}, {9, 14, 11, 5, 8, 12, 15, 1, 13, 3, 0, 10, 2, 6, 4, 7},
+    {11, 15, 5, 0, 1, 9, 8, 6, 14, 10, 2, 12, 3, 4, 7, 13}};
+
+// The 250 bits of one array of a G, 31 bits at a time.
+struct GBits {
+  uint32_t w[8];
+  template <int AT>
+  __device__ __forceinline__ void put(uint32_t v) {
+    w[AT >> 5] |= v << (AT & 31);
+    if constexpr ((AT & 31) != 0 && (AT >> 5) + 1 < 8) w[(AT >> 5) + 1] |= v >> (32 - (AT & 31));
+  }
+  // ORed into the image at bit `at`.
+  __device__ __forceinline__ void store(uint32_t* img, int at) const {
+    uint32_t* d = img + (at >> 5);
+    const int sh = at & 31;
+    atomicOr(d, w[0] << sh);
+#pragma unroll
+    for (int k = 1; k < 7; k++) d[k] = __funnelshift_l(w[k - 1], w[k], sh);
+    atomicOr(d + 7, __funnelshift_l(w[6], w[7], sh));
+    const uint32_t hi = __funnelshift_l(w[7], 0u, sh);
+    if (hi) atomicOr(d + 8, hi);
+  }
+};
+
+__device__ __forceinline__ void ws_or(uint32_t* img, int at, uint32_t v) {
+  const int sh = at & 31;
+  atomicOr(img + (at >> 5), v << sh);
+  if (sh) atomicOr(img + (at >> 5) + 1, v >> (32 - sh));
+}
+
+template <int AT>
+__device__ __forceinline__ uint32_t ws_add(uint32_t x, uint32_t y, GBits& z, GBits& a, GBits& b) {
+  const uint32_t sum = x + y, cin = sum ^ x ^ y;
+  const uint32_t l = (x ^ cin) & 0x7FFFFFFFu, r = (y ^ cin) & 0x7FFFFFFFu;
+  z.put<AT>(l & r);
+  a.put<AT>(l);
+  b.put<AT>(r);
+  return sum;
+}
+
+__global__ void __launch_bounds__(WS_THREADS)
+witness_small_kernel(const flock_compression* __restrict__ in, size_t n_in, size_t n_total, uint64_t* gz, uint64_t* ga,
+                     uint64_t* gb, uint8_t* stripe) {
+  extern __shared__ __align__(16) uint32_t ws_smem[];
+  uint32_t* img[3] = {ws_smem, ws_smem + WS_COMPS * WS_STRIDE, ws_smem + 2 * WS_COMPS * WS_STRIDE};  // z, a, b
+  uint32_t* msgs = ws_smem + 3 * WS_COMPS * WS_STRIDE;
+  const int t = threadIdx.x;
+  const size_t slot0 = (size_t)blockIdx.x * WS_COMPS;
+  const int n_valid = n_total - slot0 < WS_COMPS ? (int)(n_total - slot0) : WS_COMPS;
+  for (int e = t; e < 3 * WS_COMPS * WS_STRIDE / 4; e += WS_THREADS)
+    reinterpret_cast<uint4*>(ws_smem)[e] = make_uint4(0, 0, 0, 0);
+  for (int e = t; e < WS_COMPS * 16; e += WS_THREADS) {
+    const size_t slot = slot0 + (e >> 4);
+    msgs[(e >> 4) * 17 + (e & 15)] = slot < n_in ? in[slot].m[e & 15] : 0u;
+  }
+  __syncthreads();
+  if (t < 4 * WS_COMPS) {
+    const int comp = t >> 2, q = t & 3;
+    const size_t slot = slot0 + comp;
+    uint32_t *z = img[0] + comp * WS_STRIDE, *ia = img[1] + comp * WS_STRIDE, *ib = img[2] + comp * WS_STRIDE;
+    const uint32_t* m = msgs + comp * 17;
+    uint32_t cv0 = 0, cv1 = 0, tail = 0;
+    if (slot < n_in) {
+      const flock_compression& x = in[slot];
+      cv0 = x.cv[q];
+      cv1 = x.cv[4 + q];
+      tail = q == 0 ? (uint32_t)x.counter : q == 1 ? (uint32_t)(x.counter >> 32) : q == 2 ? x.block_len : x.flags;
+    }
+    uint32_t a = cv0, b = cv1, c = q == 0 ? b3::IV(0) : q == 1 ? b3::IV(1) : q == 2 ? b3::IV(2) : b3::IV(3), d = tail;
+    // input words (z = a = value, b = all ones) and the constant bit
+    z[q] = ia[q] = cv0;
+    z[4 + q] = ia[4 + q] = cv1;
+    if (q == 0) {
+      atomicOr(&z[16], 1u);
+      atomicOr(&ia[16], 1u);
+      atomicOr(&ib[36], 1u);
+    }
+    for (int k = q; k < 36; k += 4) ib[k] = 0xFFFFFFFFu;
+    for (int i = 4 * q; i < 4 * q + 4; i++) {
+      ws_or(z, 513 + 32 * i, m[i]);
+      ws_or(ia, 513 + 32 * i, m[i]);
+    }
+    ws_or(z, 1025 + 32 * q, tail);
+    ws_or(ia, 1025 + 32 * q, tail);
+#pragma unroll 1
+    for (int h = 0; h < 14; h++) {  // half rounds: columns, then diagonals
+      const bool diag = h & 1;
+      if (diag) {
+        b = __shfl_sync(0xffffffffu, b, q + 1, 4);
+        c = __shfl_sync(0xffffffffu, c, q + 2, 4);
+        d = __shfl_sync(0xffffffffu, d, q + 3, 4);
+      }
+      const int mi = (diag ? 8 : 0) + 2 * q;
+      const uint32_t mx = m[ws_msg[h >> 1][mi]], my = m[ws_msg[h >> 1][mi + 1]];
+      GBits gz_, ga_, gb_;
+#pragma unroll
+      for (int k = 0; k < 8; k++) gz_.w[k] = ga_.w[k] = gb_.w[k] = 0;
+      const uint32_t t0 = ws_add<0>(a, b, gz_, ga_, gb_);
+      const uint32_t a1 = ws_add<31>(t0, mx, gz_, ga_, gb_);
+      const uint32_t d1 = b3::rotr(d ^ a1, 16);
+      const uint32_t c1 = ws_add<62>(c, d1, gz_, ga_, gb_);
+      const uint32_t b1 = b3::rotr(b ^ c1, 12);
+      const uint32_t t1 = ws_add<93>(a1, b1, gz_, ga_, gb_);
+      a = ws_add<124>(t1, my, gz_, ga_, gb_);
+      d = b3::rotr(d1 ^ a, 8);
+      c = ws_add<155>(c1, d, gz_, ga_, gb_);
+      b = b3::rotr(b1 ^ c, 7);
+      gz_.put<186>(b); ga_.put<186>(b); gb_.put<186>(0xFFFFFFFFu);
+      gz_.put<218>(d); ga_.put<218>(d); gb_.put<218>(0xFFFFFFFFu);
+      const int at = kGFirst + kGBits * (4 * h + q);
+      gz_.store(z, at);
+      ga_.store(ia, at);
+      gb_.store(ib, at);
+      if (diag) {
+        b = __shfl_sync(0xffffffffu, b, q + 3, 4);
+        c = __shfl_sync(0xffffffffu, c, q + 2, 4);
+        d = __shfl_sync(0xffffffffu, d, q + 1, 4);
+      }
+    }
+    z[8 + q] = ia[8 + q] = a ^ c;
+    z[12 + q] = ia[12 + q] = b ^ d;
+    ws_or(z, kOutHi + 32 * q, c ^ cv0);
+    ws_or(ia, kOutHi + 32 * q, c ^ cv0);
+    ws_or(ib, kOutHi + 32 * q, 0xFFFFFFFFu);
+    ws_or(z, kOutHi + 128 + 32 * q, d ^ cv1);
+    ws_or(ia, kOutHi + 128 + 32 * q, d ^ cv1);
+    ws_or(ib, kOutHi + 128 + 32 * q, 0xFFFFFFFFu);
+  }
+  __syncthreads();
+  uint64_t* out[3] = {gz, ga, gb};
+  for (int k = 0; k < 3; k++) {
+    if (!out[k]) continue;
+    uint4* g = reinterpret_cast<uint4*>(out[k] + slot0 * KWORDS);
+    for (int e = t; e < n_valid * 128; e += WS_THREADS)
+      g[e] = *reinterpret_cast<const uint4*>(img[k] + (e >> 7) * WS_STRIDE + 4 * (e & 127));
+  }
+  if (stripe) {
+    for (int item = t; item < (n_valid >> 3) * KWORDS; item += WS_THREADS) {
+      const int grp = item / KWORDS, w = item % KWORDS;
+      uint64_t r8[8], outw[8];
+#pragma unroll
+      for (int r = 0; r < 8; r++) {
+        const uint2 v = *reinterpret_cast<const uint2*>(img[0] + (8 * grp + r) * WS_STRIDE + 2 * w);
+        r8[r] = v.x | ((uint64_t)v.y << 32);
+      }
+#pragma unroll
+      for (int p = 0; p < 8; p++) {
+        uint64_t x = 0;
+#pragma unroll
+        for (int r = 0; r < 8; r++) x |= ((r8[r] >> (8 * p)) & 0xFFull) << (8 * r);
+        outw[p] = transpose8x8(x);
+      }
+      uint4* dst = reinterpret_cast<uint4*>(stripe + ((slot0 >> 3) + grp) * (size_t)FLOCK_K + (size_t)w * 64);
+#pragma unroll
+      for (int k = 0; k < 4; k++)
+        dst[k] = make_uint4((uint32_t)outw[2 * k], (uint32_t)(outw[2 * k] >> 32), (uint32_t)outw[2 * k + 1],
+                            (uint32_t)(outw[2 * k + 1] >> 32));
+    }
+  }
+}
+
 }  // namespace
 
 int flock_launch_witness(const flock_compression* d_in, size_t n_in, int n_blocks_log, void* d_z, void* d_a,
@@ -246,6 +427,15 @@ int flock_launch_witness(const flock_compression* d_in, size_t n_in, int n_block
   size_t n_total = (size_t)1 << n_blocks_log;
   if (n_in > n_total || n_blocks_log < 3) return FLOCK_ERR_SHAPE;
   if ((d_a == nullptr) != (d_b == nullptr)) return FLOCK_ERR_SHAPE;
+  if (n_total <= kSmallWitness) {
+    flock_once_per_device((const void*)witness_small_kernel, [] {
+      cudaFuncSetAttribute(witness_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM);
+    });
+    witness_small_kernel<<<(unsigned)((n_total + WS_COMPS - 1) / WS_COMPS), WS_THREADS, WS_SMEM, stream>>>(
+        d_in, n_in, n_total, (uint64_t*)d_z, (uint64_t*)d_a, (uint64_t*)d_b, (uint8_t*)d_stripe);
+    flock_count_launch();
+    return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+  }
   const int threads = 32 * WARPS_PER_BLOCK;
   size_t blocks = (n_total + threads - 1) / threads;
   size_t smem = (size_t)WARPS_PER_BLOCK * 3 * 32 * STAGE_STRIDE * sizeof(uint64_t);
