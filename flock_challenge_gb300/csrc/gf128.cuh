@@ -42,6 +42,11 @@ __device__ __forceinline__ void gf_load2(const gf128* p, gf128& a, gf128& b) {
                  "=r"(b.w[3])
                : "l"(p));
 }
+__device__ __forceinline__ void gf_store2(gf128* p, gf128 a, gf128 b) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(p), "r"(a.w[0]), "r"(a.w[1]),
+               "r"(a.w[2]), "r"(a.w[3]), "r"(b.w[0]), "r"(b.w[1]), "r"(b.w[2]), "r"(b.w[3])
+               : "memory");
+}
 __device__ __forceinline__ void gf_store(void* p, gf128 a) {
   *reinterpret_cast<uint4*>(p) = make_uint4(a.w[0], a.w[1], a.w[2], a.w[3]);
 }

@@ -771,15 +771,18 @@ zc_round_grp_kernel(const void* __restrict__ in0, const void* __restrict__ in1, 
         } else {
           const gf128* A = reinterpret_cast<const gf128*>(in0);
           const gf128* B = reinterpret_cast<const gf128*>(in1);
-          const gf128 p0 = A[4 * j], p1 = A[4 * j + 1], p2 = A[4 * j + 2], p3 = A[4 * j + 3];
+          gf128 p0, p1, p2, p3, q0, q1, q2, q3;
+          gf_load2(&A[4 * j], p0, p1);
+          gf_load2(&A[4 * j + 2], p2, p3);
+          gf_load2(&B[4 * j], q0, q1);
+          gf_load2(&B[4 * j + 2], q2, q3);
           a0 = gf_add(p0, gf_mul_tab(rtab, gf_add(p0, p1), rot));
           a1 = gf_add(p2, gf_mul_tab(rtab, gf_add(p2, p3), rot));
-          const gf128 q0 = B[4 * j], q1 = B[4 * j + 1], q2 = B[4 * j + 2], q3 = B[4 * j + 3];
           b0 = gf_add(q0, gf_mul_tab(rtab, gf_add(q0, q1), rot));
           b1 = gf_add(q2, gf_mul_tab(rtab, gf_add(q2, q3), rot));
         }
-        Aout[2 * j] = a0; Aout[2 * j + 1] = a1;
-        Bout[2 * j] = b0; Bout[2 * j + 1] = b1;
+        gf_store2(&Aout[2 * j], a0, a1);
+        gf_store2(&Bout[2 * j], b0, b1);
         const uint32_t sh = (uint32_t)(jm * m_mul);
         acc9_shift_xor(t1, gf_mul_wide(a1, b1), sh);
         acc9_shift_xor(ti, gf_mul_wide(gf_add(a0, a1), gf_add(b0, b1)), sh);
