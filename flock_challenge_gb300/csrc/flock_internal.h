@@ -60,6 +60,20 @@ int flock_zc_small_grid(size_t n_pairs);
 int flock_launch_zc_round_small(const void* in0, const void* in1, size_t n_pairs, int skip, const uint64_t rho[2],
                                 const void* lag, void* Aout, void* Bout, const void* eq, void* eq_next,
                                 void* partials, cudaStream_t st);
+// Rounds 0..5 on the tensor cores. fold_a: A0 = the skip fold of a's rows times
+// e1[x_o mod 2^lo_bits]. round_mma: one round over the tables (skip: in_a = A0, in_b
+// = b's bit rows, Bout = B0 written; otherwise both bound at rho into Aout, Bout)
+// with 2^hi_bits high outer indices (weights e2), 2^a_bits phi8 classes (weights
+// cw) and 2^m_bits shift pairs x^(m_mul jm); `grid` rows (G(1), G(inf)) of
+// partials, grid at most 2^(hi_bits + a_bits). unweight: A[i] *= e[(i >> shift)
+// mod 2^lo_bits], n entries. lo_bits + m_bits at least 7.
+int flock_launch_zc_fold_a(const void* a, const void* lag, const void* e1, int lo_bits, int hi_bits, void* A0,
+                           cudaStream_t st);
+int flock_launch_zc_round_mma(const void* in_a, const void* in_b, int skip, const uint64_t rho[2], const void* lag,
+                              void* Aout, void* Bout, const void* e2, const uint64_t cw[4][2], int hi_bits, int a_bits,
+                              int m_bits, int m_mul, int lo_bits, void* partials, int grid, int* fault,
+                              cudaStream_t st);
+int flock_launch_zc_unweight(void* A, size_t n, const void* e, int shift, int lo_bits, cudaStream_t st);
 int flock_launch_bind_pairs(const void* A, const void* B, size_t n, const uint64_t rho[2], void* Aout, void* Bout,
                             cudaStream_t st);
 

@@ -345,6 +345,9 @@ constexpr size_t kHostTailPairs = 512;
 // fold instead of zerocheck round 1 (2^14: round 1 0.26 ms with it; 0.19 ms
 // without, and the fold 0.05 ms).
 constexpr int kFoldCLog = 14;
+// Proofs of at least 2^kMmaRoundsLog compressions run zerocheck rounds 0..5 on the
+// tensor cores (both sides' times at zc_round_mma_kernel).
+constexpr int kMmaRoundsLog = 12;
 // Proofs of at least 2^kSplitMsgLog compressions compute the combined basis and
 // the first Ligerito message in two launches, the message on the tensor cores.
 constexpr int kSplitMsgLog = 13;
@@ -867,6 +870,20 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       F dinv;
       int n_vars;  // variables of the split tables: the round's, less the m_bits after the first a_bits where grp
     };
+    // Rounds 0 .. mma_end - 1 (the grouped ones) on the tensor cores
+    // (zc_round_mma_kernel): from 2^kMmaRoundsLog compressions, unless an outer
+    // challenge whose weight goes into the A table is 0 or 1 (then it could not
+    // be divided out).
+    int mma_end = 0;
+    const int n_out_vars = m - 13, mma_lo = std::min(10, std::max(6, n_out_vars - 8)), mma_hi = n_out_vars - mma_lo;
+    bool mma_rounds = n_log >= kMmaRoundsLog;
+    F a_scale = F::one();  // from round mma_end on the A table is 1 / a_scale of the protocol's
+    if (mma_rounds) {
+      F p = F::one();
+      for (int k = 13; k < 13 + mma_lo; k++) p = p * (r[k] * (F::one() + r[k]));
+      mma_rounds = !p.zero();
+      if (mma_rounds) a_scale = hf::inv(p);
+    }
     auto round_eq = [&](int i) {
       const int nv = m - (6 + i + 1);
       // lowest of the round's variables r[7 + i ..] that are fixed challenges: phi8 ones (r7, r8)
@@ -876,7 +893,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       q.f0 = std::max(9, 7 + i);
       q.m_bits = std::max(0, 13 - q.f0);
       q.small = ((size_t)1 << nv) <= FLOCK_ZC_SMALL_PAIRS;  // 2^nv pairs
-      q.grp = !q.small && q.m_bits > 0 && nv > q.a_bits + q.m_bits;
+      q.grp = (!q.small || mma_rounds) && q.m_bits > 0 && nv > q.a_bits + q.m_bits;
       for (int k = q.f0; q.grp && k < 13; k++) q.grp = shift_var(k);
       q.dinv = F::one();
       if (q.grp) {
@@ -896,6 +913,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       }
       return q;
     };
+    F *mma_e1 = nullptr, *mma_e2 = nullptr, *mma_inv = nullptr;
     std::vector<RoundEq> qs;
     std::vector<std::pair<size_t, size_t>> eq_off;  // (lo, hi) F128 offsets in zceq
     {
@@ -908,13 +926,26 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         eq_off.push_back({tot, tot + ((size_t)1 << q.lob)});
         tot += ((size_t)1 << q.lob) + ((size_t)1 << hb);
       }
+      if (mma_rounds)
+        while (mma_end < 6 && qs[mma_end].grp) mma_end++;
+      mma_rounds = mma_end > 0;
+      const size_t mma_off = tot;  // E1, E2, then eq of 1 + r (a multiple of 1 / E1)
+      if (mma_rounds) tot += ((size_t)2 << mma_lo) + ((size_t)1 << mma_hi) + 1;
       F* deq = (F*)S->zceq.get(tot * 16);
       FlockEqBatch eb;
       eb.n_jobs = 0;
       for (int k = 6; k < m; k++) u2(r[k], eb.r[k - 6]);
+      if (mma_rounds) {
+        mma_e1 = deq + mma_off;
+        mma_e2 = mma_e1 + ((size_t)1 << mma_lo);
+        mma_inv = mma_e2 + ((size_t)1 << mma_hi);
+        for (int k = 0; k < mma_lo; k++) u2(F::one() + r[13 + k], eb.r[m - 6 + k]);
+        eb.jobs[eb.n_jobs++] = {mma_e1, mma_e2, mma_lo, mma_hi, 7, n_out_vars, 0};
+        eb.jobs[eb.n_jobs++] = {mma_inv, mma_inv + ((size_t)1 << mma_lo), mma_lo, 0, m - 6, mma_lo, 0};
+      }
       // a small round's table comes out of the small round before it
       for (int i = 0; i < n_mlv; i++)
-        if (i == 0 || !qs[i].small || !qs[i - 1].small) {
+        if (i >= mma_end && (i == 0 || i == mma_end || !qs[i].small || !qs[i - 1].small)) {
           if (eb.n_jobs >= FLOCK_EQ_JOBS) throw Fail(FLOCK_ERR_SHAPE, "eq tables");
           const RoundEq& q = qs[i];
           eb.jobs[eb.n_jobs++] = {deq + eq_off[i].first, deq + eq_off[i].second, q.lob, q.n_vars - q.lob, i + 1,
@@ -940,7 +971,20 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       if (i > 0) u2(rho.back(), rp);
       int grid;
       void* dpart;
-      if (q.grp) {
+      if (i < mma_end) {
+        uint64_t cw[4][2];
+        for (int k = 0; k < 4; k++) {
+          F w8 = F::one();  // eq of the phi8 variables r[7 + i ..] at the class's bits
+          for (int v = 0; v < q.a_bits; v++) w8 = w8 * (((k >> v) & 1) ? r[7 + i + v] : F::one() + r[7 + i + v]);
+          u2(w8, cw[k]);
+        }
+        if (i == 0) FK(flock_launch_zc_fold_a(da, dlag, mma_e1, mma_lo, mma_hi, dA0, st));
+        grid = std::min(152, 1 << (mma_hi + q.a_bits));
+        dpart = part_buf(*S, (size_t)grid * 2 * 16);
+        FK(flock_launch_zc_round_mma(i == 0 ? dA0 : curA, i == 0 ? db : curB, i == 0, rp, dlag, i == 0 ? nullptr : nxtA,
+                                     i == 0 ? dB0 : nxtB, mma_e2, cw, mma_hi, q.a_bits, q.m_bits, 1 << (q.f0 - 9), mma_lo,
+                                     dpart, grid, S->fault(), st));
+      } else if (q.grp) {
         grid = (int)std::min<size_t>(n_pairs >> (q.lob + q.m_bits), 152 * 4);
         dpart = part_buf(*S, (size_t)grid * 2 * 16);
         FK(flock_launch_zc_round_grp(i == 0 ? da : curA, i == 0 ? db : curB, n_pairs, i == 0, rp, dlag,
@@ -970,6 +1014,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       if (i > 0) {
         std::swap(curA, nxtA);
         std::swap(curB, nxtB);
+      }
+      // round i's pairs have 6 - i inner index bits, its entries one more
+      if (mma_rounds && i == mma_end - 1) FK(flock_launch_zc_unweight(curA, 2 * n_pairs, mma_inv, 7 - i, mma_lo, st));
+      if (mma_rounds && i >= mma_end) {
+        g[0] = g[0] * a_scale;
+        g[1] = g[1] * a_scale;
       }
       zc_rounds.push_back({g[0], g[1]});
       tr.observe(g[0]);
@@ -1012,6 +1062,10 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         hf::weighted_round(tA.data(), tB.data(), eq.data(), tA.size() / 2, &g1, &gi);
         g1 = g1 * qs[i].dinv;
         gi = gi * qs[i].dinv;
+        if (mma_rounds) {
+          g1 = g1 * a_scale;
+          gi = gi * a_scale;
+        }
         zc_rounds.push_back({g1, gi});
         tr.observe(g1);
         tr.observe(gi);
@@ -1022,6 +1076,8 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       fa = tA[0];
       fb = tB[0];
     }
+    if (mma_rounds) fa = fa * a_scale;
+    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "zerocheck round");
     tr.observe(fa);
     tr.observe(fb);
     T.zc_rounds_ms = clk.lap();

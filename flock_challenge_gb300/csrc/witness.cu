@@ -249,8 +249,8 @@ witness_kernel(const flock_compression* __restrict__ in, size_t n_in, size_t n_t
 // neighbours by atomic ORs), the rounds in one loop body. The block then leaves
 // in 16-byte vectors, the stripe bytes by the same 8x8 transposes. 2^8
 // compressions: 70 us through witness_kernel, 11 us so; 2^13: 61 us and 27 us;
-// 2^14: 62 us and 46 us; 2^15: 84 us so (half the threads idle in a G's serial part, so the
-// bandwidth-bound form wins beyond).
+// 2^14: 62 us and 46 us; 2^15: 84 us so (half of a block's threads wait while the
+// rounds run, so the bandwidth-bound form wins beyond).
 constexpr int WS_COMPS = 16, WS_THREADS = 128, WS_STRIDE = 512 + 4;  // 32-bit words of a block's image, padded
 constexpr size_t WS_SMEM = ((size_t)3 * WS_COMPS * WS_STRIDE + WS_COMPS * 17) * 4;
 constexpr size_t kSmallWitness = (size_t)1 << 14;  // slots

@@ -23,6 +23,7 @@
 // packed word x >> 1), so the opening reuses it.
 #include <algorithm>
 
+#include "bit_outer.cuh"
 #include "flock_internal.h"
 #include "gf128.cuh"
 #include "gf_tab.cuh"
@@ -870,6 +871,254 @@ zc_round_small_kernel(const void* __restrict__ in0, const void* __restrict__ in1
   gf_block_sum_lanes(p, 1, partials + 2 * blockIdx.x);  // G(1) from the odd lanes, G(inf) from the even ones
 }
 
+// ---- multilinear rounds 0..5 on the tensor cores ----------------------------
+//
+// The rounds' sums weigh a product of the tables by eq of the fixed inner
+// challenges and of the outer ones (the rows' index x_o). A sum of products runs
+// on the tensor cores for any number of pairs of one weight (bit_outer.cuh), so
+// the weights are taken out of the pairs: eq of the low lo_bits outer
+// variables, E1, is multiplied into the A table once, by zc_fold_a_kernel, whose
+// byte tables of the Lagrange weights carry the factor for free (a CTA takes one
+// low outer index), and stays there while rounds 0..5 bind the inner variables;
+// eq of the other outer variables, E2, and the phi8 challenges' weight are one
+// factor per unit (a high outer index and a phi8 class), multiplied into the
+// unit's two sums; and the shift challenges' weights are powers x^(m_mul jm),
+// jm = lane / 2 and so the same for all of a lane's pairs, applied to A's values as
+// they are expanded. After the last of these rounds the A table is divided by E1
+// (zc_unweight_kernel), up to a constant the host knows.
+//
+// The tiles go as in lig_fold_msg_kernel: eight warps of A, eight of B (SKIP:
+// round 0, B's values come from the bit rows; otherwise both bind at rho through
+// its byte tables), one thread issuing the MMAs. Bound by the shared-memory data
+// path. 2^18 compressions: round 0 2,110 us as carry-less products
+// (zc_round_grp_kernel), 1,144 us so and 405 us for the fold of A; rounds 1..5
+// 2,771 us and 2,146 us; 2^13: rounds 0..2 232 us and 165 + 19 us. Used from 2^12
+// compressions (one chain of 2^12: 2.21 -> 2.16 ms; below, round 0 alone exceeds
+// the small rounds' limit); the grouped kernels stay for 2^11 and for an outer
+// challenge of 0 or 1.
+__global__ void __launch_bounds__(256)
+zc_fold_a_kernel(const uint64_t* __restrict__ W, const gf128* __restrict__ lag, const gf128* __restrict__ e1,
+                 int lo_bits, size_t n_hi, int parts, gf128* __restrict__ A0) {
+  __shared__ gf128 tab[256 * 8];  // [value][byte position], as in zc_round_grp_kernel
+  __shared__ gf128 wl[64];
+  const int t = threadIdx.x;
+  const size_t lo = blockIdx.x / parts;
+  const int part = blockIdx.x % parts;
+  if (t < 64) wl[t] = gf_mul(gf_load(&lag[t]), gf_load(&e1[lo]));
+  __syncthreads();
+  if (t < 128) {
+    const int c = t & 7, g = t >> 3;
+    gf128 v = gf_zero();
+#pragma unroll
+    for (int k = 4; k < 8; k++)
+      if ((g >> (k - 4)) & 1) v = gf_add(v, wl[8 * c + k]);
+#pragma unroll
+    for (int k = 0; k < 16; k++) {
+      if (k) v = gf_add(v, wl[8 * c + gf_tab_ctz4(k)]);
+      tab[((16 * g + (k ^ (k >> 1))) << 3) + c] = v;
+    }
+  }
+  __syncthreads();
+  // two outer indices of 128 rows at a time
+  const size_t h1 = n_hi * (part + 1) / parts;
+  for (size_t h = n_hi * part / parts + (t >> 7); h < h1; h += 2) {
+    const size_t row = (((h << lo_bits) | lo) << 7) + (t & 127);
+    const uint64_t w = W[row];
+    gf128 r = gf_zero();
+#pragma unroll
+    for (int k = 0; k < 8; k++) {
+      const int c = (t + k) & 7;
+      r = gf_add(r, tab[((((uint32_t)(w >> (8 * c))) & 255) << 3) + c]);
+    }
+    gf_store(&A0[row], r);
+  }
+}
+
+// A[i] *= e[(i >> shift) & mask], the entry's low outer index
+__global__ void __launch_bounds__(256)
+zc_unweight_kernel(gf128* __restrict__ A, size_t n, const gf128* __restrict__ e, int shift, int lo_bits) {
+  const size_t mask = ((size_t)1 << lo_bits) - 1;
+  for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
+    gf_store(&A[i], gf_mul(gf_load(&A[i]), gf_load(&e[(i >> shift) & mask])));
+}
+
+struct ZcClassWeights {
+  gf128 w[4];
+};
+
+constexpr int ZM_PRODUCERS = 512, ZM_THREADS = ZM_PRODUCERS + 32, ZM_SLOTS = 4;
+template <bool SKIP>
+constexpr size_t kZmSmem = (size_t)ZM_SLOTS * bo::SLOT + (SKIP ? (size_t)256 * 8 * 16 : (size_t)GF_TAB_ENTRIES * 16);
+static_assert(kZmSmem<false> <= 232448, "round shared memory above the 227 KB per-block limit");
+
+template <bool SKIP>
+__global__ void __launch_bounds__(ZM_THREADS, 1)
+zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b, const gf128 rho,
+                    const gf128* __restrict__ lag, gf128* __restrict__ Aout, gf128* __restrict__ Bout,
+                    const gf128* __restrict__ e2, const __grid_constant__ ZcClassWeights cw, int n_units, int a_bits,
+                    int m_bits, int m_mul, int lo_bits, gf128* __restrict__ partials, volatile int* fault) {
+  extern __shared__ __align__(128) uint8_t zm_smem[];
+  // done[tau mod 8]: the MMAs of tile tau of the CTA's sequence (see lig_fold_msg_kernel)
+  __shared__ uint64_t full[ZM_SLOTS], done[8], unit_done;
+  __shared__ uint32_t tmem_slot, poly[2][2][4][5];
+  constexpr int AHEAD = 4;
+  uint8_t* slots = zm_smem;
+  gf128* tab = reinterpret_cast<gf128*>(zm_smem + (size_t)ZM_SLOTS * bo::SLOT);
+  const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+  const int log_t = lo_bits + m_bits - 7, T = 1 << log_t;  // tiles per unit
+  const int units = (n_units - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;  // this CTA's: at least one
+  const int n = units << log_t;
+  if (warp == 0) tc::tmem_alloc(&tmem_slot, 512);
+  if (t == 0) {
+    for (int k = 0; k < ZM_SLOTS; k++) tc::mbar_init(&full[k], 2);
+    for (int k = 0; k < 8; k++) tc::mbar_init(&done[k], 1);
+    tc::mbar_init(&unit_done, 1);
+    tc::mbar_fence_init();
+  }
+  if constexpr (SKIP) {
+    if (t < 128) {
+      const int c = t & 7, g = t >> 3;
+      gf128 v = gf_zero();
+#pragma unroll
+      for (int k = 4; k < 8; k++)
+        if ((g >> (k - 4)) & 1) v = gf_add(v, gf_load(&lag[8 * c + k]));
+#pragma unroll
+      for (int k = 0; k < 16; k++) {
+        if (k) v = gf_add(v, gf_load(&lag[8 * c + gf_tab_ctz4(k)]));
+        tab[((16 * g + (k ^ (k >> 1))) << 3) + c] = v;
+      }
+    }
+  } else {
+    for (int it = t; it < 256; it += ZM_THREADS) gf_tab_row_direct(rho, reinterpret_cast<uint4*>(tab), it);
+  }
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  const uint32_t tmem = tmem_slot, sf = tmem + 256;
+  if (warp < 4) tc::tmem_fill32(sf + ((uint32_t)(32 * warp) << 16), 0x7f7f7f7fu);
+  tc::fence_before();
+  __syncthreads();
+  tc::fence_after();
+  bool ok = true;
+  const bool is_b = warp >= 8;
+  const int w8 = warp & 7;
+  const uint32_t rot = t & 15, sh = (uint32_t)(m_mul * ((lane >> 1) & ((1 << m_bits) - 1)));
+  // value i of step k of tile tau: pair p = 128 tile + 16 k + lane / 2 of its
+  // unit's class, value lane & 1
+  auto index = [&](int tau, int k) {
+    const size_t u = (size_t)blockIdx.x + (size_t)(tau >> log_t) * gridDim.x;
+    const size_t p = (size_t)(tau & (T - 1)) * bo::TILE + 16 * k + (lane >> 1);
+    const size_t xo = ((u >> a_bits) << lo_bits) | (p >> m_bits);
+    const size_t j = (((xo << m_bits) | (p & (((size_t)1 << m_bits) - 1))) << a_bits) | (u & (((size_t)1 << a_bits) - 1));
+    return 2 * j + (lane & 1);
+  };
+  gf128 y0[AHEAD], y1[AHEAD];
+  auto load = [&](int tau, int k) {
+    const size_t i = index(tau, k);
+    const int q = k % AHEAD;
+    if constexpr (SKIP) {
+      if (is_b) {
+        const uint2 v = reinterpret_cast<const uint2*>(in_b)[i];
+        y0[q].w[0] = v.x;
+        y0[q].w[1] = v.y;
+      } else {
+        y0[q] = gf_load(reinterpret_cast<const gf128*>(in_a) + i);
+      }
+    } else {
+      gf_load2(reinterpret_cast<const gf128*>(is_b ? in_b : in_a) + 2 * i, y0[q], y1[q]);
+    }
+  };
+  if (t < ZM_PRODUCERS && w8 < n) {
+#pragma unroll
+    for (int k = 0; k < AHEAD; k++) load(w8, k);
+  }
+  gf128 acc = gf_zero();  // threads 0, 1: the weighted sums
+  int tau = w8;           // this warp's next tile
+  for (int ul = 0; ul < units; ul++) {
+    const int tau_end = (ul + 1) << log_t;
+    if (t < ZM_PRODUCERS) {
+      for (; tau < tau_end && ok; tau += 8) {
+        gf128 v[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const int q = k % AHEAD;
+          if constexpr (SKIP) {
+            if (is_b) {
+              const uint64_t w = y0[q].w[0] | ((uint64_t)y0[q].w[1] << 32);
+              gf128 r = gf_zero();
+#pragma unroll
+              for (int s = 0; s < 8; s++) {
+                const int c = (t + s) & 7;
+                r = gf_add(r, tab[((((uint32_t)(w >> (8 * c))) & 255) << 3) + c]);
+              }
+              v[k] = r;
+              gf_store(&Bout[index(tau, k)], r);
+            } else {
+              v[k] = y0[q];
+            }
+          } else {
+            v[k] = gf_add(y0[q], gf_mul_tab(reinterpret_cast<const uint4*>(tab), gf_add(y0[q], y1[q]), rot));
+            gf_store(&(is_b ? Bout : Aout)[index(tau, k)], v[k]);
+          }
+          if (k + AHEAD < 8) load(tau, k + AHEAD);
+          else if (tau + 8 < n) load(tau + 8, k + AHEAD - 8);
+        }
+        // the even lane takes the sum a_0 + a_1 (G(inf)), the odd one keeps a_1 (G(1))
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+          const gf128 o = gf_shfl_xor(v[k], 1);
+          if (!(lane & 1)) v[k] = gf_add(v[k], o);
+          if (!is_b) {  // times x^sh
+            const uint32_t ov = __funnelshift_l(v[k].w[3], 0u, sh);
+            v[k].w[3] = __funnelshift_l(v[k].w[2], v[k].w[3], sh);
+            v[k].w[2] = __funnelshift_l(v[k].w[1], v[k].w[2], sh);
+            v[k].w[1] = __funnelshift_l(v[k].w[0], v[k].w[1], sh);
+            v[k].w[0] = (v[k].w[0] << sh) ^ ov ^ (ov << 1) ^ (ov << 2) ^ (ov << 7);
+          }
+        }
+        const int slot = tau % ZM_SLOTS;
+        if (tau >= ZM_SLOTS)
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(tau - ZM_SLOTS) % 8], ((tau - ZM_SLOTS) / 8) & 1));
+        if (ok) bo::put_tile(v, slots + slot * bo::SLOT + (is_b ? bo::SIDE : 0), 1 - (lane & 1));
+        tc::fence_smem_for_mma();
+        __syncwarp();
+        if (lane == 0) tc::mbar_arrive(&full[slot]);
+      }
+    } else if (lane == 0) {
+      for (int x = ul << log_t; x < tau_end && ok; x++) {
+        const int slot = x % ZM_SLOTS;
+        ok = tc::mbar_wait(&full[slot], (x / ZM_SLOTS) & 1);
+        if (!ok) break;
+        tc::fence_after();
+        bo::mma_slot(tc::smem_addr(slots + slot * bo::SLOT), tmem, sf, (x & (T - 1)) == 0);
+        tc::mma_commit(&done[x % 8]);
+      }
+      tc::mma_commit(&unit_done);
+    }
+    __syncwarp();
+    ok = tc::mbar_wait(&unit_done, ul & 1) && ok;
+    __syncwarp();
+    tc::fence_after();
+    if (warp < 8) bo::read_quadrant(tmem + 128 * (warp >> 2), poly[ul & 1][warp >> 2][warp & 3]);
+    tc::fence_before();
+    if (__syncthreads_or(!ok)) {  // the counts are read, or a wait gave up
+      ok = false;
+      break;
+    }
+    tc::fence_after();
+    if (t < 2) {
+      const size_t u = (size_t)blockIdx.x + (size_t)ul * gridDim.x;
+      const gf128 w = gf_mul(cw.w[u & (((size_t)1 << a_bits) - 1)], gf_load(&e2[u >> a_bits]));
+      acc = gf_add(acc, gf_mul(w, bo::combine(poly[ul & 1][t])));
+    }
+  }
+  if (!ok) *fault = 1;
+  if (t < 2) partials[2 * blockIdx.x + t] = acc;
+  tc::fence_before();
+  __syncthreads();
+  if (warp == 0) tc::tmem_free(tmem, 512);
+}
+
 // Final bind of the last round: out[j] = A0 + rho (A0 + A1).
 __global__ void bind_pairs_kernel(const gf128* __restrict__ A, const gf128* __restrict__ B, size_t n, gf128 rho,
                                   gf128* __restrict__ Aout, gf128* __restrict__ Bout) {
@@ -1001,6 +1250,53 @@ int flock_launch_zc_round_small(const void* in0, const void* in1, size_t n_pairs
     zc_round_small_kernel<false><<<grid, threads, 0, st>>>(
         in0, in1, n_pairs, r, (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)eq, (gf128*)eq_next,
         (gf128*)partials);
+  flock_count_launch();
+  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+}
+
+int flock_launch_zc_fold_a(const void* a, const void* lag, const void* e1, int lo_bits, int hi_bits, void* A0,
+                           cudaStream_t st) {
+  const size_t n_hi = (size_t)1 << hi_bits;
+  size_t parts = 1;  // at least two CTAs per SM
+  while ((parts << lo_bits) < 512 && 2 * parts <= n_hi) parts *= 2;
+  zc_fold_a_kernel<<<(unsigned)(parts << lo_bits), 256, 0, st>>>((const uint64_t*)a, (const gf128*)lag,
+                                                                (const gf128*)e1, lo_bits, n_hi, (int)parts, (gf128*)A0);
+  flock_count_launch();
+  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+}
+
+int flock_launch_zc_unweight(void* A, size_t n, const void* e, int shift, int lo_bits, cudaStream_t st) {
+  const size_t grid = std::min<size_t>((n + 255) / 256, (size_t)152 * 16);
+  zc_unweight_kernel<<<(unsigned)grid, 256, 0, st>>>((gf128*)A, n, (const gf128*)e, shift, lo_bits);
+  flock_count_launch();
+  return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
+}
+
+int flock_launch_zc_round_mma(const void* in_a, const void* in_b, int skip, const uint64_t rho[2], const void* lag,
+                              void* Aout, void* Bout, const void* e2, const uint64_t cw[4][2], int hi_bits, int a_bits,
+                              int m_bits, int m_mul, int lo_bits, void* partials, int grid, int* fault,
+                              cudaStream_t st) {
+  const int n_units = 1 << (hi_bits + a_bits);
+  if (a_bits < 0 || a_bits > 2 || m_bits < 1 || m_bits > 4 || m_mul < 1 || m_mul * ((1 << m_bits) - 1) > 15 ||
+      lo_bits + m_bits < 7 || hi_bits < 0 || hi_bits + a_bits > 24 || grid < 1 || grid > n_units)
+    return FLOCK_ERR_SHAPE;
+  flock_once_per_device((const void*)zc_round_mma_kernel<true>, [] {
+    cudaFuncSetAttribute(zc_round_mma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZmSmem<true>);
+    cudaFuncSetAttribute(zc_round_mma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kZmSmem<false>);
+  });
+  auto gf = [](const uint64_t v[2]) {
+    return gf128{{(uint32_t)v[0], (uint32_t)(v[0] >> 32), (uint32_t)v[1], (uint32_t)(v[1] >> 32)}};
+  };
+  ZcClassWeights w;
+  for (int k = 0; k < 4; k++) w.w[k] = gf(cw[k]);
+  if (skip)
+    zc_round_mma_kernel<true><<<grid, ZM_THREADS, kZmSmem<true>, st>>>(
+        in_a, in_b, gf(rho), (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)e2, w, n_units, a_bits, m_bits,
+        m_mul, lo_bits, (gf128*)partials, fault);
+  else
+    zc_round_mma_kernel<false><<<grid, ZM_THREADS, kZmSmem<false>, st>>>(
+        in_a, in_b, gf(rho), (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)e2, w, n_units, a_bits, m_bits,
+        m_mul, lo_bits, (gf128*)partials, fault);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }
