@@ -427,7 +427,9 @@ int flock_launch_witness(const flock_compression* d_in, size_t n_in, int n_block
   size_t n_total = (size_t)1 << n_blocks_log;
   if (n_in > n_total || n_blocks_log < 3) return FLOCK_ERR_SHAPE;
   if ((d_a == nullptr) != (d_b == nullptr)) return FLOCK_ERR_SHAPE;
-  if (n_total <= kSmallWitness) {
+  // (its 16-byte stores; witness_kernel stores z, a and b by 8 bytes)
+  const bool aligned = (((uintptr_t)d_z | (uintptr_t)d_a | (uintptr_t)d_b) & 15) == 0;
+  if (n_total <= kSmallWitness && aligned) {
     flock_once_per_device((const void*)witness_small_kernel, [] {
       cudaFuncSetAttribute(witness_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM);
     });
