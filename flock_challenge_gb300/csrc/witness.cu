@@ -15,7 +15,7 @@
 // completes witness word w at the same instruction. Completed 64-bit words are
 // staged per warp in shared memory and written out 16 words at a time as
 // 128-byte runs per compression; the stripe bytes of each group of eight
-// compressions are produced from the same staging by 8x8 bit transposes.
+// compressions are produced from the same staging by bit transposes.
 #include <cstdint>
 
 #include "blake3.cuh"
@@ -41,12 +41,45 @@ struct WarpCtx {
   int lane;
 };
 
-__device__ __forceinline__ uint64_t transpose8x8(uint64_t x) {
-  uint64_t t;
-  t = (x ^ (x >> 7)) & 0x00AA00AA00AA00AAull; x = x ^ t ^ (t << 7);
-  t = (x ^ (x >> 14)) & 0x0000CCCC0000CCCCull; x = x ^ t ^ (t << 14);
-  t = (x ^ (x >> 28)) & 0x00000000F0F0F0F0ull; x = x ^ t ^ (t << 28);
-  return x;
+// The stripe bytes of one witness word of eight compressions (rows): byte 8 p + i
+// of the 64 is bit i of byte p of the rows, row r at bit r. Three rounds of bit
+// exchanges between the rows' registers (row bit against bit index), after
+// which row i holds the bytes of bit i, then 4 x 4 byte transposes.
+// Gathering each byte of the rows by shifts and transposing 8 x 8 bits at a time
+// cost several times the instructions: 2^17 slots of witness_kernel 199 -> 180 us,
+// 0.89 of the measured HBM rate.
+__device__ __forceinline__ void stripe_exchange(uint32_t& a, uint32_t& b, int k, uint32_t low) {
+  const uint32_t t = ((a >> k) ^ b) & low;
+  b ^= t;
+  a ^= t << k;
+}
+
+__device__ __forceinline__ void stripe_bytes(const uint64_t* rows, uint4* out) {
+#pragma unroll
+  for (int h = 0; h < 2; h++) {  // bytes 0..3 and 4..7 of the words
+    uint32_t v[8];
+#pragma unroll
+    for (int r = 0; r < 8; r++) v[r] = (uint32_t)(rows[r] >> (32 * h));
+#pragma unroll
+    for (int r = 0; r < 4; r++) stripe_exchange(v[r], v[r + 4], 4, 0x0F0F0F0Fu);
+#pragma unroll
+    for (int r = 0; r < 4; r++) stripe_exchange(v[r + (r & 2)], v[r + (r & 2) + 2], 2, 0x33333333u);
+#pragma unroll
+    for (int r = 0; r < 4; r++) stripe_exchange(v[2 * r], v[2 * r + 1], 1, 0x55555555u);
+    uint32_t w[4][2];  // [byte][bits 0..3, 4..7]
+#pragma unroll
+    for (int q = 0; q < 2; q++) {
+      const uint32_t x0 = __byte_perm(v[4 * q], v[4 * q + 1], 0x5140), x1 = __byte_perm(v[4 * q], v[4 * q + 1], 0x7362);
+      const uint32_t y0 = __byte_perm(v[4 * q + 2], v[4 * q + 3], 0x5140);
+      const uint32_t y1 = __byte_perm(v[4 * q + 2], v[4 * q + 3], 0x7362);
+      w[0][q] = __byte_perm(x0, y0, 0x5410);
+      w[1][q] = __byte_perm(x0, y0, 0x7632);
+      w[2][q] = __byte_perm(x1, y1, 0x5410);
+      w[3][q] = __byte_perm(x1, y1, 0x7632);
+    }
+    out[2 * h] = make_uint4(w[0][0], w[0][1], w[1][0], w[1][1]);
+    out[2 * h + 1] = make_uint4(w[2][0], w[2][1], w[3][0], w[3][1]);
+  }
 }
 
 // Writes the 16 staged words (global word index w0..w0+15) of all lanes.
@@ -84,20 +117,9 @@ __device__ __noinline__ void flush_words(uint64_t* sz, uint64_t* gz, uint64_t* g
         uint64_t r8[8];
 #pragma unroll
         for (int r = 0; r < 8; r++) r8[r] = c.sz[(8 * grp + r) * STAGE_STRIDE + w];
-        uint64_t outw[8];
-#pragma unroll
-        for (int p = 0; p < 8; p++) {
-          uint64_t x = 0;
-#pragma unroll
-          for (int r = 0; r < 8; r++) x |= ((r8[r] >> (8 * p)) & 0xFFull) << (8 * r);
-          outw[p] = transpose8x8(x);
-        }
         size_t byte_idx = (c.warp_slot0 >> 3) + grp;
         uint4* dst = reinterpret_cast<uint4*>(c.stripe + byte_idx * (size_t)FLOCK_K + (size_t)(w0 + w) * 64);
-#pragma unroll
-        for (int q = 0; q < 4; q++)
-          dst[q] = make_uint4((uint32_t)outw[2 * q], (uint32_t)(outw[2 * q] >> 32), (uint32_t)outw[2 * q + 1],
-                              (uint32_t)(outw[2 * q + 1] >> 32));
+        stripe_bytes(r8, dst);
       }
     }
   }
@@ -247,7 +269,7 @@ witness_kernel(const flock_compression* __restrict__ in, size_t n_in, size_t n_t
 // witness bits are packed in registers, shifted to their place in the block and
 // joined into the block's image in shared memory (the words a G shares with its
 // neighbours by atomic ORs), the rounds in one loop body. The block then leaves
-// in 16-byte vectors, the stripe bytes by the same 8x8 transposes. 2^8
+// in 16-byte vectors, the stripe bytes by the same transposes. 2^8
 // compressions: 70 us through witness_kernel, 11 us so; 2^13: 61 us and 27 us;
 // 2^14: 62 us and 46 us; 2^15: 84 us so (half of a block's threads wait while the
 // rounds run, so the bandwidth-bound form wins beyond).
@@ -398,24 +420,14 @@ witness_small_kernel(const flock_compression* __restrict__ in, size_t n_in, size
   if (stripe) {
     for (int item = t; item < (n_valid >> 3) * KWORDS; item += WS_THREADS) {
       const int grp = item / KWORDS, w = item % KWORDS;
-      uint64_t r8[8], outw[8];
+      uint64_t r8[8];
 #pragma unroll
       for (int r = 0; r < 8; r++) {
         const uint2 v = *reinterpret_cast<const uint2*>(img[0] + (8 * grp + r) * WS_STRIDE + 2 * w);
         r8[r] = v.x | ((uint64_t)v.y << 32);
       }
-#pragma unroll
-      for (int p = 0; p < 8; p++) {
-        uint64_t x = 0;
-#pragma unroll
-        for (int r = 0; r < 8; r++) x |= ((r8[r] >> (8 * p)) & 0xFFull) << (8 * r);
-        outw[p] = transpose8x8(x);
-      }
       uint4* dst = reinterpret_cast<uint4*>(stripe + ((slot0 >> 3) + grp) * (size_t)FLOCK_K + (size_t)w * 64);
-#pragma unroll
-      for (int k = 0; k < 4; k++)
-        dst[k] = make_uint4((uint32_t)outw[2 * k], (uint32_t)(outw[2 * k] >> 32), (uint32_t)outw[2 * k + 1],
-                            (uint32_t)(outw[2 * k + 1] >> 32));
+      stripe_bytes(r8, dst);
     }
   }
 }
