@@ -213,12 +213,14 @@ __device__ __forceinline__ uint64_t shfl_xor64(uint64_t v, int m) {
 //        (entry v at slot v), so the block's values come out already
 //        weighted and need no GF(2^128) product; the table is the subset
 //        sums of its basis phi8(2^k) e, k < 8 (phi8 is additive), which
-//        zc1_eq_basis_kernel computes for every block beforehand. One lookup per
-//        value: the random bytes of a quarter warp share bank groups at times
-//        (about two wavefronts per quarter-warp lookup, measured), which the
-//        load/store pipe absorbs; with two nibble tables L[v & 15] + H[v >> 4] in eight
-//        conflict-free replicas (the same 4 KiB) each value took two lookups,
-//        two index computations and a four-word XOR on the busy ALU pipe;
+//        zc1_eq_basis_kernel computes for every block beforehand. WITH_C (bound
+//        by the ALU pipe): one lookup per value, the random bytes of a
+//        quarter warp sharing bank groups at times (2.6 wavefronts per quarter
+//        warp on average). Without the c sums the shared data path is the bound
+//        (97% busy, a quarter of it these lookups), so the table is two nibble
+//        tables L[v & 15] + H[v >> 4] of eight replicas, one per bank group:
+//        two conflict-free lookups and a four-word XOR (2,725 -> 2,658 us at 2^18
+//        compressions; with the c sums 3.97 -> 4.21 ms);
 //   xch  per warp: [16 producer rows] of 20 words (64 bytes used; the odd
 //        80-byte row pitch makes the 16-byte stores conflict-free), one plane
 //        set at a time.
@@ -339,8 +341,29 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
 #pragma unroll
       for (int j = 0; j < 16; j++) t[j] ^= shfl_xor64(t[j], 16);
     }
-    // eq-weighted phi8 table of this block (see the layout above)
-    {
+    // eq-weighted phi8 tables of this block (see the layout above)
+    if constexpr (!WITH_C) {
+      // replica lane & 7 of the nibbles n0 + 4 i, n0 = lane / 8: bits 0 and 1
+      // once, bits 2 and 3 along a Gray walk
+      uint4 pb[8];
+#pragma unroll
+      for (int k = 0; k < 8; k++) pb[k] = eq_basis[xo * 8 + k];
+      const uint32_t m0 = 0u - ((uint32_t)(lane >> 3) & 1u), m1 = 0u - ((uint32_t)(lane >> 4) & 1u);
+#pragma unroll
+      for (int tb = 0; tb < 2; tb++) {
+        const uint4 *b = pb + 4 * tb;
+        uint4 e = make_uint4((b[0].x & m0) ^ (b[1].x & m1), (b[0].y & m0) ^ (b[1].y & m1),
+                             (b[0].z & m0) ^ (b[1].z & m1), (b[0].w & m0) ^ (b[1].w & m1));
+#pragma unroll
+        for (int g = 0; g < 4; g++) {
+          if (g) {
+            const uint4 a = b[g == 2 ? 3 : 2];
+            e.x ^= a.x; e.y ^= a.y; e.z ^= a.z; e.w ^= a.w;
+          }
+          my_t8[128 * tb + 8 * ((lane >> 3) + 4 * (g ^ (g >> 1))) + (lane & 7)] = e;
+        }
+      }
+    } else {
       // lane l writes T8[l + 32 i], i < 8: the part of bits 0..4 (l) once,
       // then the part of bits 5..7 (i) along a Gray walk, one XOR per entry;
       // a quarter warp's stores are 128 consecutive bytes
@@ -386,7 +409,12 @@ zc_round1_kernel(const uint64_t* __restrict__ A, const uint64_t* __restrict__ B,
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const uint32_t v8 = (bw >> (8 * q)) & 255;
-          acc_shift_xor_v(v[q], my_t8[v8], (uint32_t)mm2);
+          if constexpr (WITH_C) {
+            acc_shift_xor_v(v[q], my_t8[v8], (uint32_t)mm2);
+          } else {
+            const uint4 l = my_t8[8 * (v8 & 15) + (lane & 7)], u = my_t8[128 + 8 * (v8 >> 4) + (lane & 7)];
+            acc_shift_xor_v(v[q], make_uint4(l.x ^ u.x, l.y ^ u.y, l.z ^ u.z, l.w ^ u.w), (uint32_t)mm2);
+          }
         }
       }
 #pragma unroll
