@@ -73,9 +73,12 @@ NTT_INSTR_PER_TABLE_PRODUCT = 160
 NTT_INSTR_PER_MULTIPLY_BUTTERFLY = 259
 NTT_INSTR_PER_DEEP_BUTTERFLY = 148
 # Zerocheck round 1 at m = 30 (2^17 outer blocks of 128 rows): warp
-# instructions and DRAM bytes (read + write) of one launch, per outer block.
-ZC1_WARP_INSTR_PER_OUTER = 603870960 / 2**17
-ZC1_DRAM_BYTES_PER_OUTER = (419600128 + 3706624) / 2**17
+# instructions and DRAM bytes (read + write) of one launch, per outer block, and
+# the arrays it reads: a and b from 2^14 compressions (the c statistic is a fold
+# of its own), a, b and z below.
+ZC1_SPLIT_LOG = 14
+ZC1_WARP_INSTR_PER_OUTER = {2: 402412080 / 2**17, 3: 603870960 / 2**17}
+ZC1_DRAM_BYTES_PER_OUTER = {2: (285421312 + 3680512) / 2**17, 3: (419600128 + 3706624) / 2**17}
 
 
 def load_peaks():
@@ -304,7 +307,7 @@ def ntt_l0_structure(F, dev_index, log_d):
         tab_end = 1
         while tab_end + 1 < log_d and log_d - tab_end - 2 + 6 >= 9:
             tab_end += 2
-    tab_passes = (tab_end - 1) // 2
+    tab_passes = tab_end // 2  # layers 1 .. tab_end - 1 in pairs, one alone where the count is odd
     passes = tab_passes + (log_d - tab_end + max_f - 1) // max_f
     return tab_passes, passes, tab_end, variant, max_f
 
@@ -315,7 +318,8 @@ def rooflines(F, log2, span_ms, peaks, sms, clock_mhz, dev_index):
 
     Algorithmic bytes follow the hot-path measurement rules: the NTT reads the
     message once and writes the codeword once (16 B x rows x 64 lanes x (1 + 2));
-    zerocheck round 1 reads a, b and z once (3 x 2^m / 8 bytes); the witness
+    zerocheck round 1 reads a and b once (2 x 2^m / 8 bytes; below 2^14
+    compressions z as well); the witness
     writes z, a, b and the stripe (4 x 2,048 B) and reads 112 B per compression.
     `traffic` is the ncu DRAM traffic per launch (set) scaled to this size;
     `integer_frac` is thread instructions (ncu counts) over the same time
@@ -354,11 +358,12 @@ def rooflines(F, log2, span_ms, peaks, sms, clock_mhz, dev_index):
     # zerocheck round 1
     ms = span_ms["zerocheck_round1"]
     n_outer = (1 << m) // 64 // 128
-    alg = 3 * (1 << m) // 8
-    ins = ZC1_WARP_INSTR_PER_OUTER * 32 * n_outer
-    traffic = ZC1_DRAM_BYTES_PER_OUTER * n_outer
+    arrays = 2 if log2 >= ZC1_SPLIT_LOG else 3
+    alg = arrays * (1 << m) // 8
+    ins = ZC1_WARP_INSTR_PER_OUTER[arrays] * 32 * n_outer
+    traffic = ZC1_DRAM_BYTES_PER_OUTER[arrays] * n_outer
     out["zerocheck_round1"] = {
-        "kernel": f"zerocheck univariate-skip round 1 over 2^{m - 6} rows of a, b, z",
+        "kernel": f"zerocheck univariate-skip round 1 over 2^{m - 6} rows of {'a, b' if arrays == 2 else 'a, b, z'}",
         "bound": "hbm", "achieved": alg / (ms * 1e-3) / 1e9, "peak": hbm, "unit": "GB/s",
         "frac": alg / (ms * 1e-3) / 1e9 / hbm, "traffic": traffic, "algorithmic_bytes": alg,
         "traffic_over_algorithmic": traffic / alg, "integer_frac": ins / (ms * 1e-3) / issue_peak,
