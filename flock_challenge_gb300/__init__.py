@@ -149,6 +149,7 @@ def _proto_lib():
                                             ctypes.c_int]
         L.flock_kernel_timing.argtypes = [P, ctypes.c_int]
         L.flock_set_wait_limit.argtypes = [P, ctypes.c_double]
+        L.flock_set_kernel_wait_limit.argtypes = [P, ctypes.c_uint64]
         L.flock_last_kernel_times.argtypes = [P, ctypes.POINTER(ctypes.c_double), ctypes.c_int]
         L.flock_prove_seed.argtypes = [P, ctypes.c_uint32, ctypes.c_uint64, P, ctypes.c_size_t,
                                        ctypes.POINTER(ctypes.c_size_t)]
@@ -375,6 +376,11 @@ class Blake3Setup:
         (0: no bound); a call whose wait passes it raises FlockError (timeout)
         and the next call first waits for its queued work (flock_set_wait_limit)."""
         check(_proto_lib().flock_set_wait_limit(self.ctx.handle, float(ms)), "flock_set_wait_limit")
+
+    def set_kernel_wait_limit(self, clocks=1 << 31):
+        """Bounds each wait inside this prover's later kernels by `clocks` SM clocks
+        (flock_set_kernel_wait_limit); a call whose kernel gave up raises FlockError (timeout)."""
+        check(_proto_lib().flock_set_kernel_wait_limit(self.ctx.handle, int(clocks)), "flock_set_kernel_wait_limit")
 
     def set_kernel_timing(self, on=True):
         """CUDA-event timing of the main kernels of each proof (flock_kernel_timing)."""

@@ -363,6 +363,15 @@ int flock_set_wait_limit(flock_ctx* ctx, double limit_ms) {
   return flock_prover_set_wait_limit(ctx->prover, limit_ms);
 }
 
+int flock_set_kernel_wait_limit(flock_ctx* ctx, uint64_t clocks) {
+  if (!ctx) return FLOCK_ERR_ARG;
+  if (!ctx->prover) {
+    ctx->prover = flock_prover_create(ctx->device);
+    if (!ctx->prover) return FLOCK_ERR_CUDA;
+  }
+  return flock_prover_set_kernel_wait_limit(ctx->prover, clocks);
+}
+
 int flock_last_kernel_times(const flock_ctx* ctx, double* ms, int n) {
   if (!ctx || !ctx->prover || !ms) return FLOCK_ERR_ARG;
   return flock_prover_kernel_times(ctx->prover, ms, n);

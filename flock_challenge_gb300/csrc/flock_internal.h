@@ -25,6 +25,16 @@ int flock_launch_merkle(const void* d_data, size_t n_leaves, size_t leaf_bytes, 
 
 // ---- protocol kernels ------------------------------------------------------
 struct ZcRound1Tables;
+// The waits inside a tensor-core kernel (tc.cuh): each gives up after `limit`
+// clocks; the kernel then sets *fault and its results are unusable.
+struct FlockKernelWait {
+  int* fault;
+  uint32_t limit;
+#ifdef __CUDACC__
+  __device__ __forceinline__ void gave_up() const { *(volatile int*)fault = 1; }
+#endif
+};
+constexpr uint32_t FLOCK_KERNEL_WAIT_CLOCKS = 1u << 31;  // the default: about a second
 // eq_basis: n_outer x 8 F128 from flock_launch_zc1_eq_basis. Rows of partials: 64
 // P^AB sums, then with c (may be null) the 128 sums of the c statistic.
 int flock_launch_zc_round1(const void* a, const void* b, const void* c, size_t n_outer, const void* eq_basis,
@@ -71,19 +81,18 @@ int flock_launch_zc_fold_a(const void* a, const void* lag, const void* e1, int l
                            cudaStream_t st);
 int flock_launch_zc_round_mma(const void* in_a, const void* in_b, int skip, const uint64_t rho[2], const void* lag,
                               void* Aout, void* Bout, const void* e2, const uint64_t cw[4][2], int hi_bits, int a_bits,
-                              int m_bits, int m_mul, int lo_bits, void* partials, int grid, int* fault,
-                              cudaStream_t st);
+                              int m_bits, int m_mul, int lo_bits, void* partials, int grid,
+                              const FlockKernelWait& kw, cudaStream_t st);
 int flock_launch_zc_unweight(void* A, size_t n, const void* e, int shift, int lo_bits, cudaStream_t st);
 int flock_launch_bind_pairs(const void* A, const void* B, size_t n, const uint64_t rho[2], void* Aout, void* Bout,
                             cudaStream_t st);
 
 // z_vec[i] = sum over the outer indices o < 8 n_stripes of z[i, o] eq(o) (2^14
 // entries; n_stripes a multiple of 32, at most 2^19). scratch:
-// flock_lc_fold_scratch_bytes(n_stripes). fault: set to one if a wait inside
-// the kernel gave up (the result is then unusable).
+// flock_lc_fold_scratch_bytes(n_stripes).
 size_t flock_lc_fold_scratch_bytes(size_t n_stripes);
 int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi, int lo_bits,
-                         void* scratch, void* z_vec, int* fault, cudaStream_t st);
+                         void* scratch, void* z_vec, const FlockKernelWait& kw, cudaStream_t st);
 // The base matrices' device copies (HostCsc, r1cs_setup.h).
 struct FlockLcMatrices {
   const uint32_t *a_ptr, *a_mid, *b_ptr, *b_mid, *order, *g_ptr;
@@ -106,9 +115,8 @@ int flock_launch_combined_basis(size_t n, const void* t0_lo, const void* t0_hi, 
 
 int flock_lig_grid(size_t n_pairs);       // blocks of lig_intro_eq
 int flock_lig_fold_grid(size_t n_pairs);  // blocks of lig_fold_msg (n_pairs = n_out / 2)
-// fault: set to one if a wait inside the kernel gave up.
 int flock_launch_lig_fold_msg(const void* f, const void* b, size_t n_out, int fold, const uint64_t r[2], void* fo,
-                              void* bo_out, void* partials, int grid, int* fault, cudaStream_t st);
+                              void* bo_out, void* partials, int grid, const FlockKernelWait& kw, cudaStream_t st);
 int flock_launch_lig_intro_eq(const void* f, size_t n, const void* lo, const void* hi, int lo_bits, void* partials,
                               int grid, cudaStream_t st);
 int flock_launch_glue_eq(void* b, size_t n, const void* lo, const void* hi, int lo_bits, const uint64_t beta[2],

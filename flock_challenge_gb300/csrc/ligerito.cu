@@ -68,7 +68,7 @@ template <bool FOLD>
 __global__ void __launch_bounds__(LM_THREADS, 1)
 lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, size_t n_tiles, const gf128 r,
                     gf128* __restrict__ fo, gf128* __restrict__ bo_out, gf128* __restrict__ partials,
-                    volatile int* fault) {
+                    const FlockKernelWait kw) {
   constexpr int LM_SLOTS = kLmSlots<FOLD>, LM_AHEAD = FOLD ? 4 : 8;
   extern __shared__ __align__(128) uint8_t lm_smem[];
   // done[tau mod 8]: the MMAs of tile tau of the CTA's sequence. A tile's warps
@@ -141,7 +141,7 @@ lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, si
       }
       const int slot = tau % LM_SLOTS;
       if (tau >= LM_SLOTS)
-        ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(tau - LM_SLOTS) % 8], ((tau - LM_SLOTS) / 8) & 1));
+        ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(tau - LM_SLOTS) % 8], ((tau - LM_SLOTS) / 8) & 1, kw.limit));
       if (ok) bo::put_tile(v, slots + slot * bo::SLOT + (is_b ? bo::SIDE : 0), lane & 1);
       tc::fence_smem_for_mma();
       __syncwarp();
@@ -150,7 +150,7 @@ lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, si
   } else if (lane == 0) {
     for (int tau = 0; tau < n && ok; tau++) {
       const int slot = tau % LM_SLOTS;
-      ok = tc::mbar_wait(&full[slot], (tau / LM_SLOTS) & 1);
+      ok = tc::mbar_wait(&full[slot], (tau / LM_SLOTS) & 1, kw.limit);
       if (!ok) break;
       tc::fence_after();
       bo::mma_slot(tc::smem_addr(slots + slot * bo::SLOT), tmem, sf, tau == 0);
@@ -159,8 +159,8 @@ lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, si
     tc::mma_commit(&all_done);
   }
   __syncwarp();  // the issuing warp's other lanes stay out of its way: a lane's wait holds up the whole warp
-  ok = tc::mbar_wait(&all_done, 0) && ok;
-  if (!ok) *fault = 1;
+  ok = tc::mbar_wait(&all_done, 0, kw.limit) && ok;
+  if (!ok) kw.gave_up();
   __syncwarp();
   tc::fence_after();
   if (warp < 8) bo::read_quadrant(tmem + 128 * (warp >> 2), poly[warp >> 2][warp & 3]);
@@ -168,7 +168,11 @@ lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, si
   __syncthreads();
   if (t < 2) partials[3 * blockIdx.x + t] = bo::combine(poly[t]);
   if (t == 2) partials[3 * blockIdx.x + 2] = gf_zero();
-  if (warp == 0) tc::tmem_free(tmem, 512);
+  if (warp == 0) {
+    tc::mbar_wait(&all_done, 0, tc::kDrainClocks);  // committed by now, whatever gave up
+    __syncwarp();
+    tc::tmem_free(tmem, 512);
+  }
 }
 
 // The same for small states (at most LG_SMALL_PAIRS pairs), bound by a
@@ -455,7 +459,7 @@ int flock_lig_fold_grid(size_t n_pairs) {
 }
 
 int flock_launch_lig_fold_msg(const void* f, const void* b, size_t n_out, int fold, const uint64_t r[2], void* fo,
-                              void* bo_out, void* partials, int grid, int* fault, cudaStream_t st) {
+                              void* bo_out, void* partials, int grid, const FlockKernelWait& kw, cudaStream_t st) {
   if (n_out / 2 <= LG_SMALL_PAIRS) {
     if (grid != gf_small_grid(n_out / 2)) return FLOCK_ERR_SHAPE;
     lig_fold_msg_small_kernel<<<grid, gf_small_threads(n_out / 2), 0, st>>>(
@@ -471,10 +475,10 @@ int flock_launch_lig_fold_msg(const void* f, const void* b, size_t n_out, int fo
   });
   if (fold)
     lig_fold_msg_kernel<true><<<grid, LM_THREADS, kLmSmem<true>, st>>>(
-        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), (gf128*)fo, (gf128*)bo_out, (gf128*)partials, fault);
+        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), (gf128*)fo, (gf128*)bo_out, (gf128*)partials, kw);
   else
     lig_fold_msg_kernel<false><<<grid, LM_THREADS, kLmSmem<false>, st>>>(
-        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), nullptr, nullptr, (gf128*)partials, fault);
+        (const gf128*)f, (const gf128*)b, n_tiles, to_gf(r), nullptr, nullptr, (gf128*)partials, kw);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }

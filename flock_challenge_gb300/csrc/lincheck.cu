@@ -73,9 +73,9 @@ __device__ __forceinline__ uint4 fm_expand(uint32_t w) {
 
 __global__ void __launch_bounds__(FM_THREADS, 1)
 lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict__ eq_bits, int n_stages, int parts,
-                   uint32_t* __restrict__ partials, volatile int* fault) {
+                   uint32_t* __restrict__ partials, const FlockKernelWait kw) {
   extern __shared__ __align__(128) uint8_t fm_smem[];  // A buffers, then B buffers
-  __shared__ uint64_t a_full[FM_BUFS], b_full[FM_BUFS], done[FM_BUFS];
+  __shared__ uint64_t a_full[FM_BUFS], b_full[FM_BUFS], done[FM_BUFS], all_done;
   __shared__ uint32_t tmem_slot;
   constexpr uint32_t kABytes = FM_PLANES * FM_A_PLANE, kBBytes = FM_PLANES * FM_B_PLANE;
   uint8_t* sa = fm_smem;
@@ -91,6 +91,7 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
       tc::mbar_init(&b_full[k], FM_PRODUCERS / 32);
       tc::mbar_init(&done[k], 1);
     }
+    tc::mbar_init(&all_done, 1);
     tc::mbar_fence_init();
   }
   tc::fence_before();
@@ -121,7 +122,9 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
       for (int k = 0; k < FM_AHEAD; k++) {
         const int it = it0 + k, b = it % FM_BUFS;
         if (it >= n) break;
-        if (it >= FM_BUFS) ok = tc::mbar_wait(&done[b], (it / FM_BUFS - 1) & 1);
+        // a warp gives up as one: part of it would leave the others at the barriers below
+        if (it >= FM_BUFS)
+          ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[b], (it / FM_BUFS - 1) & 1, kw.limit));
         if (!ok) break;
         const uint32_t l01 = __byte_perm(x[k][0], x[k][1], 0x5140), h01 = __byte_perm(x[k][0], x[k][1], 0x7362);
         const uint32_t l23 = __byte_perm(x[k][2], x[k][3], 0x5140), h23 = __byte_perm(x[k][2], x[k][3], 0x7362);
@@ -142,10 +145,12 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
       tc::mbar_expect(bar, kABytes);
       tc::bulk_load(sa + (it % FM_BUFS) * kABytes, eq_bits + (size_t)(s_begin + it) * kABytes, kABytes, bar);
     };
-    for (int it = 0; it < FM_BUFS - 1 && it < n; it++) load_a(it);
+    int loads = 0;
+    for (; loads < FM_BUFS - 1 && loads < n; loads++) load_a(loads);
     for (int it = 0; it < n && ok; it++) {
       const int b = it % FM_BUFS, j = it + FM_BUFS - 1;
-      ok = tc::mbar_wait(&a_full[b], (it / FM_BUFS) & 1) && tc::mbar_wait(&b_full[b], (it / FM_BUFS) & 1);
+      ok = tc::mbar_wait(&a_full[b], (it / FM_BUFS) & 1, kw.limit) &&
+           tc::mbar_wait(&b_full[b], (it / FM_BUFS) & 1, kw.limit);
       if (!ok) break;
       tc::fence_after();
       const uint32_t a0 = tc::smem_addr(sa + b * kABytes), b0 = tc::smem_addr(sb + b * kBBytes);
@@ -157,15 +162,18 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
       tc::mma_commit(&done[b]);
       // the buffer of stage j: its last MMAs (stage j - FM_BUFS = it - 1)
       if (j < n) {
-        if (j >= FM_BUFS) ok = tc::mbar_wait(&done[j % FM_BUFS], (j / FM_BUFS - 1) & 1);
-        if (ok) load_a(j);
+        if (j >= FM_BUFS) ok = tc::mbar_wait(&done[j % FM_BUFS], (j / FM_BUFS - 1) & 1, kw.limit);
+        if (ok) load_a(loads++);
       }
     }
+    tc::mma_commit(&all_done);
+    // after a give-up the last copies may be on their way
+    for (int j = loads < FM_BUFS ? 0 : loads - FM_BUFS; !ok && j < loads; j++)
+      tc::mbar_wait(&a_full[j % FM_BUFS], (j / FM_BUFS) & 1, tc::kDrainClocks);
   }
   __syncwarp();  // the issuing warp's other lanes stay out of its way: a lane's wait holds up the whole warp
-  // every MMA is done when the last stage's commit has arrived
-  ok = tc::mbar_wait(&done[(n - 1) % FM_BUFS], ((n - 1) / FM_BUFS) & 1) && ok;
-  if (!ok) *fault = 1;
+  ok = tc::mbar_wait(&all_done, 0, kw.limit) && ok;
+  if (!ok) kw.gave_up();
   __syncwarp();
   tc::fence_after();
   // counts -> parities: lane = row e of quadrant warp & 3, a ballot per column
@@ -188,7 +196,11 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
   }
   tc::fence_before();
   __syncthreads();
-  if (warp == 0) tc::tmem_free(tmem, 512);
+  if (warp == 0) {
+    tc::mbar_wait(&all_done, 0, tc::kDrainClocks);  // committed by now, whatever gave up
+    __syncwarp();
+    tc::tmem_free(tmem, 512);
+  }
 }
 
 // comb[c] = alpha * sum_{r in colA(c)} eq[r] + sum_{r in colB(c)} eq[r] (+ beta at pin).
@@ -296,7 +308,7 @@ size_t flock_lc_fold_scratch_bytes(size_t n_stripes) {
 }
 
 int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo, const void* eq_hi, int lo_bits,
-                         void* scratch, void* z_vec, int* fault, cudaStream_t st) {
+                         void* scratch, void* z_vec, const FlockKernelWait& kw, cudaStream_t st) {
   constexpr size_t kPerStage = FM_STAGE / 8;
   if (n_stripes == 0 || n_stripes % kPerStage != 0 || n_stripes > ((size_t)1 << 19)) return FLOCK_ERR_SHAPE;
   const size_t n_planes = n_stripes / 4;
@@ -312,7 +324,7 @@ int flock_launch_lc_fold(const void* stripe, size_t n_stripes, const void* eq_lo
   const int n_stages = (int)(n_stripes / kPerStage);
   const int parts = n_stages < FM_MAX_PARTS ? n_stages : FM_MAX_PARTS;
   lc_fold_mma_kernel<<<(unsigned)(FLOCK_K / FM_COLS * parts), FM_THREADS, FM_SMEM, st>>>(
-      (const uint8_t*)stripe, bits, n_stages, parts, (uint32_t*)(parts > 1 ? partials : z_vec), fault);
+      (const uint8_t*)stripe, bits, n_stages, parts, (uint32_t*)(parts > 1 ? partials : z_vec), kw);
   flock_count_launch();
   if (cudaGetLastError() != cudaSuccess) return FLOCK_ERR_CUDA;
   return parts > 1 ? flock_launch_reduce_rows(partials, parts, FLOCK_K, z_vec, st) : FLOCK_OK;

@@ -318,6 +318,8 @@ struct ProverState {
   int* fault() {
     return pin ? reinterpret_cast<int*>(pin + kPinH2D + kPinD2H - kGrindSlot / 2) : reinterpret_cast<int*>(grind.get(64)) + 8;
   }
+  uint32_t kernel_wait_clocks = FLOCK_KERNEL_WAIT_CLOCKS;
+  FlockKernelWait kernel_wait() { return {fault(), kernel_wait_clocks}; }
   bool faulted() { return pin && *reinterpret_cast<volatile int*>(fault()) != 0; }
   bool host_atomics = false;  // the device's atomics reach pinned host memory (cudaDevAttrHostNativeAtomicSupported)
   // The host's waits for the stream (flock_stream_wait) in the current proof.
@@ -632,6 +634,12 @@ int flock_prover_set_wait_limit(ProverState* S, double limit_ms) {
   return FLOCK_OK;
 }
 
+int flock_prover_set_kernel_wait_limit(ProverState* S, uint64_t clocks) {
+  if (clocks > FLOCK_KERNEL_WAIT_CLOCKS) return FLOCK_ERR_ARG;
+  S->kernel_wait_clocks = (uint32_t)clocks;
+  return FLOCK_OK;
+}
+
 int flock_prover_set_timing(ProverState* S, bool on) {
   if (on) {
     if (cudaSetDevice(S->device) != cudaSuccess) return FLOCK_ERR_CUDA;
@@ -806,7 +814,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         const size_t n_stripes = ((size_t)1 << n_log) / 8;
         FK(flock_launch_lc_fold(ds, n_stripes, S->tlo0.p, S->thi0.p, c_lo,
                                 S->part.get(flock_lc_fold_scratch_bytes(n_stripes)), S->zvec.get(FLOCK_K * 16),
-                                S->fault(), st));
+                                S->kernel_wait(), st));
         const auto eq_words = eq_table(std::vector<F>(r.begin() + 7, r.begin() + 14));
         const void* dew = staged(*S, S->small, eq_words.data(), 128 * 16);
         hsc = host_out(*S, 128 * 16, 128 * 16);
@@ -983,7 +991,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
         dpart = part_buf(*S, (size_t)grid * 2 * 16);
         FK(flock_launch_zc_round_mma(i == 0 ? dA0 : curA, i == 0 ? db : curB, i == 0, rp, dlag, i == 0 ? nullptr : nxtA,
                                      i == 0 ? dB0 : nxtB, mma_e2, cw, mma_hi, q.a_bits, q.m_bits, 1 << (q.f0 - 9), mma_lo,
-                                     dpart, grid, S->fault(), st));
+                                     dpart, grid, S->kernel_wait(), st));
       } else if (q.grp) {
         grid = (int)std::min<size_t>(n_pairs >> (q.lob + q.m_bits), 152 * 4);
         dpart = part_buf(*S, (size_t)grid * 2 * 16);
@@ -1112,7 +1120,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       size_t n_stripes = ((size_t)1 << n_outer_log) / 8;
       void* dzv = S->zvec.get(FLOCK_K * 16);
       FK(flock_launch_lc_fold(ds, n_stripes, S->eqlo.p, S->eqhi.p, lob,
-                              S->part.get(flock_lc_fold_scratch_bytes(n_stripes)), dzv, S->fault(), st));
+                              S->part.get(flock_lc_fold_scratch_bytes(n_stripes)), dzv, S->kernel_wait(), st));
       // product sumcheck on (comb, z_vec) binding the top variable
       // (lincheck.rs:1242-1300): the same round as the chain shift sumcheck
       // Rounds over at most kHostTailLincheck entries (and the final bind)
@@ -1370,12 +1378,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       uint64_t rp[2];
       u2(rr, rp);
       if (fold) {
-        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 1, rp, falt, balt, dpart, grid, S->fault(), st));
+        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 1, rp, falt, balt, dpart, grid, S->kernel_wait(), st));
         std::swap(fcur, falt);
         std::swap(bcur, balt);
         len = n_out;
       } else {
-        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 0, rp, nullptr, nullptr, dpart, grid, S->fault(), st));
+        FK(flock_launch_lig_fold_msg(fcur, bcur, n_out, 0, rp, nullptr, nullptr, dpart, grid, S->kernel_wait(), st));
       }
       auto s = reduce_partials(*S, dpart, grid, 3);
       msgs.push_back({s[0], s[1]});
@@ -1386,7 +1394,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       int grid = flock_lig_fold_grid(len / 2);
       void* dpart = part_buf(*S, (size_t)grid * 3 * 16);
       uint64_t rp[2] = {0, 0};
-      FK(flock_launch_lig_fold_msg(fcur, dbasis, len, 0, rp, nullptr, nullptr, dpart, grid, S->fault(), st));
+      FK(flock_launch_lig_fold_msg(fcur, dbasis, len, 0, rp, nullptr, nullptr, dpart, grid, S->kernel_wait(), st));
       auto s = reduce_partials(*S, dpart, grid, 3);
       msgs.push_back({s[0], s[1]});
       tr.observe(s[0]);

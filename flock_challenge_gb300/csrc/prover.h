@@ -55,6 +55,10 @@ int flock_prover_kernel_times(const ProverState* s, double* ms, int n);
 // Bounds every host wait of the state's later calls by limit_ms (0: no
 // bound): a wait that passes it makes the call return FLOCK_ERR_TIMEOUT.
 int flock_prover_set_wait_limit(ProverState* s, double limit_ms);
+// Bounds every wait inside the state's later kernels (at most
+// FLOCK_KERNEL_WAIT_CLOCKS, the default); the call of one that gave up returns
+// FLOCK_ERR_TIMEOUT.
+int flock_prover_set_kernel_wait_limit(ProverState* s, uint64_t clocks);
 // Device bytes the state holds (its buffers grow to the largest proof seen).
 size_t flock_prover_reserved_bytes(const ProverState* s);
 // Frees the state's device buffers (after its stream is idle); the next proof

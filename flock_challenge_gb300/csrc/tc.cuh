@@ -29,10 +29,20 @@ __device__ __forceinline__ void mbar_expect(uint64_t* b, uint32_t bytes) {
 __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
 }
-// Waits for the completion of phase `parity`; false when it gave up after 2^31
-// clocks, a second (no wait of a healthy kernel comes near it).
-__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
+// Waits for the completion of phase `parity`; false when it gave up after
+// `limit` clocks (0: at once, without looking).
+//
+// A kernel whose wait gave up still owns what it started: before its block
+// leaves or its TMEM is freed, the bulk copies it issued have landed and its MMAs
+// are done, or they would write shared memory or TMEM that the next block already
+// has. Every kernel therefore waits for them with kDrainClocks, whatever its own limit:
+// copies and MMAs end by themselves, they need nothing more of the block. (Past that
+// limit too, the block leaves all the same, and what its copies and MMAs then
+// write is undefined; a second without an end is a broken device.)
+constexpr uint32_t kDrainClocks = 1u << 31;
+__device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, uint32_t limit) {
   const uint32_t a = smem_addr(b);
+  if (limit == 0) return false;
   long long t0 = 0;
   for (;;) {
     uint32_t ok;
@@ -46,7 +56,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity) {
     if (ok) return true;
     const long long t = clock64();
     if (t0 == 0) t0 = t;
-    else if (t - t0 > (1ll << 31)) return false;
+    else if (t - t0 > (long long)limit) return false;
   }
 }
 // Contiguous copy into shared memory by the copy engine (16-byte aligned both

@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(ZM_THREADS, 1)
 zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b, const gf128 rho,
                     const gf128* __restrict__ lag, gf128* __restrict__ Aout, gf128* __restrict__ Bout,
                     const gf128* __restrict__ e2, const __grid_constant__ ZcClassWeights cw, int n_units, int a_bits,
-                    int m_bits, int m_mul, int lo_bits, gf128* __restrict__ partials, volatile int* fault) {
+                    int m_bits, int m_mul, int lo_bits, gf128* __restrict__ partials, const FlockKernelWait kw) {
   extern __shared__ __align__(128) uint8_t zm_smem[];
   // done[tau mod 8]: the MMAs of tile tau of the CTA's sequence (see lig_fold_msg_kernel)
   __shared__ uint64_t full[ZM_SLOTS], done[8], unit_done;
@@ -1106,7 +1106,8 @@ zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b
         }
         const int slot = tau % ZM_SLOTS;
         if (tau >= ZM_SLOTS)
-          ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[(tau - ZM_SLOTS) % 8], ((tau - ZM_SLOTS) / 8) & 1));
+          ok = __all_sync(0xffffffffu,
+                          tc::mbar_wait(&done[(tau - ZM_SLOTS) % 8], ((tau - ZM_SLOTS) / 8) & 1, kw.limit));
         if (ok) bo::put_tile(v, slots + slot * bo::SLOT + (is_b ? bo::SIDE : 0), 1 - (lane & 1));
         tc::fence_smem_for_mma();
         __syncwarp();
@@ -1115,7 +1116,7 @@ zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b
     } else if (lane == 0) {
       for (int x = ul << log_t; x < tau_end && ok; x++) {
         const int slot = x % ZM_SLOTS;
-        ok = tc::mbar_wait(&full[slot], (x / ZM_SLOTS) & 1);
+        ok = tc::mbar_wait(&full[slot], (x / ZM_SLOTS) & 1, kw.limit);
         if (!ok) break;
         tc::fence_after();
         bo::mma_slot(tc::smem_addr(slots + slot * bo::SLOT), tmem, sf, (x & (T - 1)) == 0);
@@ -1124,13 +1125,14 @@ zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b
       tc::mma_commit(&unit_done);
     }
     __syncwarp();
-    ok = tc::mbar_wait(&unit_done, ul & 1) && ok;
+    ok = tc::mbar_wait(&unit_done, ul & 1, kw.limit) && ok;
     __syncwarp();
     tc::fence_after();
     if (warp < 8) bo::read_quadrant(tmem + 128 * (warp >> 2), poly[ul & 1][warp >> 2][warp & 3]);
     tc::fence_before();
     if (__syncthreads_or(!ok)) {  // the counts are read, or a wait gave up
       ok = false;
+      if (warp == 0) tc::mbar_wait(&unit_done, ul & 1, tc::kDrainClocks);  // committed by now
       break;
     }
     tc::fence_after();
@@ -1140,7 +1142,7 @@ zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b
       acc = gf_add(acc, gf_mul(w, bo::combine(poly[ul & 1][t])));
     }
   }
-  if (!ok) *fault = 1;
+  if (!ok) kw.gave_up();
   if (t < 2) partials[2 * blockIdx.x + t] = acc;
   tc::fence_before();
   __syncthreads();
@@ -1302,8 +1304,8 @@ int flock_launch_zc_unweight(void* A, size_t n, const void* e, int shift, int lo
 
 int flock_launch_zc_round_mma(const void* in_a, const void* in_b, int skip, const uint64_t rho[2], const void* lag,
                               void* Aout, void* Bout, const void* e2, const uint64_t cw[4][2], int hi_bits, int a_bits,
-                              int m_bits, int m_mul, int lo_bits, void* partials, int grid, int* fault,
-                              cudaStream_t st) {
+                              int m_bits, int m_mul, int lo_bits, void* partials, int grid,
+                              const FlockKernelWait& kw, cudaStream_t st) {
   const int n_units = 1 << (hi_bits + a_bits);
   if (a_bits < 0 || a_bits > 2 || m_bits < 1 || m_bits > 4 || m_mul < 1 || m_mul * ((1 << m_bits) - 1) > 15 ||
       lo_bits + m_bits < 7 || hi_bits < 0 || hi_bits + a_bits > 24 || grid < 1 || grid > n_units)
@@ -1320,11 +1322,11 @@ int flock_launch_zc_round_mma(const void* in_a, const void* in_b, int skip, cons
   if (skip)
     zc_round_mma_kernel<true><<<grid, ZM_THREADS, kZmSmem<true>, st>>>(
         in_a, in_b, gf(rho), (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)e2, w, n_units, a_bits, m_bits,
-        m_mul, lo_bits, (gf128*)partials, fault);
+        m_mul, lo_bits, (gf128*)partials, kw);
   else
     zc_round_mma_kernel<false><<<grid, ZM_THREADS, kZmSmem<false>, st>>>(
         in_a, in_b, gf(rho), (const gf128*)lag, (gf128*)Aout, (gf128*)Bout, (const gf128*)e2, w, n_units, a_bits, m_bits,
-        m_mul, lo_bits, (gf128*)partials, fault);
+        m_mul, lo_bits, (gf128*)partials, kw);
   flock_count_launch();
   return cudaGetLastError() == cudaSuccess ? FLOCK_OK : FLOCK_ERR_CUDA;
 }

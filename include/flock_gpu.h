@@ -28,7 +28,8 @@ enum {
   FLOCK_ERR_ARG = -4,     /* null or inconsistent argument */
   FLOCK_ERR_CAPACITY = -5,/* output buffer too small */
   FLOCK_ERR_TIMEOUT = -6, /* a bounded wait or search gave up: a host wait passed the context's
-                           wait limit (flock_set_wait_limit), or the grind's nonce range ran out */
+                           wait limit (flock_set_wait_limit), a wait inside a kernel passed its own
+                           (flock_set_kernel_wait_limit), or the grind's nonce range ran out */
   FLOCK_ERR_VERIFY = -7,  /* an internal consistency check failed */
   FLOCK_ERR_LIMIT = -8    /* size above the fixed limit of an entry point that allocates nothing */
 };
@@ -230,6 +231,15 @@ int flock_last_kernel_times(const flock_ctx* ctx, double* ms, int n);
  * deadline (crates/flock-core/src/gpu_commit.rs:1250-1257), and on a GPU
  * error it falls back to the CPU (:1462-1465). */
 int flock_set_wait_limit(flock_ctx* ctx, double limit_ms);
+
+/* The waits inside the tensor-core kernels of this context's later proofs
+ * (each for a warp, a copy or an MMA of its own block) give up after `clocks`
+ * SM clocks; the kernel then ends in order and the call returns
+ * FLOCK_ERR_TIMEOUT, the context staying usable. The default and largest value
+ * is 2^31, about a second, which no wait of a working GPU comes near; 0: the
+ * first wait gives up, which is how the path is tested. FLOCK_ERR_ARG above
+ * 2^31. No reference counterpart. */
+int flock_set_kernel_wait_limit(flock_ctx* ctx, uint64_t clocks);
 
 /* ---- Verification -------------------------------------------------------- */
 
