@@ -15,6 +15,8 @@
 #pragma once
 #include <cstdint>
 
+#include "wait_clock.h"
+
 namespace tc {
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -30,7 +32,7 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
 }
 // Waits for the completion of phase `parity`; false when it gave up after
-// `limit` clocks (0: at once, without looking).
+// `limit` clocks of waiting (wait_clock.h; 0: at once, without looking).
 //
 // A kernel whose wait gave up still owns what it started: before its block
 // leaves or its TMEM is freed, the bulk copies it issued have landed and its MMAs
@@ -43,7 +45,7 @@ constexpr uint32_t kDrainClocks = 1u << 31;
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, uint32_t limit) {
   const uint32_t a = smem_addr(b);
   if (limit == 0) return false;
-  long long t0 = 0;
+  WaitClock wc;
   for (;;) {
     uint32_t ok;
     asm volatile(
@@ -54,9 +56,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, uint32_t
         : "r"(a), "r"(parity)
         : "memory");
     if (ok) return true;
-    const long long t = clock64();
-    if (t0 == 0) t0 = t;
-    else if (t - t0 > (long long)limit) return false;
+    if (wc.passed((uint32_t)clock(), limit)) return false;
   }
 }
 // Contiguous copy into shared memory by the copy engine (16-byte aligned both

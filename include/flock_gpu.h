@@ -234,7 +234,8 @@ int flock_set_wait_limit(flock_ctx* ctx, double limit_ms);
 
 /* The waits inside the tensor-core kernels of this context's later proofs
  * (each for a warp, a copy or an MMA of its own block) give up after `clocks`
- * SM clocks; the kernel then ends in order and the call returns
+ * SM clocks of waiting (time the GPU gives to other processes meanwhile does
+ * not count); the kernel then ends in order and the call returns
  * FLOCK_ERR_TIMEOUT, the context staying usable. The default and largest value
  * is 2^31, about a second, which no wait of a working GPU comes near; 0: the
  * first wait gives up, which is how the path is tested. FLOCK_ERR_ARG above
