@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <array>
 #include <chrono>
+#include <cstdlib>
 #include <cstring>
 #include <mutex>
 #include <stdexcept>
@@ -286,6 +287,7 @@ struct ProverState {
   DBuf in, z, a, b, stripe, cw, tree, A0, B0, A1, B1, eqlo, eqhi, eqout, part, red, lag, small, eqin, comb,
       zvec, zvec1, tlo0, thi0, tlo1, thi1, tables, bc, f1, b1, LO, basis, qbuf, qopen, rows, nidx, nodes,
       grind, lvl_cw[2], lvl_tree[2], chW, chG, zceq;
+  DBuf fault_dev;                 // fault() without pinned staging
   DBuf csc_meta, csc_ai, csc_bi;  // the base matrices (HostCsc): pointers and order, row indices
   FlockLcMatrices lcm = {};
   bool csc_ready = false;
@@ -313,14 +315,12 @@ struct ProverState {
   // host memory, so reading a round's message needs only the stream sync.
   uint8_t* mapped = nullptr;
   void* mapped_dev = nullptr;
-  // A word kernels set when a wait inside them gave up (bounded, tc.cuh); read
-  // with the next result. Host memory, or device memory nobody reads without it.
-  int* fault() {
-    return pin ? reinterpret_cast<int*>(pin + kPinH2D + kPinD2H - kGrindSlot / 2) : reinterpret_cast<int*>(grind.get(64)) + 8;
-  }
+  // A word kernels set when a wait inside them gave up (bounded, tc.cuh), cleared
+  // at the start of a proof and read by faulted(): in the pinned read area, or,
+  // without one, in device memory.
+  int* fault() { return (int*)(pin ? pin + kPinH2D + kPinD2H - kGrindSlot / 2 : fault_dev.get(4)); }
   uint32_t kernel_wait_clocks = FLOCK_KERNEL_WAIT_CLOCKS;
   FlockKernelWait kernel_wait() { return {fault(), kernel_wait_clocks}; }
-  bool faulted() { return pin && *reinterpret_cast<volatile int*>(fault()) != 0; }
   bool host_atomics = false;  // the device's atomics reach pinned host memory (cudaDevAttrHostNativeAtomicSupported)
   // The host's waits for the stream (flock_stream_wait) in the current proof.
   WaitStats waits;
@@ -329,7 +329,7 @@ struct ProverState {
     std::vector<DBuf*> v = {&in, &z, &a, &b, &stripe, &cw, &tree, &A0, &B0, &A1, &B1, &eqlo, &eqhi, &eqout, &part, &red,
             &lag, &small, &eqin, &comb, &zvec, &zvec1, &tlo0, &thi0, &tlo1, &thi1, &tables, &bc, &f1, &b1,
             &LO, &basis, &qbuf, &qopen, &rows, &nidx, &nodes, &grind, &lvl_cw[0], &lvl_cw[1],
-            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &csc_meta, &csc_ai, &csc_bi};
+            &lvl_tree[0], &lvl_tree[1], &chW, &chG, &zceq, &fault_dev, &csc_meta, &csc_ai, &csc_bi};
     for (DBuf& d : skl) v.push_back(&d);
     return v;
   }
@@ -414,6 +414,17 @@ void d2h2(ProverState& S, void* h1, const void* d1, size_t n1, void* h2, const v
   CK(flock_stream_wait(S.st, &S.waits));
   if (n1) std::memcpy(h1, p, n1);
   if (n2) std::memcpy(h2, p + off2, n2);
+}
+// The fault word, behind a wait for the kernels that may set it.
+void clear_fault(ProverState& S) {
+  if (S.pin) *S.fault() = 0;
+  else CK(cudaMemsetAsync(S.fault(), 0, 4, S.st));
+}
+bool faulted(ProverState& S) {
+  if (S.pin) return *reinterpret_cast<volatile int*>(S.fault()) != 0;
+  int f = 0;
+  d2h(S, &f, S.fault(), 4);
+  return f != 0;
 }
 void u2(const F& x, uint64_t out[2]) { out[0] = x.lo; out[1] = x.hi; }
 
@@ -580,18 +591,19 @@ ProverState* flock_prover_create(int device) {
       cudaStreamCreateWithPriority(&S->st_high, cudaStreamNonBlocking, greatest) != cudaSuccess)
     S->st_high = nullptr;
   cudaGetLastError();
-  // Without pinned staging the copies still work, through the driver's own.
+  // Without pinned staging the copies still work, through the driver's own;
+  // FLOCK_PINNED=0 in the environment does without on hosts that cannot lock memory.
+  const char* pe = std::getenv("FLOCK_PINNED");
+  const bool pinned = !(pe && pe[0] == '0');
   void* pin = nullptr;
-  if (cudaMallocHost(&pin, kPinH2D + kPinD2H) == cudaSuccess) S->pin = (uint8_t*)pin;
-  else cudaGetLastError();
+  if (pinned && cudaMallocHost(&pin, kPinH2D + kPinD2H) == cudaSuccess) S->pin = (uint8_t*)pin;
   int native = 0;
   S->host_atomics =
       cudaDeviceGetAttribute(&native, cudaDevAttrHostNativeAtomicSupported, device) == cudaSuccess && native;
   void* po = nullptr;
-  if (cudaMallocHost(&po, kPinOpen) == cudaSuccess) S->pin_open = (uint8_t*)po;
-  else cudaGetLastError();
+  if (pinned && cudaMallocHost(&po, kPinOpen) == cudaSuccess) S->pin_open = (uint8_t*)po;
   void* m = nullptr;
-  if (cudaHostAlloc(&m, kMapped, cudaHostAllocMapped) == cudaSuccess) {
+  if (pinned && cudaHostAlloc(&m, kMapped, cudaHostAllocMapped) == cudaSuccess) {
     if (cudaHostGetDevicePointer(&S->mapped_dev, m, 0) == cudaSuccess) S->mapped = (uint8_t*)m;
     else cudaFreeHost(m);
   }
@@ -688,7 +700,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     CK(flock_stream_wait(S->st, &S->waits, false));
     S->pin_off = 0;
     S->pin_open_off = 0;
-    if (S->pin) *S->fault() = 0;
+    clear_fault(*S);
     const int m = 14 + n_log;
     LigCfg cfg;
     if (!lig_config(m, 0, cfg)) return FLOCK_ERR_SHAPE;
@@ -838,7 +850,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       } else {
         if (hsc) std::memcpy(shv_c.data(), hsc, 128 * 16);  // the reduction's wait has passed
         else d2h(*S, shv_c.data(), dsc, 128 * 16);
-        if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "stripe fold");
+        if (faulted(*S)) throw Fail(FLOCK_ERR_TIMEOUT, "stripe fold");
       }
       std::vector<F> cs(64);
       for (int s = 0; s < 64; s++) cs[s] = (F::one() + r[6]) * shv_c[s] + r[6] * shv_c[64 + s];
@@ -1085,7 +1097,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       fb = tB[0];
     }
     if (mma_rounds) fa = fa * a_scale;
-    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "zerocheck round");
+    if (faulted(*S)) throw Fail(FLOCK_ERR_TIMEOUT, "zerocheck round");
     tr.observe(fa);
     tr.observe(fb);
     T.zc_rounds_ms = clk.lap();
@@ -1184,7 +1196,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       bind_top(hg, lc_rr.back());
       std::copy(hg.begin(), hg.begin() + 64, z_partial.begin());
     }
-    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "stripe fold");
+    if (faulted(*S)) throw Fail(FLOCK_ERR_TIMEOUT, "stripe fold");
     tr.observe_slice(z_partial.data(), 64);
     const F lc_skip = tr.sample();  // lincheck's skip challenge: the ab claim's z_skip
     std::vector<F> r_inner_rest(lc_rr.rbegin(), lc_rr.rend());
@@ -1530,7 +1542,7 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     // one wait for the openings' queued copies (the final opening's gathers
     // are the last work of the phase)
     CK(flock_stream_wait(st, &S->waits));
-    if (S->faulted()) throw Fail(FLOCK_ERR_TIMEOUT, "Ligerito fold");
+    if (faulted(*S)) throw Fail(FLOCK_ERR_TIMEOUT, "Ligerito fold");
     finish_open(*S, open0);
     for (Open& o : rec_opens) finish_open(*S, o);
     finish_open(*S, final_open);
