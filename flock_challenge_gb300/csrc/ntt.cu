@@ -931,7 +931,8 @@ const void* flock_ntt_twiddles_prepared(int log_d) {
 // speed differs. FLOCK_NTT_TUNE=0 in the environment turns tuning off (the
 // default depth and shape everywhere); FLOCK_NTT_VARIANT=0..4 fixes the
 // multiply-pass shape (with the default depth; 4: stage passes of all layers; 3
-// and 4 fall back to shape 1 where they do not apply).
+// and 4 fall back to shape 1 where they do not apply) and FLOCK_NTT_TAB_END beside
+// it the table passes' end layer.
 namespace {
 
 struct TuneKey {
@@ -1058,8 +1059,13 @@ TunedShape pick_shape(int log_d, int log_lanes, int start, const void* tw, const
   const TunedShape dflt{tab_layers_end(log_d, log_lanes, start), kDefaultVariant};
   if (const char* f = std::getenv("FLOCK_NTT_VARIANT")) {  // a fixed shape, for measurements
     const int v = f[0] - '0';
-    if ((v >= 0 && v < kVariants) || v == kDeepVariant) return TunedShape{dflt.tab_end, v};
-    if (v == kStageVariant) return TunedShape{stage_applies(log_d, log_lanes, start) ? start : dflt.tab_end, v};
+    if ((v >= 0 && v < kVariants) || v == kDeepVariant || v == kStageVariant) {
+      TunedShape sh{v == kStageVariant && stage_applies(log_d, log_lanes, start) ? start : dflt.tab_end, v};
+      const char* e = std::getenv("FLOCK_NTT_TAB_END");
+      const int te = e ? std::atoi(e) : -1;
+      if (te >= start && te <= log_d) sh.tab_end = te;
+      return sh;
+    }
   }
   if (!tuning_enabled()) return dflt;
   TuneKey k{0, log_d, log_lanes, start};
