@@ -893,10 +893,12 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
     // Rounds 0 .. mma_end - 1 (the grouped ones) on the tensor cores
     // (zc_round_mma_kernel): from 2^kMmaRoundsLog compressions, unless an outer
     // challenge whose weight goes into the A table is 0 or 1 (then it could not
-    // be divided out).
+    // be divided out). FLOCK_ZC_MMA=0 in the environment takes the form of those proofs
+    // for all, which is how it is tested.
     int mma_end = 0;
     const int n_out_vars = m - 13, mma_lo = std::min(10, std::max(6, n_out_vars - 8)), mma_hi = n_out_vars - mma_lo;
-    bool mma_rounds = n_log >= kMmaRoundsLog;
+    const char* ze = std::getenv("FLOCK_ZC_MMA");
+    bool mma_rounds = n_log >= kMmaRoundsLog && !(ze && ze[0] == '0');
     F a_scale = F::one();  // from round mma_end on the A table is 1 / a_scale of the protocol's
     if (mma_rounds) {
       F p = F::one();
