@@ -142,9 +142,6 @@ int flock_grind(const uint8_t digest[32], uint32_t bits, void* d_scratch, int* p
 
 // Launch counter of this library's kernels (read through flock_kernel_launches).
 int flock_launch_fold_lsb(const void* in, size_t n_out, const uint64_t r[2], void* out, cudaStream_t st);
-int flock_launch_zc_round0_skip(const void* a, const void* b, size_t n_pairs, const void* lag, void* A0, void* B0,
-                                const void* eq_lo, const void* eq_hi, int lo_bits, void* partials, int grid,
-                                cudaStream_t st);
 // Zerocheck rounds 0..5 with the fixed-challenge eq factorisation
 // (zc_round_grp_kernel): skip != 0 is round 0 from the bit rows in0, in1 (lag:
 // the 64 skip Lagrange weights); otherwise in0, in1 are bound at rho. eq_lo

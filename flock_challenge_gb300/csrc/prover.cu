@@ -1025,10 +1025,8 @@ int flock_prover_prove(ProverState* S, const flock_compression* h_in, size_t n, 
       } else {
         grid = (int)std::max<size_t>(std::min<size_t>(n_pairs >> q.lob, 152 * 4), 1);
         dpart = part_buf(*S, (size_t)grid * 2 * 16);
-        if (i == 0)  // skip fold (multilinear.rs:598-630) fused into round 0
-          FK(flock_launch_zc_round0_skip(da, db, n_pairs, dlag, dA0, dB0, elo, ehi, q.lob, dpart, grid, st));
-        else
-          FK(flock_launch_zc_round(curA, curB, n_pairs, 1, rp, nxtA, nxtB, elo, ehi, q.lob, dpart, grid, st));
+        // (never round 0, which is grouped or small at every size)
+        FK(flock_launch_zc_round(curA, curB, n_pairs, 1, rp, nxtA, nxtB, elo, ehi, q.lob, dpart, grid, st));
       }
       auto g = reduce_partials(*S, dpart, grid, 2);
       g[0] = g[0] * q.dinv;
