@@ -100,7 +100,7 @@ lig_fold_msg_kernel(const gf128* __restrict__ f, const gf128* __restrict__ b, si
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  bool ok = true;
+  bool ok = kw.limit != 0;
   if (t < LM_PRODUCERS) {
     const bool is_b = warp >= 8;
     const gf128* in = is_b ? b : f;

@@ -103,7 +103,7 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  bool ok = true;
+  bool ok = kw.limit != 0;
   if (t < FM_PRODUCERS) {
     // column word cw (four columns) of plane g: stripes 4 g .. 4 g + 3 of a stage
     const int cw = t & 63, g = t >> 6;
@@ -117,15 +117,14 @@ lc_fold_mma_kernel(const uint8_t* __restrict__ stripe, const uint8_t* __restrict
 #pragma unroll
     for (int k = 0; k < FM_AHEAD; k++)
       if (k < n) load(k, x[k]);
-    for (int it0 = 0; it0 < n && ok; it0 += FM_AHEAD) {
+    for (int it0 = 0; it0 < n; it0 += FM_AHEAD) {
 #pragma unroll
       for (int k = 0; k < FM_AHEAD; k++) {
         const int it = it0 + k, b = it % FM_BUFS;
         if (it >= n) break;
-        // a warp gives up as one: part of it would leave the others at the barriers below
-        if (it >= FM_BUFS)
-          ok = __all_sync(0xffffffffu, tc::mbar_wait(&done[b], (it / FM_BUFS - 1) & 1, kw.limit));
-        if (!ok) break;
+        // a lane that gave up stays in step, without waiting any more: leaving, it would
+        // miss its warp at the barriers below
+        if (it >= FM_BUFS && ok) ok = tc::mbar_wait(&done[b], (it / FM_BUFS - 1) & 1, kw.limit);
         const uint32_t l01 = __byte_perm(x[k][0], x[k][1], 0x5140), h01 = __byte_perm(x[k][0], x[k][1], 0x7362);
         const uint32_t l23 = __byte_perm(x[k][2], x[k][3], 0x5140), h23 = __byte_perm(x[k][2], x[k][3], 0x7362);
         uint4* row = reinterpret_cast<uint4*>(sb + b * kBBytes + g * FM_B_PLANE) + cw;

@@ -32,7 +32,8 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_addr(b)) : "memory");
 }
 // Waits for the completion of phase `parity`; false when it gave up after
-// `limit` clocks of waiting (wait_clock.h; 0: at once, without looking).
+// `limit` clocks of waiting (wait_clock.h). Kernels whose limit is zero start as
+// if a wait had given up.
 //
 // A kernel whose wait gave up still owns what it started: before its block
 // leaves or its TMEM is freed, the bulk copies it issued have landed and its MMAs
@@ -44,7 +45,6 @@ __device__ __forceinline__ void mbar_arrive(uint64_t* b) {
 constexpr uint32_t kDrainClocks = 1u << 31;
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, uint32_t parity, uint32_t limit) {
   const uint32_t a = smem_addr(b);
-  if (limit == 0) return false;
   WaitClock wc;
   for (;;) {
     uint32_t ok;

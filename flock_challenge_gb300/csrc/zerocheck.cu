@@ -964,7 +964,7 @@ zc_round_mma_kernel(const void* __restrict__ in_a, const void* __restrict__ in_b
   tc::fence_before();
   __syncthreads();
   tc::fence_after();
-  bool ok = true;
+  bool ok = kw.limit != 0;
   const bool is_b = warp >= 8;
   const int w8 = warp & 7;
   const uint32_t rot = t & 15, sh = (uint32_t)(m_mul * ((lane >> 1) & ((1 << m_bits) - 1)));
