@@ -295,8 +295,9 @@ def kernel_microbench(F, ctx_handle, peaks, torch, dev, rows_logs=(16, 18, 20), 
 def ntt_l0_structure(F, dev_index, log_d):
     """(table passes, total passes, table-pass end layer, multiply-pass shape) of
     the L0 commit NTT as the library's autotuner chose them: two-layer
-    byte-table passes from layer 1 to the tuned end layer, then multiply passes
-    of the tuned shape (the untuned default when the shape has not run)."""
+    byte-table passes from layer 1 to the tuned end layer (a one-layer pass first
+    where the layers are odd in number), then passes of the tuned shape (the
+    untuned default when the shape has not run)."""
     L = F.lib()
     L.flock_ntt_tuned_variant.argtypes = [ctypes.c_int] * 4
     L.flock_ntt_tuned_table_end.argtypes = [ctypes.c_int] * 4

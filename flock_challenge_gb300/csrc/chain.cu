@@ -95,7 +95,8 @@ chain_round_kernel(const gf128* W, const gf128* g, size_t h, int bind, const __g
 
 // The same for at most CH_SMALL_PAIRS entry pairs, bound by a thread's chain:
 // two lanes a pair (gf_round_small). 2^11 entries: chain_round_kernel 9.2 us,
-// this 5.1 us.
+// this 5.1 us; with the L2 flushed and events around, 2^13 pairs 11.9 and 7.9 us, 2^15 12.0 and
+// 11.9, 2^16 18.1 and 18.1, 2^17 28.3 and 26.3, 2^18 44.7 and 46.7, 2^20 147 and 157.
 constexpr size_t CH_SMALL_PAIRS = (size_t)1 << 17;
 __global__ void __launch_bounds__(CH_THREADS)
 chain_round_small_kernel(const gf128* W, const gf128* g, size_t h, int bind, const gf128 r, gf128* Wo, gf128* go,

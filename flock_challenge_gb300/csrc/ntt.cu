@@ -926,7 +926,10 @@ const void* flock_ntt_twiddles_prepared(int log_d) {
 // end layer, plus the deep-table pass where a depth leaves exactly the last
 // three layers of a code of 64 lanes or more (a one-layer table pass first where
 // the depths would be a layer off) and, for 8-lane codes, the stage passes from
-// every depth's end (up to 2^15 positions from every smaller one); it keeps the
+// every depth's end; up to 2^15 positions from every smaller one as well, where
+// they win (from layer 2, the call in us by end layer 2, 4, .., L2 flushed: 2^13 29, 33, 38, 38,
+// 44; 2^14 38, 40, 44, 44, 48; 2^15 60, 60, 58, 56, 58; 2^16 111, 97, 95, 95, 91,
+// 105; 2^17 199, 185, 177, 173, 165, 170). It keeps the
 // pair with the smallest sum for later calls. All candidates compute identical results; only
 // speed differs. FLOCK_NTT_TUNE=0 in the environment turns tuning off (the
 // default depth and shape everywhere); FLOCK_NTT_VARIANT=0..4 fixes the

@@ -46,8 +46,8 @@ struct WarpCtx {
 // exchanges between the rows' registers (row bit against bit index), after
 // which row i holds the bytes of bit i, then 4 x 4 byte transposes.
 // Gathering each byte of the rows by shifts and transposing 8 x 8 bits at a time
-// cost several times the instructions: 2^17 slots of witness_kernel 199 -> 180 us,
-// 0.89 of the measured HBM rate.
+// cost several times the instructions: 2^17 slots of witness_kernel 203 -> 186 us,
+// 0.86 of the measured HBM rate (199 -> 180 us, 0.89, on another GPU).
 __device__ __forceinline__ void stripe_exchange(uint32_t& a, uint32_t& b, int k, uint32_t low) {
   const uint32_t t = ((a >> k) ^ b) & low;
   b ^= t;

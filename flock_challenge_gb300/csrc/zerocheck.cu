@@ -859,8 +859,12 @@ zc_round_small_kernel(const void* __restrict__ in0, const void* __restrict__ in1
 // (zc_round_grp_kernel), 1,144 us so and 405 us for the fold of A; rounds 1..5
 // 2,771 us and 2,146 us; 2^13: rounds 0..2 232 us and 165 + 19 us. Used from 2^12
 // compressions (one chain of 2^12: 2.21 -> 2.16 ms; below, round 0 alone exceeds
-// the small rounds' limit); the grouped kernels stay for 2^11 and for an outer
-// challenge of 0 or 1.
+// the small rounds' limit); the grouped kernels stay for round 0 of 2^11 and for an
+// outer challenge of 0 or 1. The rounds run here down to round 5 at every size, so that
+// A is divided once, when it is smallest. The last of the smallest proofs lose a little by
+// it: at 2^12 rounds 4 and 5 (2^15 and 2^14 pairs) take 13.2 and 12.4 us and at 2^13 round 5 (2^15
+// pairs) 18.4 us, where zc_round_small_kernel takes 11.1 us for 2^15 and 7.4 us for 2^14 pairs;
+// from 2^16 pairs on this form is level or wins (14.3..19.8 us against 18.8; 2^17: 18.8..23.1 against 30).
 __global__ void __launch_bounds__(256)
 zc_fold_a_kernel(const uint64_t* __restrict__ W, const gf128* __restrict__ lag, const gf128* __restrict__ e1,
                  int lo_bits, size_t n_hi, int parts, gf128* __restrict__ A0) {

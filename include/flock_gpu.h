@@ -96,10 +96,15 @@ int flock_ntt(flock_ctx* ctx, void* d_data, int log_d, int log_num_ntts, int sta
  * 3: the deep-table pass, the last three layers of a code of 64 lanes or more
  * through tables of its narrow twiddles' products; 4: stage passes of an 8-lane code,
  * four positions per thread and two layers per stage) and the end layer of the
- * byte-table passes (the upper layers run as
- * two-layer table passes while a block holds at least 2^k position-quads x
- * lanes, k tuned among 8, 9, 10; the layers from the end layer on run as
- * multiply passes). The first flock_ntt / commit / proof of a shape times the
+ * byte-table passes, from which the layers run in passes of that shape. The table passes
+ * take two layers each, from start_layer to the end layer. It is one of
+ *   - the depths to which a block holds at least 2^k position-quads x lanes,
+ *     k = 8, 9, 10;
+ *   - log_d - 3 for codes of 64 lanes or more, in front of the deep-table pass; at
+ *     an odd distance from start_layer a one-layer table pass goes first;
+ *   - any smaller depth at an even distance from start_layer, for 8-lane codes of
+ *     at most 2^15 positions, in front of stage or multiply passes.
+ * The first flock_ntt / commit / proof of a shape times the
  * candidates on a scratch buffer and keeps the fastest; FLOCK_NTT_TUNE=0 in the
  * environment disables tuning (k = 9, shape 1). No reference counterpart. */
 int flock_ntt_tuned_variant(int device, int log_d, int log_lanes, int start_layer);
